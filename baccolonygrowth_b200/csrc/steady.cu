@@ -34,15 +34,25 @@
 
 #define ST_MAX_LEVELS 12
 #define ST_RED_BLOCKS 256
+/* points of the levels the one-block tail of the V-cycle holds in shared
+ * memory (32 B each: x, b, the diagonal and its reciprocal) */
+#define ST_TAIL_POINTS 6400
+#define ST_TAIL_THREADS 512
+/* unknowns of the coarsest level up to which its sweeps run as one matrix */
+#define ST_OP_MAX 32
+#define ST_CHUNK 4               /* CG iterations a captured graph holds (even: buffers alternate) */
+#define ST_FIRST 12              /* iterations queued before the host first looks */
 
 struct StLevel {
     int nx, nz;
     double h;
-    double* x;     /* correction / solution of this level's system */
+    double* x;     /* correction after pre-smoothing */
+    double* xo;    /* ... after post-smoothing (the tiles read their neighbours' x) */
     double* b;     /* right-hand side */
-    double* r;     /* residual */
     double* sig;   /* diagonal term */
-    double* dpt;   /* point diffusivity */
+    double* diag;  /* sig + the face coefficients */
+    double* cs;    /* per row: coefficient of the faces to the sides, D_k / h^2 */
+    double* cd;    /* per row: of the face to the row below; cd[nz] = 0 */
 };
 
 struct bcg_steady {
@@ -51,10 +61,20 @@ struct bcg_steady {
     int nlev;
     StLevel L[ST_MAX_LEVELS];
     int n;                       /* nx * nz */
-    double *C, *q, *F, *lam, *g;
-    double *cg_r, *cg_z, *cg_p, *cg_ap;
-    double *part, *scal;         /* reduction partials, scalars */
+    int tail;                    /* first level of the one-block tail; nlev: no level fits it */
+    int nt0, ntd;                /* blocks of the level-0 tile kernels and of the direction kernel */
+    double *C, *q, *F, *g;
+    double *cg_x, *cg_r[2], *cg_p[2], *cg_ap;
+    double *part_rn, *part_rz[2], *part_pap;   /* per-block partial results, reduced in order by their readers */
+    double* scal;                /* [0] tolerance, [1] max |rhs| */
+    int* ctl;                    /* [0] done, [1] iterations, [2] their limit */
+    double* op;                  /* coarsest level's sweeps as a matrix (column-major) */
+    double* pin;                 /* pinned host staging */
+    cudaGraphExec_t graph;       /* ST_CHUNK iterations */
+    bool graph_off;
     int ncell;
+    int* start;                  /* first of each point's cells in that order (n + 1) */
+    int* order;                  /* cell of each entry */
     double* cell;                /* x, z, L, R per cell */
     int* cell_pt;                /* grid point of each cell, -1 outside the colony rows */
     double* w;
@@ -69,107 +89,460 @@ static int st_err(cudaError_t e) { if (e != cudaSuccess) { bcg_set_cuda_error(e)
 
 __device__ __forceinline__ double face_d(double a, double b) { return a == b ? a : 2.0 * a * b / (a + b); }
 
-/* ---- operator pieces on one level --------------------------------------- */
-/* (A x)_p = sum_f Df (x_p - x_nb) / h^2 + sig_p x_p for rows k >= 1; row 0
- * is the Dirichlet row (x = 0 there) */
-__device__ __forceinline__ void st_coeffs(const StLevel& L, int i, int k, double& diag, double& off_sum,
-                                          const double* x)
-{
-    const double ih2 = 1.0 / (L.h * L.h);
-    const double dp = L.dpt[k * L.nx + i];
-    diag = L.sig[k * L.nx + i];
-    off_sum = 0.0;
-    /* below (row k-1, Dirichlet when k-1 == 0: x = 0 there) */
-    {
-        double df = face_d(dp, L.dpt[(k - 1) * L.nx + i]) * ih2;
-        diag += df;
-        if (k - 1 > 0) off_sum += df * x[(k - 1) * L.nx + i];
-    }
-    if (k + 1 < L.nz) { double df = face_d(dp, L.dpt[(k + 1) * L.nx + i]) * ih2; diag += df; off_sum += df * x[(k + 1) * L.nx + i]; }
-    if (i > 0) { double df = face_d(dp, L.dpt[k * L.nx + i - 1]) * ih2; diag += df; off_sum += df * x[k * L.nx + i - 1]; }
-    if (i + 1 < L.nx) { double df = face_d(dp, L.dpt[k * L.nx + i + 1]) * ih2; diag += df; off_sum += df * x[k * L.nx + i + 1]; }
-}
+/* ---- the preconditioned CG iteration ------------------------------------- */
+/* A x = diag x - sum_f c_f x_nb on rows k >= 1; row 0 is the Dirichlet row
+ * (x = 0 there).  A row's diffusivity is constant, so the face coefficients
+ * are one value a row (cs, cd).
+ *
+ * What bounds it: a V-cycle of these grids (8 thousand to 264 thousand
+ * points, everything in L2) moves a few MB, a microsecond or two of traffic.
+ * One kernel per half-sweep made it 215 to 260 launches, 160 of them for the
+ * ten unknowns of the coarsest level: 1.0 ms a cycle at any grid size.
+ * Here a level's whole descent (four half-sweeps, residual, restriction) is one
+ * launch, and its ascent (prolongation, four half-sweeps) another, on tiles
+ * that carry a halo as wide as the sweeps reach and recompute it; the levels
+ * that fit one block's shared memory run as one launch; and the vector
+ * updates and dot products of CG ride along in the level-0 launches. */
 
-__global__ void k_st_apply(StLevel L, const double* __restrict__ x, double* __restrict__ y)
+/* sum (MAX: largest) of `np` per-block partials, the same value in every
+ * thread, in a fixed order */
+template <bool MAX, int THREADS>
+__device__ double st_total(const double* __restrict__ part, int np, double* sh)
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= L.nx * L.nz) return;
-    int i = p % L.nx, k = p / L.nx;
-    if (k == 0) { y[p] = 0.0; return; }
-    double diag, off;
-    st_coeffs(L, i, k, diag, off, x);
-    y[p] = diag * x[p] - off;
-}
-
-/* r = b - A x */
-__global__ void k_st_resid(StLevel L)
-{
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= L.nx * L.nz) return;
-    int i = p % L.nx, k = p / L.nx;
-    if (k == 0) { L.r[p] = 0.0; return; }
-    double diag, off;
-    st_coeffs(L, i, k, diag, off, L.x);
-    L.r[p] = L.b[p] - (diag * L.x[p] - off);
-}
-
-/* one colour of red-black Gauss-Seidel; nx is odd, so a point's colour
- * (i + k) & 1 is the parity of its index p = k*nx + i */
-__global__ void k_st_rbgs(StLevel L, int colour)
-{
-    int p = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + colour;
-    if (p >= L.nx * L.nz) return;
-    int i = p % L.nx, k = p / L.nx;
-    if (k == 0) return;
-    double diag, off;
-    st_coeffs(L, i, k, diag, off, L.x);
-    L.x[p] = (L.b[p] + off) / diag;
-}
-
-/* coarse b = restriction (transpose of bilinear prolongation, / 4) of fine r */
-__global__ void k_st_restrict(StLevel Lc, StLevel Lf)
-{
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= Lc.nx * Lc.nz) return;
-    int I = p % Lc.nx, K = p / Lc.nx;
-    Lc.x[p] = 0.0;
-    if (K == 0) { Lc.b[p] = 0.0; return; }
     double s = 0.0;
-    for (int dk = -1; dk <= 1; dk++) {
-        int k = 2 * K + dk;
-        if (k <= 0 || k >= Lf.nz) continue;
-        double wk = dk == 0 ? 1.0 : 0.5;
-        for (int di = -1; di <= 1; di++) {
-            int i = 2 * I + di;
-            if (i < 0 || i >= Lf.nx) continue;
-            double wi = di == 0 ? 1.0 : 0.5;
-            s += wi * wk * Lf.r[k * Lf.nx + i];
+    for (int j = threadIdx.x; j < np; j += THREADS) s = MAX ? fmax(s, part[j]) : s + part[j];
+    for (int o = 16; o >= 1; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, s, o);
+        s = MAX ? fmax(s, v) : s + v;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = sh[0];
+    for (int w = 1; w < THREADS / 32; w++) s = MAX ? fmax(s, sh[w]) : s + sh[w];
+    return s;
+}
+/* the block's own contribution, into part[blockIdx] */
+template <bool MAX, int THREADS>
+__device__ void st_partial(double s, double* part, int block, double* sh)
+{
+    for (int o = 16; o >= 1; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, s, o);
+        s = MAX ? fmax(s, v) : s + v;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = sh[0];
+        for (int w = 1; w < THREADS / 32; w++) s = MAX ? fmax(s, sh[w]) : s + sh[w];
+        part[block] = s;
+    }
+}
+
+/* the CG vectors of one iteration as the level-0 kernels see them */
+struct StCg {
+    const int* ctl;
+    const double* rin;           /* residual before the step (first: the right-hand side) */
+    double* rout;                /* ... after it */
+    const double* ap;
+    const double* p;
+    double* x;
+    const double* part_rz;       /* r.z of the step's start */
+    const double* part_pap;
+    double* part_rn;             /* max |r| after the step */
+    int n_rz, n_pap, first;
+};
+
+/* A tile is T x T points, kept with a halo as W x W in shared memory.
+ * Points off the grid and the Dirichlet row carry a zero reciprocal diagonal,
+ * so a sweep leaves them 0; the outermost ring is never updated, and what is
+ * stale there moves in one point per half-sweep. */
+template <int T> struct StTile { static constexpr int THREADS = T == 32 ? 512 : 256; };
+
+/* one half-sweep over a tile: colour (i + k) & 1, which is (li + lk) & 1 for
+ * an even tile origin and halo */
+template <int W, int THREADS>
+__device__ __forceinline__ void st_half_sweep(double* sx, const double* sb, const double* si, const double* rcs,
+                                              const double* rcd, int colour)
+{
+    for (int q = threadIdx.x; q < (W - 2) * (W / 2); q += THREADS) {
+        const int lk = 1 + q / (W / 2), li = 2 * (q % (W / 2)) + ((lk + colour) & 1);
+        if (li == 0 || li == W - 1) continue;
+        const int o = lk * W + li;
+        const double cs = rcs[lk];
+        double off = rcd[lk] * sx[o - W];
+        off += rcd[lk + 1] * sx[o + W];
+        off += cs * sx[o - 1];
+        off += cs * sx[o + 1];
+        sx[o] = (sb[o] + off) * si[o];
+    }
+}
+
+/* Descent on level L: x = two red-black sweeps from zero on b, and the
+ * restricted residual (the transpose of the bilinear prolongation, / 4) into
+ * the coarser level's b.  CG: level 0, whose b is the CG residual, stepped
+ * here (r -= alpha Ap, x += alpha p) with its max-norm.  SMOOTH = false (a
+ * one-level hierarchy): the CG step alone. */
+template <int T, bool CG, bool SMOOTH>
+__global__ void __launch_bounds__(StTile<T>::THREADS) k_st_down(StLevel L, StLevel Lc, StCg cg)
+{
+    constexpr int THREADS = StTile<T>::THREADS, HALO = SMOOTH ? 6 : 0, W = T + 2 * HALO;
+    if (cg.ctl[0]) return;
+    extern __shared__ __align__(16) unsigned char st_smem[];
+    double* sx = reinterpret_cast<double*>(st_smem);
+    double* sb = sx + W * W;
+    double* sd = sb + W * W;
+    double* si = sd + W * W;
+    double* rcs = si + W * W;
+    double* rcd = rcs + W;                   /* W + 1 */
+    __shared__ double sh[32];
+    const int i0 = blockIdx.x * T, k0 = blockIdx.y * T, nx = L.nx, nz = L.nz;
+    double alpha = 0.0;
+    if (CG && !cg.first) {
+        const double rz = st_total<false, THREADS>(cg.part_rz, cg.n_rz, sh);
+        const double pap = st_total<false, THREADS>(cg.part_pap, cg.n_pap, sh);
+        alpha = pap != 0.0 ? rz / pap : 0.0;
+    }
+    double rn = 0.0;
+    for (int q = threadIdx.x; q < W * W; q += THREADS) {
+        const int li = q % W, lk = q / W, i = i0 - HALO + li, k = k0 - HALO + lk;
+        double b = 0.0, d = 1.0, id = 0.0;
+        if (i >= 0 && i < nx && k >= 0 && k < nz) {
+            const size_t p = (size_t)k * nx + i;
+            if (CG) {
+                b = cg.rin[p];
+                if (!cg.first) b += -alpha * cg.ap[p];
+            } else b = L.b[p];
+            if (CG && li >= HALO && li < HALO + T && lk >= HALO && lk < HALO + T) {
+                rn = fmax(rn, fabs(b));
+                cg.rout[p] = b;
+                cg.x[p] = cg.first ? 0.0 : cg.x[p] + alpha * cg.p[p];
+            }
+            if (SMOOTH && k > 0) { d = L.diag[p]; id = 1.0 / d; }
+            else b = 0.0;
+        }
+        if (SMOOTH) { sx[q] = 0.0; sb[q] = b; sd[q] = d; si[q] = id; }
+    }
+    if (CG) st_partial<true, THREADS>(rn, cg.part_rn, blockIdx.y * gridDim.x + blockIdx.x, sh);
+    if constexpr (SMOOTH) {
+    for (int j = threadIdx.x; j <= W; j += THREADS) {
+        const int k = k0 - HALO + j;
+        if (j < W) rcs[j] = k >= 0 && k < nz ? L.cs[k] : 0.0;
+        rcd[j] = k >= 1 && k < nz ? L.cd[k] : 0.0;
+    }
+    __syncthreads();
+    for (int s = 0; s < 4; s++) {
+        st_half_sweep<W, THREADS>(sx, sb, si, rcs, rcd, s & 1);
+        __syncthreads();
+    }
+    /* the residual in place of b at the colour the last half-sweep left (the
+     * other's is 0 up to the rounding of its own update), one point around
+     * the tile; 0 off the grid and on the Dirichlet row */
+    for (int q = threadIdx.x; q < (T + 2) * (T + 2) / 2; q += THREADS) {
+        const int lk = HALO - 1 + q / (T / 2 + 1), li = HALO - 1 + 2 * (q % (T / 2 + 1)) + ((lk + HALO - 1) & 1), o = lk * W + li;
+        double r = 0.0;
+        if (si[o] != 0.0) {
+            double off = rcd[lk] * sx[o - W];
+            off += rcd[lk + 1] * sx[o + W];
+            off += rcs[lk] * sx[o - 1];
+            off += rcs[lk] * sx[o + 1];
+            r = sb[o] - (sd[o] * sx[o] - off);
+        }
+        sb[o] = r;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < T * T; q += THREADS) {
+        const int li = q % T, lk = q / T, i = i0 + li, k = k0 + lk;
+        if (i < nx && k < nz) L.x[(size_t)k * nx + i] = sx[(lk + HALO) * W + li + HALO];
+    }
+    for (int q = threadIdx.x; q < (T / 2) * (T / 2); q += THREADS) {
+        const int li = 2 * (q % (T / 2)), lk = 2 * (q / (T / 2)), i = i0 + li, k = k0 + lk;
+        if (i >= nx || k >= nz) continue;
+        double s = 0.0;
+        if (k > 0) {
+            const double* r = sb + (lk + HALO) * W + li + HALO;
+            s = r[0] + 0.25 * (((r[-W - 1] + r[-W + 1]) + r[W - 1]) + r[W + 1]);
+        }
+        Lc.b[(size_t)(k / 2) * Lc.nx + i / 2] = 0.25 * s;
+    }
+    }
+}
+
+/* Ascent on level L: x += bilinear prolongation of the coarser level, then
+ * two black-red sweeps, into xo.  CG: level 0, b = the CG residual, and the
+ * tile's share of r.z.  SMOOTH = false: the dot product alone (xo is there). */
+template <int T, bool CG, bool SMOOTH>
+__global__ void __launch_bounds__(StTile<T>::THREADS) k_st_up(StLevel L, StLevel Lc, const int* __restrict__ ctl,
+                                                              const double* __restrict__ r, double* part_rz)
+{
+    constexpr int THREADS = StTile<T>::THREADS, HALO = SMOOTH ? 4 : 0, W = T + 2 * HALO;
+    if (ctl[0]) return;
+    extern __shared__ __align__(16) unsigned char st_smem[];
+    double* sx = reinterpret_cast<double*>(st_smem);
+    double* sb = sx + W * W;
+    double* si = sb + W * W;
+    double* rcs = si + W * W;
+    double* rcd = rcs + W;                   /* W + 1 */
+    __shared__ double sh[32];
+    const int i0 = blockIdx.x * T, k0 = blockIdx.y * T, nx = L.nx, nz = L.nz;
+    const double* bsrc = CG ? r : L.b;
+    if (SMOOTH) {
+        for (int q = threadIdx.x; q < W * W; q += THREADS) {
+            const int i = i0 - HALO + q % W, k = k0 - HALO + q / W;
+            double x = 0.0, b = 0.0, id = 0.0;
+            if (i >= 0 && i < nx && k > 0 && k < nz) {
+                const size_t p = (size_t)k * nx + i;
+                const int I0 = i / 2, K0 = k / 2, I1 = (i & 1) ? I0 + 1 : I0, K1 = (k & 1) ? K0 + 1 : K0;
+                const double* c0 = Lc.xo + (size_t)K0 * Lc.nx;
+                const double* c1 = Lc.xo + (size_t)K1 * Lc.nx;
+                x = L.x[p] + 0.25 * (c0[I0] + c0[I1] + c1[I0] + c1[I1]);
+                b = bsrc[p];
+                id = 1.0 / L.diag[p];
+            }
+            sx[q] = x; sb[q] = b; si[q] = id;
+        }
+        for (int j = threadIdx.x; j <= W; j += THREADS) {
+            const int k = k0 - HALO + j;
+            if (j < W) rcs[j] = k >= 0 && k < nz ? L.cs[k] : 0.0;
+            rcd[j] = k >= 1 && k < nz ? L.cd[k] : 0.0;
+        }
+        __syncthreads();
+        for (int s = 0; s < 4; s++) {
+            st_half_sweep<W, THREADS>(sx, sb, si, rcs, rcd, 1 - (s & 1));
+            __syncthreads();
         }
     }
-    Lc.b[p] = 0.25 * s;
+    double rz = 0.0;
+    for (int q = threadIdx.x; q < T * T; q += THREADS) {
+        const int li = q % T, lk = q / T, i = i0 + li, k = k0 + lk;
+        if (i >= nx || k >= nz) continue;
+        const size_t p = (size_t)k * nx + i;
+        const int o = (lk + HALO) * W + li + HALO;
+        const double x = SMOOTH ? sx[o] : L.xo[p];
+        if (SMOOTH) L.xo[p] = x;
+        if (CG) rz += (SMOOTH ? sb[o] : r[p]) * x;
+    }
+    if (CG) st_partial<false, THREADS>(rz, part_rz, blockIdx.y * gridDim.x + blockIdx.x, sh);
 }
 
-/* fine x += bilinear prolongation of coarse x */
-__global__ void k_st_prolong(StLevel Lf, StLevel Lc)
+/* p = z + beta p (into the other buffer: neighbours read the old one), Ap and
+ * the block's share of p.Ap */
+__global__ void __launch_bounds__(256) k_st_direction(StLevel L, const int* __restrict__ ctl, const double* __restrict__ z,
+                                                      const double* __restrict__ pold, double* __restrict__ pnew,
+                                                      double* __restrict__ ap, const double* part_rz,
+                                                      const double* part_rz_old, int n_rz, int first_possible,
+                                                      double* part_pap)
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= Lf.nx * Lf.nz) return;
-    int i = p % Lf.nx, k = p / Lf.nx;
+    if (ctl[0]) return;
+    __shared__ double sh[32];
+    const bool first = first_possible && ctl[1] == 0;
+    double beta = 0.0;
+    if (!first) {
+        const double rz = st_total<false, 256>(part_rz, n_rz, sh), old = st_total<false, 256>(part_rz_old, n_rz, sh);
+        beta = old != 0.0 ? rz / old : 0.0;
+    }
+    const int nx = L.nx, nz = L.nz, n = nx * nz;
+    auto dir = [&](int p) -> double { return first ? z[p] : z[p] + beta * pold[p]; };
+    double s = 0.0;
+    for (int p = blockIdx.x * 256 + threadIdx.x; p < n; p += gridDim.x * 256) {
+        const int i = p % nx, k = p / nx;
+        const double c = dir(p);
+        double y = 0.0;
+        if (k > 0) {
+            const double cs = L.cs[k];
+            double off = 0.0;
+            if (k > 1) off += L.cd[k] * dir(p - nx);
+            if (k + 1 < nz) off += L.cd[k + 1] * dir(p + nx);
+            if (i > 0) off += cs * dir(p - 1);
+            if (i + 1 < nx) off += cs * dir(p + 1);
+            y = L.diag[p] * c - off;
+        }
+        pnew[p] = c;
+        ap[p] = y;
+        s += c * y;
+    }
+    st_partial<false, 256>(s, part_pap, blockIdx.x, sh);
+}
+
+/* the stopping rule on the residual the descent just left: max |r| <= tol
+ * max |rhs|, or the iteration limit; a zero right-hand side is done at once */
+template <int THREADS>
+__device__ bool st_stop(int* ctl, double* scal, const double* part_rn, int np, int first, double* sh)
+{
+    const double rn = st_total<true, THREADS>(part_rn, np, sh);
+    bool done;
+    if (first) done = rn == 0.0;
+    else done = rn <= scal[0] * scal[1] || ctl[1] + 1 >= ctl[2];
+    __syncthreads();                         /* every thread has read ctl and scal */
+    if (threadIdx.x == 0) {
+        if (first) scal[1] = rn;
+        else ctl[1] += 1;
+        if (done) ctl[0] = 1;
+    }
+    return done;
+}
+
+struct StTail { StLevel L[ST_MAX_LEVELS]; int l0, nlev, use_op; };
+
+/* Levels l0 .. nlev-1 of the V-cycle in one block's shared memory, and
+ * before them the stopping rule.  b of level l0 comes from device memory and
+ * its x goes back there.  The coarsest level's 40 + 40 symmetric sweeps are
+ * a fixed linear map of b: one matrix-vector product where it is small (its
+ * matrix is made once per linearisation by k_st_coarse_op), sweeps otherwise. */
+__global__ void __launch_bounds__(ST_TAIL_THREADS) k_st_tail(StTail t, int* ctl, double* scal, const double* part_rn,
+                                                             int np, int first, const double* __restrict__ b0,
+                                                             const double* __restrict__ op)
+{
+    constexpr int NT = ST_TAIL_THREADS;
+    if (ctl[0]) return;
+    __shared__ double sh[32];
+    extern __shared__ __align__(16) unsigned char st_smem[];
+    if (st_stop<NT>(ctl, scal, part_rn, np, first, sh)) return;
+    const int th = threadIdx.x;
+    double* base[ST_MAX_LEVELS];
+    double* mem = reinterpret_cast<double*>(st_smem);
+    /* per level: x, b, diag, reciprocal diag, rows' cs, rows' cd (nz + 1) */
+    for (int l = t.l0; l < t.nlev; l++) {
+        const StLevel& L = t.L[l];
+        const int n = L.nx * L.nz;
+        base[l] = mem;
+        double *x = mem, *b = mem + n, *d = mem + 2 * n, *id = mem + 3 * n, *cs = mem + 4 * n, *cd = cs + L.nz;
+        mem = cd + L.nz + 1;
+        for (int p = th; p < n; p += NT) {
+            const bool in = p >= L.nx;
+            const double v = in ? L.diag[p] : 1.0;
+            x[p] = 0.0; d[p] = v; id[p] = in ? 1.0 / v : 0.0;
+            b[p] = (l == t.l0 && in) ? b0[p] : 0.0;
+        }
+        for (int k = th; k <= L.nz; k += NT) { if (k < L.nz) cs[k] = L.cs[k]; cd[k] = k >= 1 && k < L.nz ? L.cd[k] : 0.0; }
+    }
+    __syncthreads();
+    auto sum4 = [&](const StLevel& L, const double* x, const double* cs, const double* cd, int i, int k, int p) {
+        double off = cd[k] * x[p - L.nx];
+        if (k + 1 < L.nz) off += cd[k + 1] * x[p + L.nx];
+        if (i > 0) off += cs[k] * x[p - 1];
+        if (i + 1 < L.nx) off += cs[k] * x[p + 1];
+        return off;
+    };
+    /* nx is odd, so a point's colour is the parity of its index */
+    auto half = [&](int l, int colour) {
+        const StLevel& L = t.L[l];
+        const int n = L.nx * L.nz;
+        double *x = base[l], *b = x + n, *id = x + 3 * n, *cs = x + 4 * n, *cd = cs + L.nz;
+        for (int p = L.nx + ((L.nx + colour) & 1) + 2 * th; p < n; p += 2 * NT) {
+            const int k = p / L.nx, i = p - k * L.nx;
+            x[p] = (b[p] + sum4(L, x, cs, cd, i, k, p)) * id[p];
+        }
+        __syncthreads();
+    };
+    const int last = t.nlev - 1;
+    for (int l = t.l0; l < last; l++) {
+        const StLevel &L = t.L[l], &Lc = t.L[l + 1];
+        const int n = L.nx * L.nz, nc = Lc.nx * Lc.nz;
+        double *x = base[l], *b = x + n, *d = x + 2 * n, *cs = x + 4 * n, *cd = cs + L.nz;
+        double* bc = base[l + 1] + nc;
+        half(l, 0); half(l, 1); half(l, 0); half(l, 1);
+        /* as in k_st_down, the residual of the colour updated last is left out */
+        for (int p = Lc.nx + th; p < nc; p += NT) {
+            const int K = p / Lc.nx, I = p - K * Lc.nx;
+            auto res = [&](int i, int k) {
+                if (i < 0 || i >= L.nx || k >= L.nz) return 0.0;
+                const int f = k * L.nx + i;
+                return b[f] - (d[f] * x[f] - sum4(L, x, cs, cd, i, k, f));
+            };
+            const double s = res(2 * I, 2 * K) + 0.25 * (((res(2 * I - 1, 2 * K - 1) + res(2 * I + 1, 2 * K - 1)) +
+                                                          res(2 * I - 1, 2 * K + 1)) + res(2 * I + 1, 2 * K + 1));
+            bc[p] = 0.25 * s;
+        }
+        __syncthreads();
+    }
+    {
+        const StLevel& L = t.L[last];
+        const int n = L.nx * L.nz, nu = n - L.nx;
+        double *x = base[last], *b = x + n;
+        if (t.use_op) {
+            if (th < nu) {
+                double s = 0.0;
+                for (int j = 0; j < nu; j++) s += op[j * nu + th] * b[L.nx + j];
+                x[L.nx + th] = s;
+            }
+            __syncthreads();
+        } else {
+            for (int j = 0; j < 40; j++) { half(last, 0); half(last, 1); }
+            for (int j = 0; j < 40; j++) { half(last, 1); half(last, 0); }
+        }
+    }
+    for (int l = last - 1; l >= t.l0; l--) {
+        const StLevel &L = t.L[l], &Lc = t.L[l + 1];
+        const int n = L.nx * L.nz;
+        double* x = base[l];
+        const double* xc = base[l + 1];
+        for (int p = L.nx + th; p < n; p += NT) {
+            const int k = p / L.nx, i = p - k * L.nx;
+            const int I0 = i / 2, K0 = k / 2, I1 = (i & 1) ? I0 + 1 : I0, K1 = (k & 1) ? K0 + 1 : K0;
+            x[p] += 0.25 * (xc[K0 * Lc.nx + I0] + xc[K0 * Lc.nx + I1] + xc[K1 * Lc.nx + I0] + xc[K1 * Lc.nx + I1]);
+        }
+        __syncthreads();
+        half(l, 1); half(l, 0); half(l, 1); half(l, 0);
+    }
+    const StLevel& L = t.L[t.l0];
+    for (int p = th; p < L.nx * L.nz; p += NT) L.xo[p] = base[t.l0][p];
+}
+
+/* The same steps where no level fits one block (a level of 3 rows or columns
+ * and thousands of the other): the stopping rule, then the coarsest level's
+ * half-sweeps, one launch each. */
+__global__ void __launch_bounds__(ST_TAIL_THREADS) k_st_check(int* ctl, double* scal, const double* part_rn, int np, int first)
+{
+    if (ctl[0]) return;
+    __shared__ double sh[32];
+    st_stop<ST_TAIL_THREADS>(ctl, scal, part_rn, np, first, sh);
+}
+__global__ void k_st_rbgs(StLevel L, const int* __restrict__ ctl, const double* __restrict__ b, int colour, int from_zero)
+{
+    const int p = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + colour;
+    if (p >= L.nx * L.nz || ctl[0]) return;
+    const int i = p % L.nx, k = p / L.nx;
     if (k == 0) return;
-    int I0 = i / 2, K0 = k / 2;
-    int I1 = (i & 1) ? I0 + 1 : I0, K1 = (k & 1) ? K0 + 1 : K0;
-    double v = 0.25 * (Lc.x[K0 * Lc.nx + I0] + Lc.x[K0 * Lc.nx + I1] + Lc.x[K1 * Lc.nx + I0] + Lc.x[K1 * Lc.nx + I1]);
-    Lf.x[p] += v;
+    double off = 0.0;
+    if (!from_zero) {                        /* the first half-sweep finds the last cycle's values */
+        if (k > 1) off += L.cd[k] * L.xo[p - L.nx];
+        if (k + 1 < L.nz) off += L.cd[k + 1] * L.xo[p + L.nx];
+        if (i > 0) off += L.cs[k] * L.xo[p - 1];
+        if (i + 1 < L.nx) off += L.cs[k] * L.xo[p + 1];
+    }
+    L.xo[p] = (b[p] + off) / L.diag[p];
 }
 
-/* coarse point diffusivity (injection) and diagonal term (weighted
- * average of the fine one over the restriction stencil) */
-__global__ void k_st_coarse_coeffs(StLevel Lc, StLevel Lf)
+/* ---- coefficients -------------------------------------------------------- */
+__global__ void k_st_begin(int* ctl, double* scal, double tol, int max_it) { ctl[0] = 0; ctl[1] = 0; ctl[2] = max_it; scal[0] = tol; }
+
+/* a level's row coefficients: row k of level l has the diffusivity of row k 2^l */
+__global__ void k_st_rows(StLevel L, int l, int nz_agar, double d_agar, double d_col)
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= Lc.nx * Lc.nz) return;
-    int I = p % Lc.nx, K = p / Lc.nx;
-    Lc.dpt[p] = Lf.dpt[(2 * K) * Lf.nx + 2 * I];
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k > L.nz) return;
+    const double ih2 = 1.0 / (L.h * L.h);
+    const double d = ((long)k << l) < nz_agar ? d_agar : d_col, dm = ((long)(k - 1) << l) < nz_agar ? d_agar : d_col;
+    if (k < L.nz) L.cs[k] = d * ih2;
+    L.cd[k] = k >= 1 && k < L.nz ? face_d(d, dm) * ih2 : 0.0;
+}
+/* sig + the coefficients of the point's faces (below, above, sides) */
+__device__ __forceinline__ double st_diag(const StLevel& L, int i, int k, double sig)
+{
+    double d = sig;
+    d += L.cd[k];
+    if (k + 1 < L.nz) d += L.cd[k + 1];
+    if (i > 0) d += L.cs[k];
+    if (i + 1 < L.nx) d += L.cs[k];
+    return d;
+}
+/* coarse diagonal term: weighted average of the fine one over the
+ * restriction stencil; and the diagonal */
+__device__ void st_coarse_point(const StLevel& Lc, const StLevel& Lf, int p)
+{
+    const int I = p % Lc.nx, K = p / Lc.nx;
     double s = 0.0, ws = 0.0;
     for (int dk = -1; dk <= 1; dk++) {
         int k = 2 * K + dk;
@@ -179,105 +552,108 @@ __global__ void k_st_coarse_coeffs(StLevel Lc, StLevel Lf)
             int i = 2 * I + di;
             if (i < 0 || i >= Lf.nx) continue;
             double wi = di == 0 ? 1.0 : 0.5;
-            s += wi * wk * Lf.sig[k * Lf.nx + i];
+            s += wi * wk * Lf.sig[(size_t)k * Lf.nx + i];
             ws += wi * wk;
         }
     }
-    Lc.sig[p] = s / ws;
+    const double sig = s / ws;
+    Lc.sig[p] = sig;
+    Lc.diag[p] = K > 0 ? st_diag(Lc, I, K, sig) : 1.0;
+}
+__global__ void k_st_coarse_coeffs(StLevel Lc, StLevel Lf)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < Lc.nx * Lc.nz) st_coarse_point(Lc, Lf, p);
+}
+/* levels l0 .. nlev-1 one after another in one block; then, where the
+ * coarsest level has at most ST_OP_MAX unknowns, the matrix of its 40 + 40
+ * sweeps: warp j runs them on the j-th unit vector */
+__global__ void __launch_bounds__(1024) k_st_coarse_rest(StTail t, double* op)
+{
+    for (int l = t.l0; l < t.nlev; l++) {
+        for (int p = threadIdx.x; p < t.L[l].nx * t.L[l].nz; p += blockDim.x) st_coarse_point(t.L[l], t.L[l - 1], p);
+        __syncthreads();
+    }
+    if (!t.use_op) return;
+    const StLevel& L = t.L[t.nlev - 1];
+    const int nx = L.nx, nu = nx * (L.nz - 1);
+    const int j = threadIdx.x >> 5, u = threadIdx.x & 31;
+    if (j >= nu) return;                     /* whole warp */
+    const int p = nx + (u < nu ? u : 0), i = p % nx, k = p / nx;
+    const bool on = u < nu;
+    const double id = on ? 1.0 / L.diag[p] : 0.0;
+    const double cs = L.cs[k], cdn = k > 1 ? L.cd[k] : 0.0, cup = k + 1 < L.nz ? L.cd[k + 1] : 0.0;
+    const double cl = i > 0 ? cs : 0.0, cr = i + 1 < nx ? cs : 0.0;
+    const double b = u == j ? 1.0 : 0.0;
+    const int colour = (nx + u) & 1;
+    double x = 0.0;
+    for (int s = 0; s < 160; s++) {
+        /* 40 x (0, 1), then 40 x (1, 0) */
+        const int c = s < 80 ? (s & 1) : 1 - (s & 1);
+        double off = cdn * __shfl_sync(0xffffffffu, x, k > 1 ? u - nx : u);
+        off += cup * __shfl_sync(0xffffffffu, x, (u + nx) & 31);
+        off += cl * __shfl_sync(0xffffffffu, x, i > 0 ? u - 1 : u);
+        off += cr * __shfl_sync(0xffffffffu, x, (u + 1) & 31);
+        if (on && colour == c) x = (b + off) * id;
+    }
+    if (on) op[j * nu + u] = x;
 }
 
 /* ---- problem-specific kernels ------------------------------------------ */
-__global__ void k_st_init(int n, int nx, int nz_agar, double d_agar, double d_col, double c0,
-                          double* dpt, double* C, double* q)
-{
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    int k = p / nx;
-    dpt[p] = k < nz_agar ? d_agar : d_col;
-    C[p] = c0;
-    q[p] = 0.0;
-}
-
-/* deposition of the cells' weighted L*R (one thread per grid point,
- * cells pre-sorted by point on the host, so the sum order is fixed) */
-__global__ void k_st_deposit(int n, double h, const int* __restrict__ start, const int* __restrict__ order,
-                             const double* __restrict__ cell, const double* __restrict__ w, double* __restrict__ q)
+/* C = c0, and the deposition of the cells' weighted L*R (one thread per grid
+ * point; bcg_steady_set_cells sorted the cells by point, so the sum order is
+ * fixed and a point's entries lie side by side) */
+__global__ void k_st_deposit(int n, double h, double c0, const int* __restrict__ start, const int* __restrict__ order,
+                             const double* __restrict__ cell, const double* __restrict__ w, double* __restrict__ q,
+                             double* __restrict__ C)
 {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     double s = 0.0;
-    for (int j = start[p]; j < start[p + 1]; j++) {
-        int c = order[j];
-        s += w[c] * cell[4 * c + 2] * cell[4 * c + 3];
+    const int e = start[p + 1];
+#pragma unroll 4
+    for (int j = start[p]; j < e; j++) {
+        const int c = order[j];
+        const double2 lr = *reinterpret_cast<const double2*>(cell + 4 * (size_t)c + 2);
+        s += w[c] * lr.x * lr.y;
     }
     q[p] = s / (h * h);
+    C[p] = c0;
 }
 
-/* F(C) (the Newton right-hand side b = F) and the linearised diagonal */
-__global__ void k_st_newton_rhs(StLevel L, const double* __restrict__ C, const double* __restrict__ q,
-                                double vmax, double km, double* __restrict__ F)
+/* F(C) (the Newton right-hand side), the linearised diagonal, and the
+ * block's max |F| */
+__global__ void __launch_bounds__(256) k_st_newton_rhs(StLevel L, const double* __restrict__ C, const double* __restrict__ q,
+                                                       double vmax, double km, double* __restrict__ F, double* part)
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= L.nx * L.nz) return;
-    int i = p % L.nx, k = p / L.nx;
-    if (k == 0) { F[p] = 0.0; L.sig[p] = 0.0; L.b[p] = 0.0; return; }
-    const double ih2 = 1.0 / (L.h * L.h);
-    const double dp = L.dpt[p];
-    double flux = 0.0;
-    flux += face_d(dp, L.dpt[p - L.nx]) * ih2 * (C[p - L.nx] - C[p]);
-    if (k + 1 < L.nz) flux += face_d(dp, L.dpt[p + L.nx]) * ih2 * (C[p + L.nx] - C[p]);
-    if (i > 0) flux += face_d(dp, L.dpt[p - 1]) * ih2 * (C[p - 1] - C[p]);
-    if (i + 1 < L.nx) flux += face_d(dp, L.dpt[p + 1]) * ih2 * (C[p + 1] - C[p]);
-    const double c = C[p];
-    const double f = flux - q[p] * vmax * c / (km + c);
-    F[p] = f;
-    L.b[p] = f;
-    L.sig[p] = q[p] * vmax * km / ((km + c) * (km + c));
-}
-
-/* deterministic dot product / max-norm: per-block partials, then one block */
-__global__ void k_st_dot_part(int n, const double* __restrict__ a, const double* __restrict__ b, double* part, int mode)
-{
-    __shared__ double sh[256];
-    double s = 0.0;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
-        s = mode == 0 ? s + a[p] * b[p] : fmax(s, fabs(a[p]));
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] = mode == 0 ? sh[threadIdx.x] + sh[threadIdx.x + o] : fmax(sh[threadIdx.x], sh[threadIdx.x + o]);
-        __syncthreads();
+    __shared__ double sh[32];
+    const int p = blockIdx.x * 256 + threadIdx.x;
+    double f = 0.0;
+    if (p < L.nx * L.nz) {
+        const int i = p % L.nx, k = p / L.nx;
+        double sig = 0.0, diag = 1.0;
+        if (k > 0) {
+            const double cs = L.cs[k], c = C[p];
+            double flux = 0.0;
+            flux += L.cd[k] * (C[p - L.nx] - c);
+            if (k + 1 < L.nz) flux += L.cd[k + 1] * (C[p + L.nx] - c);
+            if (i > 0) flux += cs * (C[p - 1] - c);
+            if (i + 1 < L.nx) flux += cs * (C[p + 1] - c);
+            f = flux - q[p] * vmax * c / (km + c);
+            sig = q[p] * vmax * km / ((km + c) * (km + c));
+            diag = st_diag(L, i, k, sig);
+        }
+        F[p] = f;
+        L.sig[p] = sig;
+        L.diag[p] = diag;
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-__global__ void k_st_dot_final(int nb, const double* part, double* out, int mode)
-{
-    __shared__ double sh[256];
-    double s = 0.0;
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) s = mode == 0 ? s + part[j] : fmax(s, part[j]);
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] = mode == 0 ? sh[threadIdx.x] + sh[threadIdx.x + o] : fmax(sh[threadIdx.x], sh[threadIdx.x + o]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = sh[0];
+    st_partial<true, 256>(fabs(f), part, blockIdx.x, sh);
 }
 
-/* y = a*x + y, or y = x + a*y (mode 1) */
-__global__ void k_st_axpy(int n, const double* __restrict__ a, int neg, const double* __restrict__ x, double* __restrict__ y, int mode)
-{
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    double s = neg ? -*a : *a;
-    y[p] = mode == 0 ? y[p] + s * x[p] : x[p] + s * y[p];
-}
-__global__ void k_st_ratio(const double* num, const double* den, double* out) { *out = *den != 0.0 ? *num / *den : 0.0; }
-__global__ void k_st_add(int n, const double* __restrict__ x, double* __restrict__ y) { int p = blockIdx.x * blockDim.x + threadIdx.x; if (p < n) y[p] += x[p]; }
 /* dst = -src, zero on the Dirichlet row */
 __global__ void k_st_neg(int n, int nx, const double* __restrict__ src, double* __restrict__ dst)
 { int p = blockIdx.x * blockDim.x + threadIdx.x; if (p < n) dst[p] = p < nx ? 0.0 : -src[p]; }
-__global__ void k_st_copy(int n, const double* __restrict__ a, double* __restrict__ b) { int p = blockIdx.x * blockDim.x + threadIdx.x; if (p < n) b[p] = a[p]; }
+__global__ void k_st_add(int n, const double* __restrict__ x, double* __restrict__ y) { int p = blockIdx.x * blockDim.x + threadIdx.x; if (p < n) y[p] += x[p]; }
 
 /* gradients: per point contributions to dL/d(d_agar, d_colony, vmax, km),
  * reduced per block in fixed order; and dL/dw per cell */
@@ -341,85 +717,151 @@ __global__ void k_st_grad_w(int ncell, double h, const double* __restrict__ cell
 /* ---- host side ---------------------------------------------------------- */
 static unsigned nblk(int n) { return (unsigned)((n + 255) / 256); }
 
-static void st_vcycle(bcg_steady* s, int l)
+/* Tile side: 32 recomputes least (a 44 x 44 box for 1024 points), 16 keeps
+ * four times the blocks busy.  32 from the size where its tiles still fill
+ * half the SMs. */
+static int st_tile(const StLevel& L)
 {
-    StLevel& L = s->L[l];
-    const int n = L.nx * L.nz;
-    if (l == s->nlev - 1) {
-        for (int j = 0; j < 40; j++) { k_st_rbgs<<<nblk((n + 1) / 2), 256, 0, s->stream>>>(L, 0); k_st_rbgs<<<nblk((n + 1) / 2), 256, 0, s->stream>>>(L, 1); }
-        for (int j = 0; j < 40; j++) { k_st_rbgs<<<nblk((n + 1) / 2), 256, 0, s->stream>>>(L, 1); k_st_rbgs<<<nblk((n + 1) / 2), 256, 0, s->stream>>>(L, 0); }
-        return;
+    return ((L.nx + 31) / 32) * ((L.nz + 31) / 32) >= 74 ? 32 : 16;
+}
+static dim3 st_tiles(const StLevel& L, int T) { return dim3((unsigned)((L.nx + T - 1) / T), (unsigned)((L.nz + T - 1) / T)); }
+static size_t st_down_smem(int T) { const int W = T + 12; return sizeof(double) * (4 * W * W + 2 * W + 1); }
+static size_t st_up_smem(int T) { const int W = T + 8; return sizeof(double) * (3 * W * W + 2 * W + 1); }
+static size_t st_tail_smem(const bcg_steady* s)
+{
+    size_t d = 0;
+    for (int l = s->tail; l < s->nlev; l++) d += 4 * (size_t)s->L[l].nx * s->L[l].nz + 2 * (size_t)s->L[l].nz + 1;
+    return d * sizeof(double);
+}
+static int st_coarsest(const bcg_steady* s) { const StLevel& L = s->L[s->nlev - 1]; return L.nx * (L.nz - 1); }
+
+template <bool CG, bool SMOOTH>
+static void st_down(bcg_steady* s, int l, const StCg& cg)
+{
+    const StLevel &L = s->L[l], &Lc = s->L[l + 1 < s->nlev ? l + 1 : l];
+    if (st_tile(L) == 32) k_st_down<32, CG, SMOOTH><<<st_tiles(L, 32), 512, SMOOTH ? st_down_smem(32) : 0, s->stream>>>(L, Lc, cg);
+    else k_st_down<16, CG, SMOOTH><<<st_tiles(L, 16), 256, SMOOTH ? st_down_smem(16) : 0, s->stream>>>(L, Lc, cg);
+}
+template <bool CG, bool SMOOTH>
+static void st_up(bcg_steady* s, int l, const double* r, double* part_rz)
+{
+    const StLevel &L = s->L[l], &Lc = s->L[l + 1 < s->nlev ? l + 1 : l];
+    if (st_tile(L) == 32) k_st_up<32, CG, SMOOTH><<<st_tiles(L, 32), 512, SMOOTH ? st_up_smem(32) : 0, s->stream>>>(L, Lc, s->ctl, r, part_rz);
+    else k_st_up<16, CG, SMOOTH><<<st_tiles(L, 16), 256, SMOOTH ? st_up_smem(16) : 0, s->stream>>>(L, Lc, s->ctl, r, part_rz);
+}
+
+/* the CG step of iteration `it` (0: the start), the stopping rule and the
+ * V-cycle on the new residual, up to z in L[0].xo and the shares of r.z */
+static void st_cycle(bcg_steady* s, const double* rhs, int it)
+{
+    const int cur = it & 1;
+    const bool first = it == 0;
+    double* r = s->cg_r[cur];
+    StCg cg = {s->ctl, first ? rhs : s->cg_r[cur ^ 1], r, s->cg_ap, s->cg_p[cur ^ 1], s->cg_x,
+               s->part_rz[cur ^ 1], s->part_pap, s->part_rn, s->nt0, s->ntd, first ? 1 : 0};
+    const bool one = s->nlev == 1;
+    if (one) st_down<true, false>(s, 0, cg); else st_down<true, true>(s, 0, cg);
+    const int down_to = s->tail < s->nlev ? s->tail : s->nlev - 1;
+    for (int l = 1; l < down_to; l++) st_down<false, true>(s, l, cg);
+    if (s->tail < s->nlev) {
+        StTail t;
+        memcpy(t.L, s->L, sizeof(t.L));
+        t.l0 = s->tail; t.nlev = s->nlev; t.use_op = st_coarsest(s) <= ST_OP_MAX;
+        k_st_tail<<<1, ST_TAIL_THREADS, st_tail_smem(s), s->stream>>>(t, s->ctl, s->scal, s->part_rn, s->nt0, first,
+                                                                      s->tail == 0 ? r : s->L[s->tail].b, s->op);
+    } else {
+        StLevel& L = s->L[s->nlev - 1];
+        const double* b = one ? r : L.b;
+        const unsigned nb = nblk((L.nx * L.nz + 1) / 2);
+        k_st_check<<<1, ST_TAIL_THREADS, 0, s->stream>>>(s->ctl, s->scal, s->part_rn, s->nt0, first);
+        for (int j = 0; j < 160; j++)
+            k_st_rbgs<<<nb, 256, 0, s->stream>>>(L, s->ctl, b, j < 80 ? (j & 1) : 1 - (j & 1), j == 0);
     }
-    for (int j = 0; j < 2; j++) { k_st_rbgs<<<nblk((n + 1) / 2), 256, 0, s->stream>>>(L, 0); k_st_rbgs<<<nblk((n + 1) / 2), 256, 0, s->stream>>>(L, 1); }
-    k_st_resid<<<nblk(n), 256, 0, s->stream>>>(L);
-    StLevel& Lc = s->L[l + 1];
-    k_st_restrict<<<nblk(Lc.nx * Lc.nz), 256, 0, s->stream>>>(Lc, L);
-    st_vcycle(s, l + 1);
-    k_st_prolong<<<nblk(n), 256, 0, s->stream>>>(L, Lc);
-    for (int j = 0; j < 2; j++) { k_st_rbgs<<<nblk((n + 1) / 2), 256, 0, s->stream>>>(L, 1); k_st_rbgs<<<nblk((n + 1) / 2), 256, 0, s->stream>>>(L, 0); }
+    for (int l = down_to - 1; l >= 1; l--) st_up<false, true>(s, l, r, nullptr);
+    if (one) st_up<true, false>(s, 0, r, s->part_rz[cur]); else st_up<true, true>(s, 0, r, s->part_rz[cur]);
 }
-
-/* z = M^-1 r with M one symmetric V-cycle from zero */
-static void st_precond(bcg_steady* s, const double* r, double* z)
+/* iteration `it` >= 1: direction, step, stopping rule, next z.  Iterations
+ * after the one that stopped do nothing. */
+static void st_iteration(bcg_steady* s, int it)
 {
-    StLevel& L = s->L[0];
-    const int n = L.nx * L.nz;
-    k_st_copy<<<nblk(n), 256, 0, s->stream>>>(n, r, L.b);
-    cudaMemsetAsync(L.x, 0, sizeof(double) * n, s->stream);
-    st_vcycle(s, 0);
-    k_st_copy<<<nblk(n), 256, 0, s->stream>>>(n, L.x, z);
+    const int cur = it & 1;
+    /* the buffers alternate: iteration it reads r, p and r.z of it - 1 */
+    k_st_direction<<<s->ntd, 256, 0, s->stream>>>(s->L[0], s->ctl, s->L[0].xo, s->cg_p[cur], s->cg_p[cur ^ 1], s->cg_ap,
+                                                  s->part_rz[cur ^ 1], s->part_rz[cur], s->nt0, 1, s->part_pap);
+    st_cycle(s, nullptr, it);
 }
-
-static int st_reduce(bcg_steady* s, const double* a, const double* b, int n, int mode, int slot)
+/* ST_CHUNK iterations, the first of them odd, as one graph launch; plain
+ * launches where no graph can be made */
+static int st_chunk(bcg_steady* s)
 {
-    k_st_dot_part<<<ST_RED_BLOCKS, 256, 0, s->stream>>>(n, a, b, s->part, mode);
-    k_st_dot_final<<<1, 256, 0, s->stream>>>(ST_RED_BLOCKS, s->part, s->scal + slot, mode);
+    if (!s->graph && !s->graph_off) {
+        cudaGraph_t g = nullptr;
+        cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) {
+            for (int j = 1; j <= ST_CHUNK; j++) st_iteration(s, j);
+            e = cudaStreamEndCapture(s->stream, &g);
+        }
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&s->graph, g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (e != cudaSuccess) { cudaGetLastError(); s->graph = nullptr; s->graph_off = true; }
+    }
+    if (s->graph) return st_err(cudaGraphLaunch(s->graph, s->stream));
+    for (int j = 1; j <= ST_CHUNK; j++) st_iteration(s, j);
     return st_err(cudaGetLastError());
 }
 
-static int st_read(bcg_steady* s, int slot, double* v)
+/* solve A x = rhs (A from the current level-0 sig/diag) by PCG to
+ * ||r||_inf <= tol * ||rhs||_inf; x in cg_x */
+static int st_pcg(bcg_steady* s, const double* rhs, double tol, int max_it, int* iters)
 {
-    ST_TRY(cudaMemcpyAsync(v, s->scal + slot, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    /* coarse diagonals for this linearisation: the large levels on their own,
+     * the smaller ones one after another in one block */
+    k_st_begin<<<1, 1, 0, s->stream>>>(s->ctl, s->scal, tol, max_it);
+    int lr = 1;
+    for (; lr < s->nlev && s->L[lr].nx * s->L[lr].nz > ST_TAIL_POINTS; lr++)
+        k_st_coarse_coeffs<<<nblk(s->L[lr].nx * s->L[lr].nz), 256, 0, s->stream>>>(s->L[lr], s->L[lr - 1]);
+    StTail t;
+    memcpy(t.L, s->L, sizeof(t.L));
+    t.l0 = lr; t.nlev = s->nlev; t.use_op = s->tail < s->nlev && st_coarsest(s) <= ST_OP_MAX;
+    k_st_coarse_rest<<<1, 1024, 0, s->stream>>>(t, s->op);
+    st_cycle(s, rhs, 0);
+    int rc = st_err(cudaGetLastError());
+    volatile int* h = reinterpret_cast<volatile int*>(s->pin);
+    for (int done = 0, queue = ST_FIRST; !rc && !done; queue = ST_CHUNK) {
+        for (int j = 0; j < queue && !rc; j += ST_CHUNK) rc = st_chunk(s);
+        if (rc) break;
+        ST_TRY(cudaMemcpyAsync(s->pin, s->ctl, 2 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+        ST_TRY(cudaStreamSynchronize(s->stream));
+        done = h[0];
+        *iters = h[1];
+    }
+    return rc;
+}
+
+/* max |F| at C, with F, sig and the diagonal left on the device */
+static int st_newton_rhs(bcg_steady* s, double vmax, double km, double* fn)
+{
+    const int nb = (int)nblk(s->n);
+    k_st_newton_rhs<<<nb, 256, 0, s->stream>>>(s->L[0], s->C, s->q, vmax, km, s->F, s->part_rn);
+    ST_TRY(cudaGetLastError());
+    if (!fn) return BCG_OK;
+    ST_TRY(cudaMemcpyAsync(s->pin, s->part_rn, sizeof(double) * nb, cudaMemcpyDeviceToHost, s->stream));
     ST_TRY(cudaStreamSynchronize(s->stream));
+    double m = 0.0;
+    for (int b = 0; b < nb; b++) m = fmax(m, s->pin[b]);
+    *fn = m;
     return BCG_OK;
 }
 
-/* solve A x = rhs (A from the current level-0 sig/dpt) by PCG to
- * ||r||_inf <= tol * ||rhs||_inf; x in L[0]-sized buffer `x` */
-static int st_pcg(bcg_steady* s, const double* rhs, double* x, double tol, int max_it, int* iters)
+static int st_attributes()
 {
-    StLevel& L = s->L[0];
-    const int n = L.nx * L.nz;
-    /* coarse diagonals for this linearisation */
-    for (int l = 1; l < s->nlev; l++)
-        k_st_coarse_coeffs<<<nblk(s->L[l].nx * s->L[l].nz), 256, 0, s->stream>>>(s->L[l], s->L[l - 1]);
-    cudaMemsetAsync(x, 0, sizeof(double) * n, s->stream);
-    k_st_copy<<<nblk(n), 256, 0, s->stream>>>(n, rhs, s->cg_r);
-    int rc;
-    double bnorm;
-    if ((rc = st_reduce(s, rhs, rhs, n, 1, 0)) || (rc = st_read(s, 0, &bnorm))) return rc;
-    *iters = 0;
-    if (bnorm == 0.0) return BCG_OK;
-    st_precond(s, s->cg_r, s->cg_z);
-    k_st_copy<<<nblk(n), 256, 0, s->stream>>>(n, s->cg_z, s->cg_p);
-    if ((rc = st_reduce(s, s->cg_r, s->cg_z, n, 0, 1))) return rc;        /* rz */
-    for (int it = 1; it <= max_it; it++) {
-        k_st_apply<<<nblk(n), 256, 0, s->stream>>>(L, s->cg_p, s->cg_ap);
-        if ((rc = st_reduce(s, s->cg_p, s->cg_ap, n, 0, 2))) return rc;   /* pAp */
-        k_st_ratio<<<1, 1, 0, s->stream>>>(s->scal + 1, s->scal + 2, s->scal + 3);   /* alpha */
-        k_st_axpy<<<nblk(n), 256, 0, s->stream>>>(n, s->scal + 3, 0, s->cg_p, x, 0);
-        k_st_axpy<<<nblk(n), 256, 0, s->stream>>>(n, s->scal + 3, 1, s->cg_ap, s->cg_r, 0);
-        double rn;
-        if ((rc = st_reduce(s, s->cg_r, s->cg_r, n, 1, 4)) || (rc = st_read(s, 4, &rn))) return rc;
-        *iters = it;
-        if (rn <= tol * bnorm) break;
-        st_precond(s, s->cg_r, s->cg_z);
-        if ((rc = st_reduce(s, s->cg_r, s->cg_z, n, 0, 5))) return rc;   /* rz new */
-        k_st_ratio<<<1, 1, 0, s->stream>>>(s->scal + 5, s->scal + 1, s->scal + 6);   /* beta */
-        k_st_copy<<<1, 1, 0, s->stream>>>(1, s->scal + 5, s->scal + 1);
-        k_st_axpy<<<nblk(n), 256, 0, s->stream>>>(n, s->scal + 6, 0, s->cg_z, s->cg_p, 1);   /* p = z + beta p */
-    }
-    return st_err(cudaGetLastError());
+    /* set on every creation: attributes belong to the current device */
+#define ST_SMEM(k, b) if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(b)) != cudaSuccess) return BCG_E_CUDA
+    ST_SMEM((k_st_down<32, true, true>), st_down_smem(32));
+    ST_SMEM((k_st_down<32, false, true>), st_down_smem(32));
+    ST_SMEM(k_st_tail, 220 * 1024);
+#undef ST_SMEM
+    return BCG_OK;
 }
 
 extern "C" int bcg_steady_create(const bcg_steady_params* p, bcg_steady** out)
@@ -444,23 +886,48 @@ extern "C" int bcg_steady_create(const bcg_steady_params* p, bcg_steady** out)
         StLevel& L = s->L[s->nlev];
         L.nx = nx; L.nz = nz; L.h = h;
         size_t b = sizeof(double) * (size_t)nx * nz;
-        ST_ALLOC(L.x, b); ST_ALLOC(L.b, b); ST_ALLOC(L.r, b); ST_ALLOC(L.sig, b); ST_ALLOC(L.dpt, b);
+        ST_ALLOC(L.x, b); ST_ALLOC(L.xo, b); ST_ALLOC(L.b, b); ST_ALLOC(L.sig, b); ST_ALLOC(L.diag, b);
+        ST_ALLOC(L.cs, sizeof(double) * (nz + 1)); ST_ALLOC(L.cd, sizeof(double) * (nz + 1));
+        /* the Dirichlet row, which no kernel writes everywhere, is 0 */
+        if (!rc) rc = st_err(cudaMemsetAsync(L.xo, 0, b, s->stream));
         s->nlev++;
         if (nx <= 3 || nz <= 3) break;
         nx = (nx + 1) / 2; nz = (nz + 1) / 2; h *= 2;
     }
     s->n = p->nx * p->nz;
     size_t b = sizeof(double) * (size_t)s->n;
-    ST_ALLOC(s->C, b); ST_ALLOC(s->q, b); ST_ALLOC(s->F, b); ST_ALLOC(s->lam, b); ST_ALLOC(s->g, b);
-    ST_ALLOC(s->cg_r, b); ST_ALLOC(s->cg_z, b); ST_ALLOC(s->cg_p, b); ST_ALLOC(s->cg_ap, b);
-    ST_ALLOC(s->part, sizeof(double) * ST_RED_BLOCKS);
+    /* the largest set of levels, from the coarsest up, that fits the tail */
+    s->tail = s->nlev;
+    for (int l = s->nlev - 1, pts = 0; l >= (s->nlev > 1 ? 1 : 0); l--) {
+        pts += s->L[l].nx * s->L[l].nz + s->L[l].nz / 2 + 1;
+        if (pts > ST_TAIL_POINTS) break;
+        s->tail = l;
+    }
+    {
+        const dim3 t0 = st_tiles(s->L[0], st_tile(s->L[0]));
+        s->nt0 = (int)(t0.x * t0.y);
+        s->ntd = (int)nblk(s->n) < 592 ? (int)nblk(s->n) : 592;     /* 4 blocks an SM */
+    }
+    const size_t np = (size_t)(s->nt0 > (int)nblk(s->n) ? s->nt0 : (int)nblk(s->n));
+    ST_ALLOC(s->C, b); ST_ALLOC(s->q, b); ST_ALLOC(s->F, b); ST_ALLOC(s->g, b);
+    ST_ALLOC(s->cg_x, b); ST_ALLOC(s->cg_ap, b);
+    for (int j = 0; j < 2; j++) { ST_ALLOC(s->cg_r[j], b); ST_ALLOC(s->cg_p[j], b); ST_ALLOC(s->part_rz[j], sizeof(double) * np); }
+    ST_ALLOC(s->part_rn, sizeof(double) * np);
+    ST_ALLOC(s->part_pap, sizeof(double) * np);
     ST_ALLOC(s->scal, sizeof(double) * 16);
+    ST_ALLOC(s->ctl, sizeof(int) * 16);
+    ST_ALLOC(s->op, sizeof(double) * ST_OP_MAX * ST_OP_MAX);
     ST_ALLOC(s->gpart, sizeof(double) * 4 * ST_RED_BLOCKS);
+    ST_ALLOC(s->start, sizeof(int) * ((size_t)s->n + 1));
+    if (!rc) rc = st_err(cudaMemsetAsync(s->start, 0, sizeof(int) * ((size_t)s->n + 1), s->stream));
+    if (!rc) rc = st_err(cudaMallocHost((void**)&s->pin, sizeof(double) * (np > 4 * ST_RED_BLOCKS ? np : 4 * ST_RED_BLOCKS)));
     int mc = p->max_cells > 0 ? p->max_cells : 1;
     ST_ALLOC(s->cell, sizeof(double) * 4 * mc);
     ST_ALLOC(s->cell_pt, sizeof(int) * mc);
     ST_ALLOC(s->w, sizeof(double) * mc);
     ST_ALLOC(s->gw, sizeof(double) * mc);
+    ST_ALLOC(s->order, sizeof(int) * mc);
+    if (!rc) rc = st_attributes();
 #undef ST_ALLOC
     if (rc) { bcg_steady_destroy(s); return rc; }
     *out = s;
@@ -471,10 +938,17 @@ extern "C" int bcg_steady_destroy(bcg_steady* s)
 {
     if (!s) return BCG_OK;
     if (s->stream) cudaStreamSynchronize(s->stream);
-    for (int l = 0; l < s->nlev; l++) { cudaFree(s->L[l].x); cudaFree(s->L[l].b); cudaFree(s->L[l].r); cudaFree(s->L[l].sig); cudaFree(s->L[l].dpt); }
-    void* ptrs[] = {s->C, s->q, s->F, s->lam, s->g, s->cg_r, s->cg_z, s->cg_p, s->cg_ap, s->part, s->scal, s->gpart,
-                    s->cell, s->cell_pt, s->w, s->gw};
+    for (int l = 0; l < s->nlev; l++) { 
+        StLevel& L = s->L[l];
+        void* lv[] = {L.x, L.xo, L.b, L.sig, L.diag, L.cs, L.cd};
+        for (void* q : lv) if (q) cudaFree(q);
+    }
+    void* ptrs[] = {s->C, s->q, s->F, s->g, s->cg_x, s->cg_r[0], s->cg_r[1], s->cg_p[0], s->cg_p[1], s->cg_ap, s->part_rn,
+                    s->part_rz[0], s->part_rz[1], s->part_pap, s->scal, s->ctl, s->op, s->gpart,
+                    s->cell, s->cell_pt, s->w, s->gw, s->start, s->order};
     for (void* q : ptrs) if (q) cudaFree(q);
+    if (s->graph) cudaGraphExecDestroy(s->graph);
+    if (s->pin) cudaFreeHost(s->pin);
     if (s->stream) cudaStreamDestroy(s->stream);
     free(s);
     return BCG_OK;
@@ -487,36 +961,23 @@ extern "C" int bcg_steady_set_cells(bcg_steady* s, const double* xzlr, int ncell
     if (!s || ncell < 0 || ncell > s->P.max_cells || (ncell > 0 && !xzlr)) return BCG_E_ARG;
     s->ncell = ncell;
     s->solved = false;
-    if (ncell == 0) return BCG_OK;
-    ST_TRY(cudaMemcpy(s->cell, xzlr, sizeof(double) * 4 * (size_t)ncell, cudaMemcpyHostToDevice));
-    std::vector<int> pt(ncell);
-    const int nx = s->P.nx, nz = s->P.nz;
+    /* the cells of each grid point, in the order given (a counting sort) */
+    const int nx = s->P.nx, nz = s->P.nz, n = s->n;
+    std::vector<int> pt(ncell), start((size_t)n + 1, 0), order(ncell);
     for (int c = 0; c < ncell; c++) {
         long i = lround(xzlr[4 * c] / s->P.h), k = lround(xzlr[4 * c + 1] / s->P.h);
         pt[c] = (i >= 0 && i < nx && k >= s->P.nz_agar && k < nz) ? (int)(k * nx + i) : -1;
+        if (pt[c] >= 0) start[pt[c] + 1]++;
     }
-    ST_TRY(cudaMemcpy(s->cell_pt, pt.data(), sizeof(int) * ncell, cudaMemcpyHostToDevice));
-    return BCG_OK;
-}
-
-static int st_deposit(bcg_steady* s, const double* w_host)
-{
-    const int n = s->n, nc = s->ncell;
-    std::vector<int> pt(nc), start(n + 1, 0), order(nc);
-    if (nc) ST_TRY(cudaMemcpy(pt.data(), s->cell_pt, sizeof(int) * nc, cudaMemcpyDeviceToHost));
-    for (int c = 0; c < nc; c++) if (pt[c] >= 0) start[pt[c] + 1]++;
     for (int p = 0; p < n; p++) start[p + 1] += start[p];
     std::vector<int> fill(start.begin(), start.end() - 1);
-    for (int c = 0; c < nc; c++) if (pt[c] >= 0) order[fill[pt[c]]++] = c;
-    int *d_start = nullptr, *d_order = nullptr;
-    ST_TRY(cudaMallocAsync((void**)&d_start, sizeof(int) * (n + 1), s->stream));
-    ST_TRY(cudaMallocAsync((void**)&d_order, sizeof(int) * (nc > 0 ? nc : 1), s->stream));
-    ST_TRY(cudaMemcpyAsync(d_start, start.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s->stream));
-    if (nc) ST_TRY(cudaMemcpyAsync(d_order, order.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, s->stream));
-    if (nc) ST_TRY(cudaMemcpyAsync(s->w, w_host, sizeof(double) * nc, cudaMemcpyHostToDevice, s->stream));
-    k_st_deposit<<<nblk(n), 256, 0, s->stream>>>(n, s->P.h, d_start, d_order, s->cell, s->w, s->q);
-    cudaFreeAsync(d_start, s->stream);
-    cudaFreeAsync(d_order, s->stream);
+    for (int c = 0; c < ncell; c++) if (pt[c] >= 0) order[fill[pt[c]]++] = c;
+    ST_TRY(cudaMemcpyAsync(s->start, start.data(), sizeof(int) * ((size_t)n + 1), cudaMemcpyHostToDevice, s->stream));
+    if (ncell) {
+        ST_TRY(cudaMemcpyAsync(s->order, order.data(), sizeof(int) * ncell, cudaMemcpyHostToDevice, s->stream));
+        ST_TRY(cudaMemcpyAsync(s->cell_pt, pt.data(), sizeof(int) * ncell, cudaMemcpyHostToDevice, s->stream));
+        ST_TRY(cudaMemcpyAsync(s->cell, xzlr, sizeof(double) * 4 * (size_t)ncell, cudaMemcpyHostToDevice, s->stream));
+    }
     ST_TRY(cudaStreamSynchronize(s->stream));
     return BCG_OK;
 }
@@ -528,28 +989,25 @@ extern "C" int bcg_steady_solve(bcg_steady* s, const double* theta, const double
     const double d_agar = theta[0], d_col = theta[1], vmax = theta[2], km = theta[3];
     if (!(d_agar > 0) || !(d_col > 0) || !(km > 0) || !(tol > 0)) return BCG_E_ARG;
     const int n = s->n;
-    StLevel& L = s->L[0];
-    k_st_init<<<nblk(n), 256, 0, s->stream>>>(n, s->P.nx, s->P.nz_agar, d_agar, d_col, s->P.c0, L.dpt, s->C, s->q);
-    for (int l = 1; l < s->nlev; l++)
-        k_st_coarse_coeffs<<<nblk(s->L[l].nx * s->L[l].nz), 256, 0, s->stream>>>(s->L[l], s->L[l - 1]);
-    int rc = st_deposit(s, w);
-    if (rc) return rc;
-    int it = 0, cgt = 0;
+    for (int l = 0; l < s->nlev; l++)
+        k_st_rows<<<nblk(s->L[l].nz + 1), 256, 0, s->stream>>>(s->L[l], l, s->P.nz_agar, d_agar, d_col);
+    if (s->ncell) ST_TRY(cudaMemcpyAsync(s->w, w, sizeof(double) * s->ncell, cudaMemcpyHostToDevice, s->stream));
+    k_st_deposit<<<nblk(n), 256, 0, s->stream>>>(n, s->P.h, s->P.c0, s->start, s->order, s->cell, s->w, s->q, s->C);
+    int it = 0, cgt = 0, rc;
     double f0 = 0.0;
     for (; it < 50; it++) {
-        k_st_newton_rhs<<<nblk(n), 256, 0, s->stream>>>(L, s->C, s->q, vmax, km, s->F);
         double fn;
-        if ((rc = st_reduce(s, s->F, s->F, n, 1, 7)) || (rc = st_read(s, 7, &fn))) return rc;
+        if ((rc = st_newton_rhs(s, vmax, km, &fn))) return rc;
         if (it == 0) f0 = fn > 0 ? fn : 1.0;
         if (fn <= tol * f0 || fn == 0.0) break;
         int ci = 0;
         const double cg_tol = tol < 1e-8 ? (tol > 1e-14 ? tol : 1e-14) : 1e-8;
-        if ((rc = st_pcg(s, s->F, s->g, cg_tol, 200, &ci))) return rc;
+        if ((rc = st_pcg(s, s->F, cg_tol, 200, &ci))) return rc;
         cgt += ci;
-        k_st_add<<<nblk(n), 256, 0, s->stream>>>(n, s->g, s->C);   /* C += delta */
+        k_st_add<<<nblk(n), 256, 0, s->stream>>>(n, s->cg_x, s->C);   /* C += delta */
     }
-    /* keep the converged linearisation (sig, coarse diagonals) for the adjoint */
-    k_st_newton_rhs<<<nblk(n), 256, 0, s->stream>>>(L, s->C, s->q, vmax, km, s->F);
+    /* keep the converged linearisation for the adjoint */
+    if ((rc = st_newton_rhs(s, vmax, km, nullptr))) return rc;
     s->solved = true;
     memcpy(s->theta, theta, sizeof(s->theta));
     if (C_out) ST_TRY(cudaMemcpyAsync(C_out, s->C, sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream));
@@ -563,25 +1021,23 @@ extern "C" int bcg_steady_vjp(bcg_steady* s, const double* dL_dC, double* grad_t
 {
     if (!s || !dL_dC || !grad_theta || !s->solved || !(tol > 0)) return BCG_E_ARG;
     const int n = s->n;
-    StLevel& L = s->L[0];
     /* A lambda = -dL/dC (row 0 is fixed: no adjoint there) */
     ST_TRY(cudaMemcpyAsync(s->cg_ap, dL_dC, sizeof(double) * n, cudaMemcpyHostToDevice, s->stream));
     k_st_neg<<<nblk(n), 256, 0, s->stream>>>(n, s->P.nx, s->cg_ap, s->g);   /* g = -dL/dC, 0 on row 0 */
     int ci = 0;
-    int rc = st_pcg(s, s->g, s->lam, tol, 500, &ci);
+    int rc = st_pcg(s, s->g, tol, 500, &ci);
     if (rc) return rc;
     const double* th = s->theta;
-    k_st_grad_part<<<ST_RED_BLOCKS, 256, 0, s->stream>>>(L, s->P.nz_agar, th[0], th[1], s->C, s->q, s->lam, th[2], th[3], s->gpart);
-    std::vector<double> gp(4 * ST_RED_BLOCKS);
-    ST_TRY(cudaMemcpyAsync(gp.data(), s->gpart, sizeof(double) * gp.size(), cudaMemcpyDeviceToHost, s->stream));
+    k_st_grad_part<<<ST_RED_BLOCKS, 256, 0, s->stream>>>(s->L[0], s->P.nz_agar, th[0], th[1], s->C, s->q, s->cg_x, th[2], th[3], s->gpart);
+    ST_TRY(cudaMemcpyAsync(s->pin, s->gpart, sizeof(double) * 4 * ST_RED_BLOCKS, cudaMemcpyDeviceToHost, s->stream));
     if (grad_w && s->ncell > 0) {
-        k_st_grad_w<<<nblk(s->ncell), 256, 0, s->stream>>>(s->ncell, s->P.h, s->cell, s->cell_pt, s->C, s->lam, th[2], th[3], s->gw);
+        k_st_grad_w<<<nblk(s->ncell), 256, 0, s->stream>>>(s->ncell, s->P.h, s->cell, s->cell_pt, s->C, s->cg_x, th[2], th[3], s->gw);
         ST_TRY(cudaMemcpyAsync(grad_w, s->gw, sizeof(double) * s->ncell, cudaMemcpyDeviceToHost, s->stream));
     }
     ST_TRY(cudaStreamSynchronize(s->stream));
     for (int j = 0; j < 4; j++) {
         double t = 0.0;
-        for (int b = 0; b < ST_RED_BLOCKS; b++) t += gp[4 * b + j];
+        for (int b = 0; b < ST_RED_BLOCKS; b++) t += s->pin[4 * b + j];
         grad_theta[j] = t;
     }
     return BCG_OK;
