@@ -35,8 +35,10 @@
 #define ST_MAX_LEVELS 12
 #define ST_RED_BLOCKS 256
 /* points of the levels the one-block tail of the V-cycle holds in shared
- * memory (32 B each: x, b, the diagonal and its reciprocal) */
+ * memory (32 B each: x, b, the reciprocal diagonal, neighbour sums) */
 #define ST_TAIL_POINTS 6400
+/* points a half-sweep updates on the levels one warp of the tail runs alone */
+#define ST_WARP_POINTS 96
 #define ST_TAIL_THREADS 512
 /* unknowns of the coarsest level up to which its sweeps run as one matrix */
 #define ST_OP_MAX 32
@@ -51,6 +53,7 @@ struct StLevel {
     double* b;     /* right-hand side */
     double* sig;   /* diagonal term */
     double* diag;  /* sig + the face coefficients */
+    double* id;    /* 1 / diag, 0 on the Dirichlet row */
     double* cs;    /* per row: coefficient of the faces to the sides, D_k / h^2 */
     double* cd;    /* per row: of the face to the row below; cd[nz] = 0 */
 };
@@ -69,6 +72,7 @@ struct bcg_steady {
     double* scal;                /* [0] tolerance, [1] max |rhs| */
     int* ctl;                    /* [0] done, [1] iterations, [2] their limit */
     double* op;                  /* coarsest level's sweeps as a matrix (column-major) */
+    double* image;               /* the tail's coefficients as it keeps them */
     double* pin;                 /* pinned host staging */
     cudaGraphExec_t graph;       /* ST_CHUNK iterations */
     bool graph_off;
@@ -102,7 +106,11 @@ __device__ __forceinline__ double face_d(double a, double b) { return a == b ? a
  * launch, and its ascent (prolongation, four half-sweeps) another, on tiles
  * that carry a halo as wide as the sweeps reach and recompute it; the levels
  * that fit one block's shared memory run as one launch; and the vector
- * updates and dot products of CG ride along in the level-0 launches. */
+ * updates and dot products of CG ride along in the level-0 launches.
+ * Measured, device time of one CG iteration with its V-cycle: 129 x 65 points
+ * 38 us (tail 22, descent 6.5, ascent 5.1, direction 4.2), 513 x 257 points
+ * 68 us, each 1000 us before.  What bounds it now is the chain of dependent
+ * phases: the tail's 50 (5 levels), about 0.35 us each. */
 
 /* sum (MAX: largest) of `np` per-block partials, the same value in every
  * thread, in a fixed order */
@@ -121,6 +129,23 @@ __device__ double st_total(const double* __restrict__ part, int np, double* sh)
     s = sh[0];
     for (int w = 1; w < THREADS / 32; w++) s = MAX ? fmax(s, sh[w]) : s + sh[w];
     return s;
+}
+/* two sums at once */
+template <int THREADS>
+__device__ void st_total2(const double* __restrict__ pa, int na, const double* __restrict__ pb, int nb, double* sh,
+                          double& ta, double& tb)
+{
+    double a = 0.0, b = 0.0;
+    for (int j = threadIdx.x; j < na || j < nb; j += THREADS) {
+        const double va = j < na ? pa[j] : 0.0, vb = j < nb ? pb[j] : 0.0;
+        a += va; b += vb;
+    }
+    for (int o = 16; o >= 1; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); b += __shfl_xor_sync(0xffffffffu, b, o); }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) { sh[threadIdx.x >> 5] = a; sh[32 + (threadIdx.x >> 5)] = b; }
+    __syncthreads();
+    ta = sh[0]; tb = sh[32];
+    for (int w = 1; w < THREADS / 32; w++) { ta += sh[w]; tb += sh[32 + w]; }
 }
 /* the block's own contribution, into part[blockIdx] */
 template <bool MAX, int THREADS>
@@ -154,28 +179,40 @@ struct StCg {
     int n_rz, n_pap, first;
 };
 
-/* A tile is T x T points, kept with a halo as W x W in shared memory.
+/* A tile is T x T points, kept with a halo as W x W in shared memory, the two
+ * colours in separate halves (entry j of row lk of colour c is column
+ * 2 j + ((lk + c) & 1)): a half-sweep then reads whole rows of entries side
+ * by side, where one array would cost every access twice the bank cycles.
  * Points off the grid and the Dirichlet row carry a zero reciprocal diagonal,
  * so a sweep leaves them 0; the outermost ring is never updated, and what is
  * stale there moves in one point per half-sweep. */
 template <int T> struct StTile { static constexpr int THREADS = T == 32 ? 512 : 256; };
 
+/* neighbours' part of A x at one point, and the Gauss-Seidel update from it:
+ * two short chains of multiply-adds */
+__device__ __forceinline__ double st_off(double cs, double cd, double cu, double l, double r, double d, double u)
+{
+    return fma(cs, l + r, fma(cd, d, cu * u));
+}
+/* where column li, row lk of a W-wide tile is kept */
+template <int W> __device__ __forceinline__ int st_at(int li, int lk) { return ((li + lk) & 1) * (W * W / 2) + lk * (W / 2) + (li >> 1); }
 /* one half-sweep over a tile: colour (i + k) & 1, which is (li + lk) & 1 for
- * an even tile origin and halo */
-template <int W, int THREADS>
-__device__ __forceinline__ void st_half_sweep(double* sx, const double* sb, const double* si, const double* rcs,
+ * an even tile origin and halo.  KEEP: the point's neighbour sum takes the
+ * place of its b (see the residual). */
+template <int W, int THREADS, bool KEEP>
+__device__ __forceinline__ void st_half_sweep(double* sx, double* sb, const double* si, const double* rcs,
                                               const double* rcd, int colour)
 {
-    for (int q = threadIdx.x; q < (W - 2) * (W / 2); q += THREADS) {
-        const int lk = 1 + q / (W / 2), li = 2 * (q % (W / 2)) + ((lk + colour) & 1);
-        if (li == 0 || li == W - 1) continue;
-        const int o = lk * W + li;
-        const double cs = rcs[lk];
-        double off = rcd[lk] * sx[o - W];
-        off += rcd[lk + 1] * sx[o + W];
-        off += cs * sx[o - 1];
-        off += cs * sx[o + 1];
-        sx[o] = (sb[o] + off) * si[o];
+    constexpr int HW = W / 2;
+    const double* other = sx + (1 - colour) * (W * HW);
+    const int own = colour * (W * HW);
+#pragma unroll
+    for (int q = threadIdx.x; q < (W - 2) * HW; q += THREADS) {
+        const int lk = 1 + q / HW, j = q % HW, par = (lk + colour) & 1, o = lk * HW + j;
+        if (par ? j == HW - 1 : j == 0) continue;          /* the ring */
+        const double off = st_off(rcs[lk], rcd[lk], rcd[lk + 1], other[o - 1 + par], other[o + par], other[o - HW], other[o + HW]);
+        sx[own + o] = (sb[own + o] + off) * si[own + o];
+        if (KEEP) sb[own + o] = off;
     }
 }
 
@@ -188,84 +225,101 @@ template <int T, bool CG, bool SMOOTH>
 __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_down(StLevel L, StLevel Lc, StCg cg)
 {
     constexpr int THREADS = StTile<T>::THREADS, HALO = SMOOTH ? 6 : 0, W = T + 2 * HALO;
-    if (cg.ctl[0]) return;
+    constexpr int PER = (W * W + THREADS - 1) / THREADS;
     extern __shared__ __align__(16) unsigned char st_smem[];
     double* sx = reinterpret_cast<double*>(st_smem);
     double* sb = sx + W * W;
-    double* sd = sb + W * W;
-    double* si = sd + W * W;
+    double* si = sb + W * W;
     double* rcs = si + W * W;
     double* rcd = rcs + W;                   /* W + 1 */
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     const int i0 = blockIdx.x * T, k0 = blockIdx.y * T, nx = L.nx, nz = L.nz;
+    const int done = cg.ctl[0];
+    /* every load is under way before anything waits for one */
+    double b[PER], a[PER], id[PER], pv[PER], xv[PER];
+    const bool step = CG && !cg.first;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int q = threadIdx.x + j * THREADS, li = q % W, lk = q / W, i = i0 - HALO + li, k = k0 - HALO + lk;
+        b[j] = a[j] = id[j] = pv[j] = xv[j] = 0.0;
+        if (q < W * W && i >= 0 && i < nx && k >= 0 && k < nz) {
+            const size_t p = (size_t)k * nx + i;
+            b[j] = CG ? cg.rin[p] : L.b[p];
+            if (SMOOTH) id[j] = L.id[p];
+            if (step) {
+                a[j] = cg.ap[p];
+                if (li >= HALO && li < HALO + T && lk >= HALO && lk < HALO + T) { pv[j] = cg.p[p]; xv[j] = cg.x[p]; }
+            }
+        }
+    }
+    double c1 = 0.0, c2 = 0.0;
+    if (SMOOTH && threadIdx.x <= W) {
+        const int k = k0 - HALO + threadIdx.x;
+        c1 = k >= 0 && k < nz ? L.cs[k] : 0.0;
+        c2 = k >= 1 && k < nz ? L.cd[k] : 0.0;
+    }
+    if (done) return;
+    if (SMOOTH && threadIdx.x <= W) {
+        if (threadIdx.x < W) rcs[threadIdx.x] = c1;
+        rcd[threadIdx.x] = c2;
+    }
     double alpha = 0.0;
-    if (CG && !cg.first) {
-        const double rz = st_total<false, THREADS>(cg.part_rz, cg.n_rz, sh);
-        const double pap = st_total<false, THREADS>(cg.part_pap, cg.n_pap, sh);
+    if (step) {
+        double rz, pap;
+        st_total2<THREADS>(cg.part_rz, cg.n_rz, cg.part_pap, cg.n_pap, sh, rz, pap);
         alpha = pap != 0.0 ? rz / pap : 0.0;
     }
     double rn = 0.0;
-    for (int q = threadIdx.x; q < W * W; q += THREADS) {
-        const int li = q % W, lk = q / W, i = i0 - HALO + li, k = k0 - HALO + lk;
-        double b = 0.0, d = 1.0, id = 0.0;
-        if (i >= 0 && i < nx && k >= 0 && k < nz) {
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int q = threadIdx.x + j * THREADS, li = q % W, lk = q / W, i = i0 - HALO + li, k = k0 - HALO + lk;
+        if (q >= W * W) continue;
+        if (step) b[j] += -alpha * a[j];
+        if (CG && li >= HALO && li < HALO + T && lk >= HALO && lk < HALO + T && i < nx && k < nz) {
             const size_t p = (size_t)k * nx + i;
-            if (CG) {
-                b = cg.rin[p];
-                if (!cg.first) b += -alpha * cg.ap[p];
-            } else b = L.b[p];
-            if (CG && li >= HALO && li < HALO + T && lk >= HALO && lk < HALO + T) {
-                rn = fmax(rn, fabs(b));
-                cg.rout[p] = b;
-                cg.x[p] = cg.first ? 0.0 : cg.x[p] + alpha * cg.p[p];
-            }
-            if (SMOOTH && k > 0) { d = L.diag[p]; id = 1.0 / d; }
-            else b = 0.0;
+            rn = fmax(rn, fabs(b[j]));
+            cg.rout[p] = b[j];
+            cg.x[p] = step ? xv[j] + alpha * pv[j] : 0.0;
         }
-        if (SMOOTH) { sx[q] = 0.0; sb[q] = b; sd[q] = d; si[q] = id; }
+        if (SMOOTH) { const int o = st_at<W>(li, lk); sx[o] = 0.0; sb[o] = b[j]; si[o] = id[j]; }
     }
     if (CG) st_partial<true, THREADS>(rn, cg.part_rn, blockIdx.y * gridDim.x + blockIdx.x, sh);
     if constexpr (SMOOTH) {
-    for (int j = threadIdx.x; j <= W; j += THREADS) {
-        const int k = k0 - HALO + j;
-        if (j < W) rcs[j] = k >= 0 && k < nz ? L.cs[k] : 0.0;
-        rcd[j] = k >= 1 && k < nz ? L.cd[k] : 0.0;
-    }
-    __syncthreads();
-    for (int s = 0; s < 4; s++) {
-        st_half_sweep<W, THREADS>(sx, sb, si, rcs, rcd, s & 1);
         __syncthreads();
-    }
-    /* the residual in place of b at the colour the last half-sweep left (the
-     * other's is 0 up to the rounding of its own update), one point around
-     * the tile; 0 off the grid and on the Dirichlet row */
-    for (int q = threadIdx.x; q < (T + 2) * (T + 2) / 2; q += THREADS) {
-        const int lk = HALO - 1 + q / (T / 2 + 1), li = HALO - 1 + 2 * (q % (T / 2 + 1)) + ((lk + HALO - 1) & 1), o = lk * W + li;
-        double r = 0.0;
-        if (si[o] != 0.0) {
-            double off = rcd[lk] * sx[o - W];
-            off += rcd[lk + 1] * sx[o + W];
-            off += rcs[lk] * sx[o - 1];
-            off += rcs[lk] * sx[o + 1];
-            r = sb[o] - (sd[o] * sx[o] - off);
+        st_half_sweep<W, THREADS, false>(sx, sb, si, rcs, rcd, 0);
+        __syncthreads();
+        st_half_sweep<W, THREADS, false>(sx, sb, si, rcs, rcd, 1);
+        __syncthreads();
+        st_half_sweep<W, THREADS, true>(sx, sb, si, rcs, rcd, 0);
+        __syncthreads();
+        st_half_sweep<W, THREADS, false>(sx, sb, si, rcs, rcd, 1);
+        __syncthreads();
+        /* The residual b + off - diag x.  A point of the colour updated last
+         * has none; one of the other colour was left with diag x = b + off of
+         * the neighbours it saw then, so its residual is the change of off
+         * since.  In place of that sum, one point around the tile; 0 off the
+         * grid and on the Dirichlet row. */
+        for (int q = threadIdx.x; q < (T + 2) * (T / 2 + 1); q += THREADS) {
+            const int lk = HALO - 1 + q / (T / 2 + 1), par = lk & 1, j = (HALO - 1 + 1 - par) / 2 + q % (T / 2 + 1), o = lk * (W / 2) + j;
+            const double* other = sx + W * W / 2;
+            const double off = st_off(rcs[lk], rcd[lk], rcd[lk + 1], other[o - 1 + par], other[o + par], other[o - W / 2], other[o + W / 2]);
+            sb[o] = si[o] != 0.0 ? off - sb[o] : 0.0;
         }
-        sb[o] = r;
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < T * T; q += THREADS) {
-        const int li = q % T, lk = q / T, i = i0 + li, k = k0 + lk;
-        if (i < nx && k < nz) L.x[(size_t)k * nx + i] = sx[(lk + HALO) * W + li + HALO];
-    }
-    for (int q = threadIdx.x; q < (T / 2) * (T / 2); q += THREADS) {
-        const int li = 2 * (q % (T / 2)), lk = 2 * (q / (T / 2)), i = i0 + li, k = k0 + lk;
-        if (i >= nx || k >= nz) continue;
-        double s = 0.0;
-        if (k > 0) {
-            const double* r = sb + (lk + HALO) * W + li + HALO;
-            s = r[0] + 0.25 * (((r[-W - 1] + r[-W + 1]) + r[W - 1]) + r[W + 1]);
+        for (int q = threadIdx.x; q < T * T; q += THREADS) {
+            const int li = q % T, lk = q / T, i = i0 + li, k = k0 + lk;
+            if (i < nx && k < nz) L.x[(size_t)k * nx + i] = sx[st_at<W>(li + HALO, lk + HALO)];
         }
-        Lc.b[(size_t)(k / 2) * Lc.nx + i / 2] = 0.25 * s;
-    }
+        __syncthreads();
+        for (int q = threadIdx.x; q < (T / 2) * (T / 2); q += THREADS) {
+            const int li = 2 * (q % (T / 2)), lk = 2 * (q / (T / 2)), i = i0 + li, k = k0 + lk;
+            if (i >= nx || k >= nz) continue;
+            double s = 0.0;
+            if (k > 0) {
+                const double* r = sb + (lk + HALO) * (W / 2) + (li + HALO) / 2;      /* colour 0, an even row */
+                s = r[0] + 0.25 * ((r[-W / 2 - 1] + r[-W / 2]) + (r[W / 2 - 1] + r[W / 2]));
+            }
+            Lc.b[(size_t)(k / 2) * Lc.nx + i / 2] = 0.25 * s;
+        }
     }
 }
 
@@ -277,7 +331,8 @@ __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_up(StLevel L, StLevel
                                                               const double* __restrict__ r, double* part_rz)
 {
     constexpr int THREADS = StTile<T>::THREADS, HALO = SMOOTH ? 4 : 0, W = T + 2 * HALO;
-    if (ctl[0]) return;
+    constexpr int PER = (W * W + THREADS - 1) / THREADS;
+    const int done = ctl[0];
     extern __shared__ __align__(16) unsigned char st_smem[];
     double* sx = reinterpret_cast<double*>(st_smem);
     double* sb = sx + W * W;
@@ -287,38 +342,55 @@ __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_up(StLevel L, StLevel
     __shared__ double sh[32];
     const int i0 = blockIdx.x * T, k0 = blockIdx.y * T, nx = L.nx, nz = L.nz;
     const double* bsrc = CG ? r : L.b;
-    if (SMOOTH) {
-        for (int q = threadIdx.x; q < W * W; q += THREADS) {
-            const int i = i0 - HALO + q % W, k = k0 - HALO + q / W;
-            double x = 0.0, b = 0.0, id = 0.0;
-            if (i >= 0 && i < nx && k > 0 && k < nz) {
+    if constexpr (SMOOTH) {
+        /* only the colour the first half-sweep reads needs its value */
+        double x[PER], b[PER], id[PER], c[PER][4];
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const int q = threadIdx.x + j * THREADS, li = q % W, lk = q / W, i = i0 - HALO + li, k = k0 - HALO + lk;
+            x[j] = b[j] = id[j] = c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.0;
+            if (q < W * W && i >= 0 && i < nx && k > 0 && k < nz) {
                 const size_t p = (size_t)k * nx + i;
-                const int I0 = i / 2, K0 = k / 2, I1 = (i & 1) ? I0 + 1 : I0, K1 = (k & 1) ? K0 + 1 : K0;
-                const double* c0 = Lc.xo + (size_t)K0 * Lc.nx;
-                const double* c1 = Lc.xo + (size_t)K1 * Lc.nx;
-                x = L.x[p] + 0.25 * (c0[I0] + c0[I1] + c1[I0] + c1[I1]);
-                b = bsrc[p];
-                id = 1.0 / L.diag[p];
+                if (((li + lk) & 1) == 0) {
+                    const int I0 = i / 2, K0 = k / 2, I1 = (i & 1) ? I0 + 1 : I0, K1 = (k & 1) ? K0 + 1 : K0;
+                    const double* c0 = Lc.xo + (size_t)K0 * Lc.nx;
+                    const double* c1 = Lc.xo + (size_t)K1 * Lc.nx;
+                    x[j] = L.x[p];
+                    c[j][0] = c0[I0]; c[j][1] = c0[I1]; c[j][2] = c1[I0]; c[j][3] = c1[I1];
+                }
+                b[j] = bsrc[p];
+                id[j] = L.id[p];
             }
-            sx[q] = x; sb[q] = b; si[q] = id;
         }
-        for (int j = threadIdx.x; j <= W; j += THREADS) {
-            const int k = k0 - HALO + j;
-            if (j < W) rcs[j] = k >= 0 && k < nz ? L.cs[k] : 0.0;
-            rcd[j] = k >= 1 && k < nz ? L.cd[k] : 0.0;
+        double r1 = 0.0, r2 = 0.0;
+        if (threadIdx.x <= W) {
+            const int k = k0 - HALO + threadIdx.x;
+            r1 = k >= 0 && k < nz ? L.cs[k] : 0.0;
+            r2 = k >= 1 && k < nz ? L.cd[k] : 0.0;
+        }
+        if (done) return;
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const int q = threadIdx.x + j * THREADS, o = st_at<W>(q % W, q / W);
+            if (q < W * W) { sx[o] = x[j] + 0.25 * ((c[j][0] + c[j][1]) + (c[j][2] + c[j][3])); sb[o] = b[j]; si[o] = id[j]; }
+        }
+        if (threadIdx.x <= W) {
+            if (threadIdx.x < W) rcs[threadIdx.x] = r1;
+            rcd[threadIdx.x] = r2;
         }
         __syncthreads();
         for (int s = 0; s < 4; s++) {
-            st_half_sweep<W, THREADS>(sx, sb, si, rcs, rcd, 1 - (s & 1));
+            st_half_sweep<W, THREADS, false>(sx, sb, si, rcs, rcd, 1 - (s & 1));
             __syncthreads();
         }
     }
+    if (!SMOOTH && done) return;
     double rz = 0.0;
     for (int q = threadIdx.x; q < T * T; q += THREADS) {
         const int li = q % T, lk = q / T, i = i0 + li, k = k0 + lk;
         if (i >= nx || k >= nz) continue;
         const size_t p = (size_t)k * nx + i;
-        const int o = (lk + HALO) * W + li + HALO;
+        const int o = SMOOTH ? st_at<W>(li + HALO, lk + HALO) : 0;
         const double x = SMOOTH ? sx[o] : L.xo[p];
         if (SMOOTH) L.xo[p] = x;
         if (CG) rz += (SMOOTH ? sb[o] : r[p]) * x;
@@ -334,29 +406,40 @@ __global__ void __launch_bounds__(256) k_st_direction(StLevel L, const int* __re
                                                       const double* part_rz_old, int n_rz, int first_possible,
                                                       double* part_pap)
 {
-    if (ctl[0]) return;
-    __shared__ double sh[32];
+    __shared__ double sh[64];
+    const int done = ctl[0];
     const bool first = first_possible && ctl[1] == 0;
-    double beta = 0.0;
-    if (!first) {
-        const double rz = st_total<false, 256>(part_rz, n_rz, sh), old = st_total<false, 256>(part_rz_old, n_rz, sh);
-        beta = old != 0.0 ? rz / old : 0.0;
-    }
     const int nx = L.nx, nz = L.nz, n = nx * nz;
-    auto dir = [&](int p) -> double { return first ? z[p] : z[p] + beta * pold[p]; };
-    double s = 0.0;
-    for (int p = blockIdx.x * 256 + threadIdx.x; p < n; p += gridDim.x * 256) {
-        const int i = p % nx, k = p / nx;
-        const double c = dir(p);
+    double beta = 0.0, s = 0.0;
+    for (int p = blockIdx.x * 256 + threadIdx.x, turn = 0; p < n || turn == 0; p += gridDim.x * 256, turn++) {
+        /* the loads of a thread's first point are under way while the dot
+         * products are reduced; a missing neighbour reads the point itself
+         * with a zero coefficient */
+        const bool on = p < n;
+        const int pc = on ? p : 0, i = pc % nx, k = pc / nx;
+        const int pd = k > 1 ? pc - nx : pc, pu = k + 1 < nz ? pc + nx : pc, pl = i > 0 ? pc - 1 : pc, pr = i + 1 < nx ? pc + 1 : pc;
+        const double zc = z[pc], zd = z[pd], zu = z[pu], zl = z[pl], zr = z[pr];
+        const double oc = pold[pc], od = pold[pd], ou = pold[pu], ol = pold[pl], orr = pold[pr];
+        const double cs = L.cs[k], cd = L.cd[k], cu = L.cd[k + 1], dg = L.diag[pc];
+        if (turn == 0) {
+            if (done) return;
+            if (!first) {
+                double rz, old;
+                st_total2<256>(part_rz, n_rz, part_rz_old, n_rz, sh, rz, old);
+                beta = old != 0.0 ? rz / old : 0.0;
+            }
+        }
+        if (!on) break;
+        auto dir = [&](double zz, double oo) { return first ? zz : zz + beta * oo; };
+        const double c = dir(zc, oc);
         double y = 0.0;
         if (k > 0) {
-            const double cs = L.cs[k];
             double off = 0.0;
-            if (k > 1) off += L.cd[k] * dir(p - nx);
-            if (k + 1 < nz) off += L.cd[k + 1] * dir(p + nx);
-            if (i > 0) off += cs * dir(p - 1);
-            if (i + 1 < nx) off += cs * dir(p + 1);
-            y = L.diag[p] * c - off;
+            if (k > 1) off += cd * dir(zd, od);
+            if (k + 1 < nz) off += cu * dir(zu, ou);
+            if (i > 0) off += cs * dir(zl, ol);
+            if (i + 1 < nx) off += cs * dir(zr, orr);
+            y = dg * c - off;
         }
         pnew[p] = c;
         ap[p] = y;
@@ -385,109 +468,200 @@ __device__ bool st_stop(int* ctl, double* scal, const double* part_rn, int np, i
 
 struct StTail { StLevel L[ST_MAX_LEVELS]; int l0, nlev, use_op; };
 
+/* A level in the tail's shared memory: each array as two colour halves (entry
+ * j of row k of colour c is column 2 j + ((k + c) & 1)), rows of `hw` entries
+ * and a zero, which stands for the missing neighbour of either side; x has a
+ * zero row above the grid.  An entry past the last column has a zero
+ * reciprocal diagonal and stays 0. */
+struct StShared { int nx, nz, hw, ph, half, halfx; unsigned mag; int x, b, id, o, cs, cd; };
+
+/* Offsets of the tail's levels.  What a linearisation fixes (id, cs, cd) comes
+ * first, in one piece that k_st_coarse_rest lays out in device memory once and
+ * the tail copies with loads that do not wait for each other; the working
+ * arrays follow.  Returns the length of that piece (even); *all = the whole. */
+__host__ __device__ inline int st_tail_layout(const StLevel* L, int l0, int nlev, StShared* S, int* all)
+{
+    int at = 0;
+    for (int l = l0; l < nlev; l++) {
+        StShared& v = S[l];
+        v.nx = L[l].nx; v.nz = L[l].nz; v.hw = (v.nx + 1) / 2; v.ph = v.hw + 1;
+        v.half = v.ph * v.nz; v.halfx = v.ph * (v.nz + 1);
+        v.mag = 0xffffffffu / (unsigned)v.hw + 1u;
+        v.id = at; v.cs = v.id + 2 * v.half; v.cd = v.cs + v.nz;
+        at = v.cd + v.nz + 1;
+    }
+    at += at & 1;
+    const int image = at;
+    for (int l = l0; l < nlev; l++) {
+        StShared& v = S[l];
+        v.x = at; v.b = v.x + 2 * v.halfx; v.o = v.b + 2 * v.half;
+        at = v.o + v.half;
+    }
+    *all = at;
+    return image;
+}
+/* entry of column i, row k in an array whose colour halves are `half` apart */
+__device__ __forceinline__ int st_entry(const StShared& L, int half, int i, int k) { return ((i + k) & 1) * half + k * L.ph + (i >> 1); }
+
+__device__ __forceinline__ void st_sync(bool one) { if (one) __syncwarp(); else __syncthreads(); }
+
+/* one half-sweep of a level by `nth` threads; KEEP: keep the neighbour sums */
+template <bool KEEP>
+__device__ __forceinline__ void st_shared_half(double* m, const StShared& L, int colour, int th, int nth)
+{
+    const int n = L.hw * (L.nz - 1);
+    double* x = m + L.x + colour * L.halfx;
+    const double* other = m + L.x + (1 - colour) * L.halfx;
+    const double* b = m + L.b + colour * L.half;
+    const double* id = m + L.id + colour * L.half;
+    for (int q = th; q < n; q += nth) {
+        const int kk = (int)__umulhi((unsigned)q, L.mag), k = kk + 1, par = (k + colour) & 1;
+        const int p = k * L.ph + q - kk * L.hw;
+        const double off = st_off(m[L.cs + k], m[L.cd + k], m[L.cd + k + 1], other[p - 1 + par], other[p + par],
+                                  other[p - L.ph], other[p + L.ph]);
+        x[p] = (b[p] + off) * id[p];
+        if (KEEP) m[L.o + p] = off;
+    }
+}
+__device__ __forceinline__ void st_shared_down(double* m, const StShared L, const StShared Lc, int th, int nth, bool one)
+{
+    st_shared_half<false>(m, L, 0, th, nth); st_sync(one);
+    st_shared_half<false>(m, L, 1, th, nth); st_sync(one);
+    st_shared_half<true>(m, L, 0, th, nth); st_sync(one);
+    st_shared_half<false>(m, L, 1, th, nth); st_sync(one);
+    /* residual of colour 0 and restriction, as in k_st_down */
+    {
+        const double* other = m + L.x + L.halfx;
+        for (int q = th; q < L.hw * (L.nz - 1); q += nth) {
+            const int kk = (int)__umulhi((unsigned)q, L.mag), k = kk + 1, par = k & 1;
+            const int p = k * L.ph + q - kk * L.hw;
+            const double off = st_off(m[L.cs + k], m[L.cd + k], m[L.cd + k + 1], other[p - 1 + par], other[p + par],
+                                      other[p - L.ph], other[p + L.ph]);
+            m[L.o + p] = m[L.id + p] != 0.0 ? off - m[L.o + p] : 0.0;
+        }
+    }
+    st_sync(one);
+    const unsigned magc = 0xffffffffu / (unsigned)Lc.nx + 1u;
+    for (int q = th; q < Lc.nx * (Lc.nz - 1); q += nth) {
+        const int kk = (int)__umulhi((unsigned)q, magc), K = kk + 1, I = q - kk * Lc.nx;
+        const double* r = m + L.o + 2 * K * L.ph + I;
+        double s = r[0], c = 0.0;
+        c += r[-L.ph - 1] + r[-L.ph];                    /* column -1 reads the row's zero */
+        if (K + 1 < Lc.nz) c += r[L.ph - 1] + r[L.ph];
+        m[Lc.b + st_entry(Lc, Lc.half, I, K)] = 0.25 * (s + 0.25 * c);
+    }
+    st_sync(one);
+}
+__device__ __forceinline__ void st_shared_up(double* m, const StShared L, const StShared Lc, int th, int nth, bool one)
+{
+    const double* c = m + Lc.x;
+    for (int q = th; q < L.hw * (L.nz - 1); q += nth) {
+        const int kk = (int)__umulhi((unsigned)q, L.mag), k = kk + 1, j = q - kk * L.hw, K = k >> 1;
+        if (k & 1) {
+            if (j < L.hw - 1)
+                m[L.x + k * L.ph + j] += 0.25 * ((c[st_entry(Lc, Lc.halfx, j, K)] + c[st_entry(Lc, Lc.halfx, j + 1, K)]) +
+                                                 (c[st_entry(Lc, Lc.halfx, j, K + 1)] + c[st_entry(Lc, Lc.halfx, j + 1, K + 1)]));
+        } else m[L.x + k * L.ph + j] += c[st_entry(Lc, Lc.halfx, j, K)];
+    }
+    st_sync(one);
+    st_shared_half<false>(m, L, 1, th, nth); st_sync(one);
+    st_shared_half<false>(m, L, 0, th, nth); st_sync(one);
+    st_shared_half<false>(m, L, 1, th, nth); st_sync(one);
+    st_shared_half<false>(m, L, 0, th, nth); st_sync(one);
+}
+
 /* Levels l0 .. nlev-1 of the V-cycle in one block's shared memory, and
  * before them the stopping rule.  b of level l0 comes from device memory and
  * its x goes back there.  The coarsest level's 40 + 40 symmetric sweeps are
  * a fixed linear map of b: one matrix-vector product where it is small (its
- * matrix is made once per linearisation by k_st_coarse_op), sweeps otherwise. */
-__global__ void __launch_bounds__(ST_TAIL_THREADS) k_st_tail(StTail t, int* ctl, double* scal, const double* part_rn,
-                                                             int np, int first, const double* __restrict__ b0,
-                                                             const double* __restrict__ op)
+ * matrix is made once per linearisation by k_st_coarse_rest), sweeps otherwise.
+ * What bounds it is the chain of some 50 phases, each a shared-memory round
+ * trip, a few dependent FP64 operations and a barrier; the levels of a few
+ * dozen points run on one warp, whose barrier costs next to nothing. */
+__global__ void __launch_bounds__(ST_TAIL_THREADS) k_st_tail(const __grid_constant__ StTail t, int* ctl, double* scal,
+                                                             const double* part_rn, int np, int first,
+                                                             const double* __restrict__ b0, const double* __restrict__ op,
+                                                             const double* __restrict__ image)
 {
     constexpr int NT = ST_TAIL_THREADS;
-    if (ctl[0]) return;
     __shared__ double sh[32];
+    __shared__ StShared lv[ST_MAX_LEVELS];
+    __shared__ double sop[ST_OP_MAX * ST_OP_MAX];
+    __shared__ int len[2];
     extern __shared__ __align__(16) unsigned char st_smem[];
-    if (st_stop<NT>(ctl, scal, part_rn, np, first, sh)) return;
-    const int th = threadIdx.x;
-    double* base[ST_MAX_LEVELS];
-    double* mem = reinterpret_cast<double*>(st_smem);
-    /* per level: x, b, diag, reciprocal diag, rows' cs, rows' cd (nz + 1) */
-    for (int l = t.l0; l < t.nlev; l++) {
-        const StLevel& L = t.L[l];
-        const int n = L.nx * L.nz;
-        base[l] = mem;
-        double *x = mem, *b = mem + n, *d = mem + 2 * n, *id = mem + 3 * n, *cs = mem + 4 * n, *cd = cs + L.nz;
-        mem = cd + L.nz + 1;
-        for (int p = th; p < n; p += NT) {
-            const bool in = p >= L.nx;
-            const double v = in ? L.diag[p] : 1.0;
-            x[p] = 0.0; d[p] = v; id[p] = in ? 1.0 / v : 0.0;
-            b[p] = (l == t.l0 && in) ? b0[p] : 0.0;
+    double* m = reinterpret_cast<double*>(st_smem);
+    const int th = threadIdx.x, last = t.nlev - 1;
+    const int done = ctl[0];
+    if (th == 0) len[0] = st_tail_layout(t.L, t.l0, t.nlev, lv, &len[1]);
+    const int nu = t.L[last].nx * (t.L[last].nz - 1);
+    if (t.use_op) for (int q = th; q < nu * nu; q += NT) sop[q] = op[q];
+    __syncthreads();
+    {
+        const int n16 = len[0] / 2;
+        const double2* src = reinterpret_cast<const double2*>(image);
+        double2* dst = reinterpret_cast<double2*>(m);
+        for (int q0 = th; q0 < n16; q0 += 8 * NT) {
+            double2 v[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) if (q0 + j * NT < n16) v[j] = src[q0 + j * NT];
+#pragma unroll
+            for (int j = 0; j < 8; j++) if (q0 + j * NT < n16) dst[q0 + j * NT] = v[j];
         }
-        for (int k = th; k <= L.nz; k += NT) { if (k < L.nz) cs[k] = L.cs[k]; cd[k] = k >= 1 && k < L.nz ? L.cd[k] : 0.0; }
+        for (int q = len[0] + th; q < len[1]; q += NT) m[q] = 0.0;
     }
     __syncthreads();
-    auto sum4 = [&](const StLevel& L, const double* x, const double* cs, const double* cd, int i, int k, int p) {
-        double off = cd[k] * x[p - L.nx];
-        if (k + 1 < L.nz) off += cd[k + 1] * x[p + L.nx];
-        if (i > 0) off += cs[k] * x[p - 1];
-        if (i + 1 < L.nx) off += cs[k] * x[p + 1];
-        return off;
-    };
-    /* nx is odd, so a point's colour is the parity of its index */
-    auto half = [&](int l, int colour) {
-        const StLevel& L = t.L[l];
-        const int n = L.nx * L.nz;
-        double *x = base[l], *b = x + n, *id = x + 3 * n, *cs = x + 4 * n, *cd = cs + L.nz;
-        for (int p = L.nx + ((L.nx + colour) & 1) + 2 * th; p < n; p += 2 * NT) {
-            const int k = p / L.nx, i = p - k * L.nx;
-            x[p] = (b[p] + sum4(L, x, cs, cd, i, k, p)) * id[p];
-        }
-        __syncthreads();
-    };
-    const int last = t.nlev - 1;
-    for (int l = t.l0; l < last; l++) {
-        const StLevel &L = t.L[l], &Lc = t.L[l + 1];
-        const int n = L.nx * L.nz, nc = Lc.nx * Lc.nz;
-        double *x = base[l], *b = x + n, *d = x + 2 * n, *cs = x + 4 * n, *cd = cs + L.nz;
-        double* bc = base[l + 1] + nc;
-        half(l, 0); half(l, 1); half(l, 0); half(l, 1);
-        /* as in k_st_down, the residual of the colour updated last is left out */
-        for (int p = Lc.nx + th; p < nc; p += NT) {
-            const int K = p / Lc.nx, I = p - K * Lc.nx;
-            auto res = [&](int i, int k) {
-                if (i < 0 || i >= L.nx || k >= L.nz) return 0.0;
-                const int f = k * L.nx + i;
-                return b[f] - (d[f] * x[f] - sum4(L, x, cs, cd, i, k, f));
-            };
-            const double s = res(2 * I, 2 * K) + 0.25 * (((res(2 * I - 1, 2 * K - 1) + res(2 * I + 1, 2 * K - 1)) +
-                                                          res(2 * I - 1, 2 * K + 1)) + res(2 * I + 1, 2 * K + 1));
-            bc[p] = 0.25 * s;
-        }
-        __syncthreads();
-    }
     {
-        const StLevel& L = t.L[last];
-        const int n = L.nx * L.nz, nu = n - L.nx;
-        double *x = base[last], *b = x + n;
+        const StShared S = lv[t.l0];
+        const int n = S.nx * S.nz;
+        const unsigned mag = 0xffffffffu / (unsigned)S.nx + 1u;
+#pragma unroll 4
+        for (int p = S.nx + th; p < n; p += NT) {
+            const int k = (int)__umulhi((unsigned)p, mag);
+            m[S.b + st_entry(S, S.half, p - k * S.nx, k)] = b0[p];
+        }
+    }
+    if (done) return;
+    if (st_stop<NT>(ctl, scal, part_rn, np, first, sh)) return;
+    __syncthreads();
+    int lw = t.l0;                           /* first level one warp runs alone */
+    while (lw < last && lv[lw].hw * (lv[lw].nz - 1) > ST_WARP_POINTS) lw++;
+    for (int l = t.l0; l < lw; l++) st_shared_down(m, lv[l], lv[l + 1], th, NT, false);
+    const StShared B = lv[last];
+    if (!t.use_op && lw == last) {           /* a coarsest level of many unknowns: sweeps by the block */
+        for (int j = 0; j < 160; j++) {
+            st_shared_half<false>(m, B, j < 80 ? (j & 1) : 1 - (j & 1), th, NT);
+            __syncthreads();
+        }
+    } else if (th < 32) {
+        for (int l = lw; l < last; l++) st_shared_down(m, lv[l], lv[l + 1], th, 32, true);
         if (t.use_op) {
             if (th < nu) {
                 double s = 0.0;
-                for (int j = 0; j < nu; j++) s += op[j * nu + th] * b[L.nx + j];
-                x[L.nx + th] = s;
+                for (int j = 0, k = 1, i = 0; j < nu; j++) {
+                    s = fma(sop[j * nu + th], m[B.b + st_entry(B, B.half, i, k)], s);
+                    if (++i == B.nx) { i = 0; k++; }
+                }
+                m[B.x + st_entry(B, B.halfx, th % B.nx, 1 + th / B.nx)] = s;
             }
-            __syncthreads();
+            __syncwarp();
         } else {
-            for (int j = 0; j < 40; j++) { half(last, 0); half(last, 1); }
-            for (int j = 0; j < 40; j++) { half(last, 1); half(last, 0); }
+            for (int j = 0; j < 160; j++) {
+                st_shared_half<false>(m, B, j < 80 ? (j & 1) : 1 - (j & 1), th, 32);
+                __syncwarp();
+            }
         }
+        for (int l = last - 1; l >= lw; l--) st_shared_up(m, lv[l], lv[l + 1], th, 32, true);
     }
-    for (int l = last - 1; l >= t.l0; l--) {
-        const StLevel &L = t.L[l], &Lc = t.L[l + 1];
-        const int n = L.nx * L.nz;
-        double* x = base[l];
-        const double* xc = base[l + 1];
-        for (int p = L.nx + th; p < n; p += NT) {
-            const int k = p / L.nx, i = p - k * L.nx;
-            const int I0 = i / 2, K0 = k / 2, I1 = (i & 1) ? I0 + 1 : I0, K1 = (k & 1) ? K0 + 1 : K0;
-            x[p] += 0.25 * (xc[K0 * Lc.nx + I0] + xc[K0 * Lc.nx + I1] + xc[K1 * Lc.nx + I0] + xc[K1 * Lc.nx + I1]);
-        }
-        __syncthreads();
-        half(l, 1); half(l, 0); half(l, 1); half(l, 0);
+    __syncthreads();
+    for (int l = lw - 1; l >= t.l0; l--) st_shared_up(m, lv[l], lv[l + 1], th, NT, false);
+    const StShared S = lv[t.l0];
+    double* out = t.L[t.l0].xo;
+    const unsigned mag = 0xffffffffu / (unsigned)S.nx + 1u;
+#pragma unroll 4
+    for (int p = th; p < S.nx * S.nz; p += NT) {
+        const int k = (int)__umulhi((unsigned)p, mag);
+        out[p] = m[S.x + st_entry(S, S.halfx, p - k * S.nx, k)];
     }
-    const StLevel& L = t.L[t.l0];
-    for (int p = th; p < L.nx * L.nz; p += NT) L.xo[p] = base[t.l0][p];
 }
 
 /* The same steps where no level fits one block (a level of 3 rows or columns
@@ -558,21 +732,37 @@ __device__ void st_coarse_point(const StLevel& Lc, const StLevel& Lf, int p)
     }
     const double sig = s / ws;
     Lc.sig[p] = sig;
-    Lc.diag[p] = K > 0 ? st_diag(Lc, I, K, sig) : 1.0;
+    const double diag = K > 0 ? st_diag(Lc, I, K, sig) : 1.0;
+    Lc.diag[p] = diag;
+    Lc.id[p] = K > 0 ? 1.0 / diag : 0.0;
 }
 __global__ void k_st_coarse_coeffs(StLevel Lc, StLevel Lf)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < Lc.nx * Lc.nz) st_coarse_point(Lc, Lf, p);
 }
-/* levels l0 .. nlev-1 one after another in one block; then, where the
+/* levels l0 .. nlev-1 one after another in one block; the tail's image of
+ * them (st_tail_layout); then, where the
  * coarsest level has at most ST_OP_MAX unknowns, the matrix of its 40 + 40
  * sweeps: warp j runs them on the j-th unit vector */
-__global__ void __launch_bounds__(1024) k_st_coarse_rest(StTail t, double* op)
+__global__ void __launch_bounds__(1024) k_st_coarse_rest(const __grid_constant__ StTail t, int tail, double* op, double* image)
 {
+    __shared__ StShared lv[ST_MAX_LEVELS];
+    __shared__ int all;
+    if (threadIdx.x == 0) st_tail_layout(t.L, tail, t.nlev, lv, &all);
     for (int l = t.l0; l < t.nlev; l++) {
         for (int p = threadIdx.x; p < t.L[l].nx * t.L[l].nz; p += blockDim.x) st_coarse_point(t.L[l], t.L[l - 1], p);
         __syncthreads();
+    }
+    __syncthreads();
+    for (int l = tail; l < t.nlev; l++) {
+        const StShared S = lv[l];
+        const StLevel& L = t.L[l];
+        for (int p = threadIdx.x; p < 2 * S.half; p += blockDim.x) {
+            const int c = p >= S.half, k = (p - c * S.half) / S.ph, j = p - c * S.half - k * S.ph, i = 2 * j + ((k + c) & 1);
+            image[S.id + p] = j < S.hw && i < S.nx ? L.id[k * S.nx + i] : 0.0;
+        }
+        for (int k = threadIdx.x; k <= S.nz; k += blockDim.x) { if (k < S.nz) image[S.cs + k] = L.cs[k]; image[S.cd + k] = L.cd[k]; }
     }
     if (!t.use_op) return;
     const StLevel& L = t.L[t.nlev - 1];
@@ -581,7 +771,7 @@ __global__ void __launch_bounds__(1024) k_st_coarse_rest(StTail t, double* op)
     if (j >= nu) return;                     /* whole warp */
     const int p = nx + (u < nu ? u : 0), i = p % nx, k = p / nx;
     const bool on = u < nu;
-    const double id = on ? 1.0 / L.diag[p] : 0.0;
+    const double id = on ? L.id[p] : 0.0;
     const double cs = L.cs[k], cdn = k > 1 ? L.cd[k] : 0.0, cup = k + 1 < L.nz ? L.cd[k + 1] : 0.0;
     const double cl = i > 0 ? cs : 0.0, cr = i + 1 < nx ? cs : 0.0;
     const double b = u == j ? 1.0 : 0.0;
@@ -646,6 +836,7 @@ __global__ void __launch_bounds__(256) k_st_newton_rhs(StLevel L, const double* 
         F[p] = f;
         L.sig[p] = sig;
         L.diag[p] = diag;
+        L.id[p] = k > 0 ? 1.0 / diag : 0.0;
     }
     st_partial<true, 256>(fabs(f), part, blockIdx.x, sh);
 }
@@ -725,13 +916,14 @@ static int st_tile(const StLevel& L)
     return ((L.nx + 31) / 32) * ((L.nz + 31) / 32) >= 74 ? 32 : 16;
 }
 static dim3 st_tiles(const StLevel& L, int T) { return dim3((unsigned)((L.nx + T - 1) / T), (unsigned)((L.nz + T - 1) / T)); }
-static size_t st_down_smem(int T) { const int W = T + 12; return sizeof(double) * (4 * W * W + 2 * W + 1); }
+static size_t st_down_smem(int T) { const int W = T + 12; return sizeof(double) * (3 * W * W + 2 * W + 1); }
 static size_t st_up_smem(int T) { const int W = T + 8; return sizeof(double) * (3 * W * W + 2 * W + 1); }
 static size_t st_tail_smem(const bcg_steady* s)
 {
-    size_t d = 0;
-    for (int l = s->tail; l < s->nlev; l++) d += 4 * (size_t)s->L[l].nx * s->L[l].nz + 2 * (size_t)s->L[l].nz + 1;
-    return d * sizeof(double);
+    StShared S[ST_MAX_LEVELS];
+    int all = 0;
+    st_tail_layout(s->L, s->tail, s->nlev, S, &all);
+    return sizeof(double) * (size_t)all;
 }
 static int st_coarsest(const bcg_steady* s) { const StLevel& L = s->L[s->nlev - 1]; return L.nx * (L.nz - 1); }
 
@@ -768,7 +960,7 @@ static void st_cycle(bcg_steady* s, const double* rhs, int it)
         memcpy(t.L, s->L, sizeof(t.L));
         t.l0 = s->tail; t.nlev = s->nlev; t.use_op = st_coarsest(s) <= ST_OP_MAX;
         k_st_tail<<<1, ST_TAIL_THREADS, st_tail_smem(s), s->stream>>>(t, s->ctl, s->scal, s->part_rn, s->nt0, first,
-                                                                      s->tail == 0 ? r : s->L[s->tail].b, s->op);
+                                                                      s->tail == 0 ? r : s->L[s->tail].b, s->op, s->image);
     } else {
         StLevel& L = s->L[s->nlev - 1];
         const double* b = one ? r : L.b;
@@ -823,7 +1015,7 @@ static int st_pcg(bcg_steady* s, const double* rhs, double tol, int max_it, int*
     StTail t;
     memcpy(t.L, s->L, sizeof(t.L));
     t.l0 = lr; t.nlev = s->nlev; t.use_op = s->tail < s->nlev && st_coarsest(s) <= ST_OP_MAX;
-    k_st_coarse_rest<<<1, 1024, 0, s->stream>>>(t, s->op);
+    k_st_coarse_rest<<<1, 1024, 0, s->stream>>>(t, s->tail, s->op, s->image);
     st_cycle(s, rhs, 0);
     int rc = st_err(cudaGetLastError());
     volatile int* h = reinterpret_cast<volatile int*>(s->pin);
@@ -859,7 +1051,7 @@ static int st_attributes()
 #define ST_SMEM(k, b) if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(b)) != cudaSuccess) return BCG_E_CUDA
     ST_SMEM((k_st_down<32, true, true>), st_down_smem(32));
     ST_SMEM((k_st_down<32, false, true>), st_down_smem(32));
-    ST_SMEM(k_st_tail, 220 * 1024);
+    ST_SMEM(k_st_tail, 32 * ST_TAIL_POINTS);
 #undef ST_SMEM
     return BCG_OK;
 }
@@ -886,7 +1078,7 @@ extern "C" int bcg_steady_create(const bcg_steady_params* p, bcg_steady** out)
         StLevel& L = s->L[s->nlev];
         L.nx = nx; L.nz = nz; L.h = h;
         size_t b = sizeof(double) * (size_t)nx * nz;
-        ST_ALLOC(L.x, b); ST_ALLOC(L.xo, b); ST_ALLOC(L.b, b); ST_ALLOC(L.sig, b); ST_ALLOC(L.diag, b);
+        ST_ALLOC(L.x, b); ST_ALLOC(L.xo, b); ST_ALLOC(L.b, b); ST_ALLOC(L.sig, b); ST_ALLOC(L.diag, b); ST_ALLOC(L.id, b);
         ST_ALLOC(L.cs, sizeof(double) * (nz + 1)); ST_ALLOC(L.cd, sizeof(double) * (nz + 1));
         /* the Dirichlet row, which no kernel writes everywhere, is 0 */
         if (!rc) rc = st_err(cudaMemsetAsync(L.xo, 0, b, s->stream));
@@ -899,7 +1091,7 @@ extern "C" int bcg_steady_create(const bcg_steady_params* p, bcg_steady** out)
     /* the largest set of levels, from the coarsest up, that fits the tail */
     s->tail = s->nlev;
     for (int l = s->nlev - 1, pts = 0; l >= (s->nlev > 1 ? 1 : 0); l--) {
-        pts += s->L[l].nx * s->L[l].nz + s->L[l].nz / 2 + 1;
+        pts += (s->L[l].nx + 3) * (s->L[l].nz + 1) + s->L[l].nz / 2 + 2;    /* over st_tail_smem / 32 B */
         if (pts > ST_TAIL_POINTS) break;
         s->tail = l;
     }
@@ -917,6 +1109,7 @@ extern "C" int bcg_steady_create(const bcg_steady_params* p, bcg_steady** out)
     ST_ALLOC(s->scal, sizeof(double) * 16);
     ST_ALLOC(s->ctl, sizeof(int) * 16);
     ST_ALLOC(s->op, sizeof(double) * ST_OP_MAX * ST_OP_MAX);
+    ST_ALLOC(s->image, 32 * ST_TAIL_POINTS);
     ST_ALLOC(s->gpart, sizeof(double) * 4 * ST_RED_BLOCKS);
     ST_ALLOC(s->start, sizeof(int) * ((size_t)s->n + 1));
     if (!rc) rc = st_err(cudaMemsetAsync(s->start, 0, sizeof(int) * ((size_t)s->n + 1), s->stream));
@@ -940,11 +1133,11 @@ extern "C" int bcg_steady_destroy(bcg_steady* s)
     if (s->stream) cudaStreamSynchronize(s->stream);
     for (int l = 0; l < s->nlev; l++) { 
         StLevel& L = s->L[l];
-        void* lv[] = {L.x, L.xo, L.b, L.sig, L.diag, L.cs, L.cd};
+        void* lv[] = {L.x, L.xo, L.b, L.sig, L.diag, L.id, L.cs, L.cd};
         for (void* q : lv) if (q) cudaFree(q);
     }
     void* ptrs[] = {s->C, s->q, s->F, s->g, s->cg_x, s->cg_r[0], s->cg_r[1], s->cg_p[0], s->cg_p[1], s->cg_ap, s->part_rn,
-                    s->part_rz[0], s->part_rz[1], s->part_pap, s->scal, s->ctl, s->op, s->gpart,
+                    s->part_rz[0], s->part_rz[1], s->part_pap, s->scal, s->ctl, s->op, s->image, s->gpart,
                     s->cell, s->cell_pt, s->w, s->gw, s->start, s->order};
     for (void* q : ptrs) if (q) cudaFree(q);
     if (s->graph) cudaGraphExecDestroy(s->graph);
