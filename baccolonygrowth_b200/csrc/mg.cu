@@ -1220,6 +1220,13 @@ static int warm_rows(const MgConst& m, int l)
     return 64;
 }
 
+/* Levels the register-tiled smoother takes (relax mode 3).  Its time grows with
+ * the points (39 us at 2305 x 513, 130 us at 4609 x 1025), the TMA form's hardly
+ * does until its warps fill the SMs (57 and 87 us); the line lies where the two
+ * meet. */
+#define TILE_POINTS 1800000
+static bool tile_takes(const MgLevel& L) { return (long)(L.nx + 1) * (L.nz + 1) <= TILE_POINTS; }
+
 template <class T>
 static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps)
 {
@@ -1229,6 +1236,19 @@ static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps)
     if (c->relax_mode < 2 || rows < 3) {
         for (int j = 0; j < sweeps; j++) relax_level<T>(c, m, l);
         return;
+    }
+    if constexpr (sizeof(T) == 8) {
+        if (c->relax_mode == 3 && tile_takes(c->mg[l])) {
+            const int warm = warm_rows(m, l);
+            while (sweeps > 0) {
+                const int S = sweeps >= 3 ? 3 : sweeps;
+                const int rc = mg_smooth_tile(c, m, mg_lvl(c, l), l, S, warm);
+                if (rc) { c->pending_error = rc; return; }
+                swap_err<T>(c, l);
+                sweeps -= S;
+            }
+            return;
+        }
     }
     if (c->relax_mode == 3 && mg_smooth_tma_fits(c->mg[l].nx)) {
         const int warm = warm_rows(m, l);
@@ -1305,7 +1325,8 @@ int mg_kernel_attributes()
         cudaFuncSetAttribute(k_mg_smooth<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_f) != cudaSuccess ||
         cudaFuncSetAttribute(k_mg_smooth<float, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_f) != cudaSuccess)
         return BCG_E_CUDA;
-    return mg_smooth_tma_attributes();
+    const int rc = mg_tile_attributes();
+    return rc ? rc : mg_smooth_tma_attributes();
 }
 
 /* bcg_autotune(BCG_TUNE_SMOOTHER): time the fused smoother on the finest
@@ -1472,14 +1493,20 @@ template <class T>
 void mg_vcycle_t(bcg_ctx* c, const MgConst& m, int mu1, int mu2)
 {
     const int Lv = c->mg_levels;
-    for (int l = 0; l < Lv - 1; l++) {
+    const int lt = c->relax_mode == 3 && sizeof(T) == 8 ? mg_tail_level(c, m) : Lv;
+    const int down = lt < Lv - 1 ? lt : Lv - 1;      /* levels smoothed and transferred one by one */
+    for (int l = 0; l < down; l++) {
         smooth_level<T>(c, m, l, mu1);
         MgLvlT<T> Lc = lvl<T>(c, l + 1), Lf = lvl<T>(c, l);
         k_mg_restrict<T><<<grid_rows(Lc.nx + 1, restrict_rows(m, Lc, l + 1), 128), 128, 0, c->stream>>>(m, Lc, Lf, l + 1, c->inside);
         c->launches++;
     }
-    relax_coarsest<T>(c, m, Lv - 1, mu2);
-    for (int l = Lv - 2; l >= 0; l--) {
+    if (lt < Lv) {
+        MgLvl lv[BCG_MAX_MG_LEVELS];
+        for (int l = lt; l < Lv; l++) lv[l - lt] = mg_lvl(c, l);
+        mg_tail(c, m, lv, lt, mu1, mu2);
+    } else relax_coarsest<T>(c, m, Lv - 1, mu2);
+    for (int l = down - 1; l >= 0; l--) {
         MgLvlT<T> Lf = lvl<T>(c, l), Lc = lvl<T>(c, l + 1);
         k_mg_interp<T><<<grid_rows(Lf.nx / 2 + 1, Lf.nz + 1, 128), 128, 0, c->stream>>>(m, Lf, Lc, l);
         c->launches++;

@@ -47,6 +47,13 @@ int mg_smooth_tma_attributes();
 /* whether mg_smooth_tma takes a level with nx + 1 columns */
 int mg_smooth_tma_fits(int nx);
 
+/* the register-tiled smoother and the one-launch coarsest levels (mg_tile.cu):
+ * S sweeps of level L from E into E2; levels l0 .. of a V-cycle, in place */
+int mg_smooth_tile(bcg_ctx* c, const MgConst& m, const MgLvl& L, int l, int S, int warm);
+int mg_tail_level(const bcg_ctx* c, const MgConst& m);
+int mg_tail(bcg_ctx* c, const MgConst& m, const MgLvl* lvls, int l0, int mu1, int mu2);
+int mg_tile_attributes();
+
 /* One of three kernel-parameter array entries by a runtime index without
  * indexing the parameter array itself (a runtime index into a parameter
  * array makes the compiler copy the whole parameter block to per-thread
