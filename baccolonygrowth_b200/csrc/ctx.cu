@@ -74,6 +74,12 @@ int ctx_check_status(bcg_ctx* c)
     return BCG_OK;
 }
 
+int ctx_check_status_bbox(bcg_ctx* c)
+{
+    BCG_CUDA_TRY(cudaMemcpyAsync(c->host_bbox, c->bbox, sizeof(c->host_bbox), cudaMemcpyDeviceToHost, c->stream));
+    return ctx_check_status(c);
+}
+
 int ensure_pinned(bcg_ctx* c, size_t bytes)
 {
     if (bytes <= c->pinned_bytes) return BCG_OK;
@@ -226,6 +232,7 @@ extern "C" int bcg_create(const bcg_params* p, bcg_ctx** out)
         return BCG_E_CUDA;
     }
     for (int t = 0; t < BCG_T_COUNT; t++) { cudaEventCreate(&c->ev[t][0]); cudaEventCreate(&c->ev[t][1]); }
+    c->host_bbox[0] = -1;
     const size_t cap = (size_t)p->max_cells;
     c->cap = p->max_cells;
     c->kmax = p->max_neighbours;
@@ -289,6 +296,9 @@ extern "C" int bcg_create(const bcg_params* p, bcg_ctx** out)
             DALLOC(e.extra[k], X * Z * 8);
             if ((rc = fill(c, e.extra[k], 0.0, X * Z))) { bcg_destroy(c); return rc; }
         }
+        SweepBuf& t = c->sweep2[b];
+        DALLOC(t.C, X * Z * 8); DALLOC(t.W, X * Z * 8); DALLOC(t.A, X * Z * 8); DALLOC(t.O, X * Z * 8);
+        DALLOC(t.wall, X * 8 * 4 * p->max_levels_mg);
         WallBuf& w = c->wal[b];
         for (int l = 0; l < p->max_levels_mg; l++) {
             DALLOC(w.C[l], X * 8); DALLOC(w.W[l], X * 8); DALLOC(w.O[l], X * 8); DALLOC(w.A[l], X * 8);
@@ -300,6 +310,7 @@ extern "C" int bcg_create(const bcg_params* p, bcg_ctx** out)
     for (auto a : f3) { DALLOC(*a, X * Z * 8); if ((rc = fill(c, *a, 0.0, X * Z))) { bcg_destroy(c); return rc; } }
     double** f2[] = {&c->rws, &c->wds, &c->rw, &c->wd};
     for (auto a : f2) { DALLOC(*a, X * 8); if ((rc = fill(c, *a, 0.0, X))) { bcg_destroy(c); return rc; } }
+    DALLOC(c->sweep_type, X * Z);
     DALLOC(c->bbox, 64);
     BCG_CUDA_TRY(cudaMemsetAsync(c->bbox, 0, 64, c->stream));
     /* multigrid levels, Multigrid.cpp:5-33: LocalAga defaults in all arrays */
@@ -326,7 +337,7 @@ extern "C" int bcg_create(const bcg_params* p, bcg_ctx** out)
         }
     }
     DALLOC(c->mg_scratch, 1 << 20);
-    if ((rc = mg_kernel_attributes()) || (rc = mech_kernel_attributes())) { bcg_destroy(c); return rc; }
+    if ((rc = mg_kernel_attributes()) || (rc = mech_kernel_attributes()) || (rc = sweep_kernel_attributes())) { bcg_destroy(c); return rc; }
     rc = ensure_pinned(c, 1 << 16);
     if (rc) { bcg_destroy(c); return rc; }
     rc = ctx_check_status(c);
@@ -346,13 +357,15 @@ extern "C" int bcg_destroy(bcg_ctx* c)
                     c->div_list, c->div_count, c->fcw_count, c->moved, c->delta_ids, c->delta_box, c->lineage,
                     c->n_done_dev, c->draws_dev, c->div_rec, c->div_box, c->div_rect, c->div_pairs, c->div_par,
                     c->div_order, c->div_grp, c->status, c->height, c->rough_height, c->nrm_x, c->nrm_y, c->nrm_z,
-                    c->wall, c->rd, c->inside, c->rds, c->ds, c->dens, c->rws, c->wds, c->rw, c->wd, c->bbox, c->mg_scratch};
+                    c->wall, c->rd, c->inside, c->rds, c->ds, c->dens, c->rws, c->wds, c->rw, c->wd, c->bbox, c->mg_scratch, c->sweep_type};
     for (void* q : ptrs) if (q) cudaFree(q);
     for (int b = 0; b < 2; b++) {
         EnvBuf& e = c->env[b];
         void* ea[] = {e.C, e.W, e.A, e.O, e.gr1, e.gr2, e.ph, e.hydrox, e.acetic, e.buffer};
         for (void* q : ea) if (q) cudaFree(q);
         for (double* q : e.extra) if (q) cudaFree(q);
+        void* sa[] = {c->sweep2[b].C, c->sweep2[b].W, c->sweep2[b].A, c->sweep2[b].O, c->sweep2[b].wall};
+        for (void* q : sa) if (q) cudaFree(q);
         for (int l = 0; l < BCG_MAX_AGAR_LEVELS; l++) {
             void* wa[] = {c->wal[b].C[l], c->wal[b].W[l], c->wal[b].O[l], c->wal[b].A[l]};
             for (void* q : wa) if (q) cudaFree(q);
@@ -623,6 +636,7 @@ extern "C" int bcg_set_field(bcg_ctx* c, int f, int level, const double* in, siz
     if (n < v.n) return BCG_E_ARG;
     if (v.mg == 2) return BCG_E_UNSUPPORTED;  /* the agar view is derived */
     mg_res0_materialise(c);                    /* before its inputs change */
+    if (f == BCG_F_INSIDE) c->host_bbox[0] = -1;
     if (v.mg == 1) { c->mg_clean = 0; nutrient_graphs_drop(c); }   /* Err/Res may no longer be zero */
     if (!v.mg) {
         BCG_CUDA_TRY(cudaMemcpy(v.ptr, in, v.n * 8, cudaMemcpyHostToDevice));
@@ -656,5 +670,6 @@ extern "C" int bcg_set_bbox(bcg_ctx* c, int minx, int maxx, int maxz)
     if (!c) return BCG_E_ARG;
     int h[3] = {minx, maxx, maxz};
     BCG_CUDA_TRY(cudaMemcpy(c->bbox, h, sizeof(h), cudaMemcpyHostToDevice));
+    c->host_bbox[0] = -1;          /* no longer the deposition's */
     return BCG_OK;
 }

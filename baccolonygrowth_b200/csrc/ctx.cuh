@@ -38,6 +38,10 @@ struct WallBuf {
     double *C[BCG_MAX_AGAR_LEVELS], *W[BCG_MAX_AGAR_LEVELS], *O[BCG_MAX_AGAR_LEVELS], *A[BCG_MAX_AGAR_LEVELS];
 };
 
+/* one buffer of the second set the blocked sweeps write to: an EnvBuf's four
+ * species and its walls, per level carbon, waste, acetate, oxygen rows */
+struct SweepBuf { double *C, *W, *A, *O, *wall; };
+
 struct bcg_ctx {
     bcg_params P;
     int device;
@@ -96,7 +100,11 @@ struct bcg_ctx {
     WallBuf wal[2];        /* [0] = FieldWall, [1] = oldFieldWall */
     double *rd, *inside, *rds, *ds, *dens, *rws, *wds, *rw, *wd;
     int* bbox;             /* device: minx, maxx, maxz (after +-5) */
+    /* bbox as the last deposition left it, 5 boxes around the inside points it
+     * marked; [0] = -1 once either may have changed */
     int host_bbox[3];
+    SweepBuf sweep2[2];    /* nutrients.cu */
+    unsigned char* sweep_type;
     MgLevel mg[BCG_MAX_MG_LEVELS];
     int mg_levels;
     double* mg_scratch;    /* reductions */
@@ -105,6 +113,7 @@ struct bcg_ctx {
     cudaGraphExec_t nutrient_graph[2];
     int nutrient_graph_sweeps;           /* 0: none captured (dropped whenever a kernel choice changes) */
     int nutrient_graph_launches[2];
+    int nutrient_graph_blocked;          /* tile of the blocked sweeps they hold (0: single sweeps) */
     /* the captured per-step solve (bcg_mg_solve): its key (V-cycles, wall
      * buffer, whether Err and Res were clean on entry; -1: none) */
     cudaGraphExec_t solve_graph;
@@ -174,3 +183,6 @@ int mg_tune_smoother(bcg_ctx* c, int* choice);
 void mg_res0_materialise(bcg_ctx* c);
 int mg_kernel_attributes();
 int mech_kernel_attributes();
+int sweep_kernel_attributes();
+/* read bbox into host_bbox; part of the status check that ends a deposition */
+int ctx_check_status_bbox(bcg_ctx* c);

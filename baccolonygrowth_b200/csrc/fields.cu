@@ -253,7 +253,7 @@ static int deposit(bcg_ctx* c, bool smooth)
     rc = launch_surface(c, smooth);
     if (rc) return rc;
     timer_end(c, BCG_T_DENSITY, 0);
-    return ctx_check_status(c);
+    return ctx_check_status_bbox(c);
 }
 
 extern "C" int bcg_update_density(bcg_ctx* c) { return c ? deposit(c, true) : BCG_E_ARG; }
@@ -264,6 +264,7 @@ extern "C" int bcg_update_height(bcg_ctx* c)
     if (!c) return BCG_E_ARG;
     const bcg_params& P = c->P;
     if (P.refinement_grid_height > 8) return BCG_E_UNSUPPORTED;
+    c->host_bbox[0] = -1;              /* the box follows the cells, insideColonyDen does not */
     timer_begin(c, BCG_T_DENSITY);
     int rc = bin_cells(c, c->cur);
     if (rc) return rc;

@@ -34,6 +34,12 @@ struct NutConst {
     double max_carbon, max_o2;
     double kw_ph, ka_ph, kb_ph, cb_ph, c1_ph;
     double inv_bl2, inv_g1s, inv_g2s, inv_g3s;   /* 1/BoxLength^2, 1/g1s, 1/g2s, 1/g3s */
+    double inv_dc, inv_do, inv_da, inv_dw;       /* 1/(colony + agar diffusivity) per species */
+    double inv_h2[BCG_MAX_AGAR_LEVELS];          /* 1/(BoxLength^2 4^level) */
+    int same_kc;                                 /* kc_aer == kc_ana: one carbon quotient serves both */
+    double mu1, mu2, mu3;                        /* max growth + maintenance: carbon aerobic, anaerobic, acetate */
+    double kc, kw, ka_, ko_;                     /* colony diffusivity cdt / BoxLength^2 per species */
+    double sdt;                                  /* cdt / 4 */
 };
 
 static NutConst nut_const(const bcg_ctx* c)
@@ -62,6 +68,13 @@ static NutConst nut_const(const bcg_ctx* c)
     n.kw_ph = P.kw_ph; n.ka_ph = P.ka_ph; n.kb_ph = P.kb_ph; n.cb_ph = P.cb_ph; n.c1_ph = P.c1_ph;
     n.inv_bl2 = 1.0 / (P.box_length * P.box_length);
     n.inv_g1s = 1.0 / n.g1s; n.inv_g2s = 1.0 / n.g2s; n.inv_g3s = 1.0 / n.g3s;
+    n.inv_dc = 1.0 / (n.dcc + n.dac); n.inv_do = 1.0 / (n.dco + n.dao);
+    n.inv_da = 1.0 / (n.dca + n.daa); n.inv_dw = 1.0 / (n.dcw + n.daw);
+    for (int l = 0; l < BCG_MAX_AGAR_LEVELS; l++) n.inv_h2[l] = 1.0 / (P.box_length * P.box_length * (double)(1LL << (2 * l)));
+    n.same_kc = P.kc_aer == P.kc_ana;
+    n.mu1 = n.max_gr_car_aer + n.mgrCarAers; n.mu2 = n.max_gr_car_ana + n.mgrCarAnas; n.mu3 = n.max_gr_ace_aer + n.mgrAceAers;
+    n.kc = n.dcc * n.inv_bl2 * n.cdt; n.kw = n.dcw * n.inv_bl2 * n.cdt; n.ka_ = n.dca * n.inv_bl2 * n.cdt; n.ko_ = n.dco * n.inv_bl2 * n.cdt;
+    n.sdt = 0.25 * n.cdt;
     return n;
 }
 
@@ -98,6 +111,115 @@ __device__ void buffer_solve(const NutConst& n, double Cac, double& pH, double& 
     hyd = x; acetic = y; buf = z;
 }
 
+/* uptake and production rates and growth of an inside point from the averages
+ * of the species around it (Nutrients.cpp:268-344) */
+struct Rates { double fC, fO, qO, qC, qA, pA, gca, gcn, gaa; };
+__device__ __forceinline__ Rates point_rates(const NutConst& n, double Cgr, double Ogr, double Agr)
+{
+    /* x / (x + k): for x = 0 and k > 0 the quotient is x itself, taken
+     * here without the division, whose zero dividend leaves its fast
+     * path (the species start at zero, acetate everywhere) */
+    double fCgr_aer = (Cgr == 0.0 && n.kc_aer > 0.0) ? Cgr : Cgr / (Cgr + n.kc_aer);
+    double fCgr_ana = n.same_kc ? fCgr_aer : ((Cgr == 0.0 && n.kc_ana > 0.0) ? Cgr : Cgr / (Cgr + n.kc_ana));
+    double fAgr = (Agr == 0.0 && n.ka > 0.0) ? Agr : Agr / (Agr + n.ka);
+    double fOgr = (Ogr == 0.0 && n.ko > 0.0) ? Ogr : Ogr / (Ogr + n.ko);
+    const double l1 = mx(fma(n.mu1, fCgr_aer, -n.mgrCarAers), 0.0);
+    const double l2 = mx(fma(n.mu2, fCgr_ana, -n.mgrCarAnas), 0.0);
+    const double l3 = mx(fma(n.mu3, fAgr, -n.mgrAceAers), 0.0);
+    const double m1 = mn(Cgr * n.inv_g1s, 1.0), m2 = mn(Cgr * n.inv_g2s, 1.0), m3 = mn(Agr * n.inv_g3s, 1.0);
+    /* aerobic on carbon, aerobic on acetate, anaerobic; every term below is a
+     * sum of non-negative products, so factoring them out costs no digits */
+    const double ac = fCgr_aer * fOgr, aa = (1 - fCgr_aer) * fOgr, an = 1 - fOgr;
+    const double qO = fma(ac, fma(n.q_o2_car, l1, n.q_o2_car_nt * m1), aa * fma(n.q_o2_ace, l3, n.q_o2_ace_nt * m3));
+    const double qC = fma(ac, fma(n.q_car_aer, l1, n.q_car_aer_nt * m1), an * fma(n.q_car_ana, l2, n.q_car_ana_nt * m2));
+    const double qA = aa * fma(n.q_ace_aer, l3, n.q_ace_aer_nt * m3);
+    const double pA = fma(ac, n.p_ace_aer * l1, an * fma(n.p_ace_ana, l2, n.p_ace_ana_nt * m2));
+    const double GrCarAer = l1 * ac, GrCarAna = l2 * an, GrAceAer = l3 * aa;
+    Rates r;
+    r.fC = fCgr_aer; r.fO = fOgr; r.qO = qO; r.qC = qC; r.qA = qA; r.pA = pA; r.gca = GrCarAer; r.gcn = GrCarAna; r.gaa = GrAceAer;
+    return r;
+}
+
+/* the four species at a point: carbon, waste, acetate, oxygen */
+struct Sp4 { double C, W, A, O; };
+
+/* an inside point's next values (Nutrients.cpp:346-440) from its own, its
+ * neighbours above (up), below (dn: the wall for z = 0) and beside, and its
+ * shifted density */
+__device__ __forceinline__ Sp4 inside_step(const NutConst& n, const Rates& r, const Sp4& c, const Sp4& up, const Sp4& dn,
+                                           const Sp4& xp, const Sp4& xm, double DS)
+{
+    /* c + D cdt / h^2 (the four neighbours - 4 c) + cdt (rates) DS / 4 */
+    const double sc = n.sdt * DS;
+    auto lap = [](double c0, double a, double b, double d, double e) { return fma(-4.0, c0, (a + b) + (d + e)); };
+    const double Cnew = fma(-r.qC, sc, fma(n.kc, lap(c.C, up.C, dn.C, xp.C, xm.C), c.C));
+    const double Anew = fma(r.pA - r.qA, sc, fma(n.ka_, lap(c.A, up.A, dn.A, xp.A, xm.A), c.A));
+    const double Onew = fma(-r.qO, sc, fma(n.ko_, lap(c.O, up.O, dn.O, xp.O, xm.O), c.O));
+    const double Wnew = fma(n.carbon_to_waste * r.qC, 4.0 * sc, fma(n.kw, lap(c.W, up.W, dn.W, xp.W, xm.W), c.W));
+    Sp4 v;
+    v.C = mx(0.0, mn(Cnew, n.max_carbon)); v.O = mx(0.0, mn(Onew, n.max_o2)); v.A = mx(0.0, Anew); v.W = mx(0.0, Wnew);
+    return v;
+}
+/* a ring point: the mean of its inside neighbours (b: 1 where inside; bd 0 at
+ * z = 0), oxygen at its maximum (Nutrients.cpp:442-500) */
+__device__ __forceinline__ Sp4 ring_step(const NutConst& n, int bp, int bm, int bu, int bd, const Sp4& xp, const Sp4& xm,
+                                         const Sp4& up, const Sp4& dn)
+{
+    const int den = bp + bm + bu + bd;
+    const double C = (xp.C * bp + xm.C * bm + up.C * bu + dn.C * bd) / den;
+    const double W = (xp.W * bp + xm.W * bm + up.W * bu + dn.W * bd) / den;
+    const double A = (xp.A * bp + xm.A * bm + up.A * bu + dn.A * bd) / den;
+    Sp4 v;
+    v.C = mx(0.0, mn(C, n.max_carbon)); v.O = mx(0.0, n.max_o2); v.A = mx(0.0, A); v.W = mx(0.0, W);
+    return v;
+}
+/* the wall of a colony column from the colony above it and the agar below
+ * (Nutrients.cpp:525-556) */
+__device__ __forceinline__ Sp4 wall_inside(const NutConst& n, const Sp4& e, const Sp4& g)
+{
+    Sp4 v;
+    v.C = mx(0.0, mn((n.dcc * e.C + n.dac * g.C) * n.inv_dc, n.max_carbon));
+    v.O = mx(0.0, mn((n.dco * e.O + n.dao * g.O) * n.inv_do, n.max_o2));
+    v.A = mx(0.0, (n.dca * e.A + n.daa * g.A) * n.inv_da);
+    v.W = mx(0.0, (n.dcw * e.W + n.daw * g.W) * n.inv_dw);
+    return v;
+}
+/* any other wall point: the second differences along the wall (xx) and to
+ * the agar below; p the previous value (oxygen not used) */
+__device__ __forceinline__ Sp4 wall_diffuse(const NutConst& n, double ih2, const Sp4& p, const Sp4& xx, const Sp4& g)
+{
+    const double Czz = 2.0 * (g.C - p.C) * ih2, Wzz = 2.0 * (g.W - p.W) * ih2, Azz = 2.0 * (g.A - p.A) * ih2;
+    Sp4 v;
+    v.C = mx(0.0, mn(p.C + n.dac * (xx.C + Czz) * n.cdt, n.max_carbon));
+    v.O = mx(0.0, n.max_o2);
+    v.A = mx(0.0, p.A + n.daa * (xx.A + Azz) * n.cdt);
+    v.W = mx(0.0, p.W + n.daw * (xx.W + Wzz) * n.cdt);
+    return v;
+}
+/* second differences along wall `level` at x (Nutrients.cpp:558-640); at(l, x)
+ * gives the previous wall */
+template <class At>
+__device__ __forceinline__ Sp4 wall_along(const NutConst& n, int level, int x, const Sp4& p, const At& at)
+{
+    const int X = n.X;
+    const double ih2 = n.inv_h2[level];
+    Sp4 v = {0.0, 0.0, 0.0, 0.0};
+    auto diff = [&](const Sp4& a, const Sp4& b, double f) {
+        v.C = (a.C + b.C - 2 * p.C) * f; v.W = (a.W + b.W - 2 * p.W) * f; v.A = (a.A + b.A - 2 * p.A) * f;
+    };
+    if (level > 0 && x >= X / 4 - 1 && x <= X * 3 / 4) {
+        if (x == X / 4 - 1) diff(at(level, x - 1), at(level - 1, 0), ih2);
+        else if (x == X * 3 / 4) diff(at(level, x + 1), at(level - 1, X - 2), ih2);
+    } else if (level < n.A - 1 && (x == 0 || x == X - 1)) {
+        if (x == 0) diff(at(level, x + 2), at(level + 1, X / 4 - 1), 0.25 * ih2);
+        else diff(at(level, x - 1), at(level + 1, X * 3 / 4), ih2);
+    } else if (level == n.A - 1 && (x == 0 || x == X - 1)) {
+        const Sp4 a = at(level, x == 0 ? 1 : X - 2);
+        v.C = (a.C - p.C) * ih2; v.W = (a.W - p.W) * ih2; v.A = (a.A - p.A) * ih2;
+    } else diff(at(level, x - 1), at(level, x + 1), ih2);
+    return v;
+}
+
 struct EnvP { double *C, *W, *A, *O, *gr1, *gr2, *ph, *hyd, *ace, *buf; };
 static EnvP envp(bcg_ctx* c, int b)
 {
@@ -106,6 +228,7 @@ static EnvP envp(bcg_ctx* c, int b)
     return p;
 }
 struct WallP { const double *C, *W, *O, *A; };
+__device__ __forceinline__ Sp4 env_at(const EnvP& e, size_t i) { return Sp4{e.C[i], e.W[i], e.A[i], e.O[i]}; }
 /* Environment's GrCarAer, GrCarAna, GrAceAer, qCarmnt, qAcemnt, pAcemnt,
  * qOxymnt (Nutrients.cpp:328-344); all null when the sweep's current
  * buffer is not Environment or its values do not survive the call */
@@ -159,85 +282,27 @@ __device__ __forceinline__ void colony_point(const NutConst& n, int x, int z, co
             buffer_solve(n, Agr, ph, hy, ac, bu);
             prev.ph[id] = ph; prev.hyd[id] = hy; prev.ace[id] = ac; prev.buf[id] = bu;
         }
-        /* x / (x + k): for x = 0 and k > 0 the quotient is x itself, taken
-         * here without the division, whose zero dividend leaves its fast
-         * path (the species start at zero, acetate everywhere) */
-        double fCgr_aer = (Cgr == 0.0 && n.kc_aer > 0.0) ? Cgr : Cgr / (Cgr + n.kc_aer);
-        double fCgr_ana = (Cgr == 0.0 && n.kc_ana > 0.0) ? Cgr : Cgr / (Cgr + n.kc_ana);
-        double fAgr = (Agr == 0.0 && n.ka > 0.0) ? Agr : Agr / (Agr + n.ka);
-        double fOgr = (Ogr == 0.0 && n.ko > 0.0) ? Ogr : Ogr / (Ogr + n.ko), fIgr = 0;
-        double l1 = mx((n.max_gr_car_aer + n.mgrCarAers) * fCgr_aer - n.mgrCarAers, 0.0);
-        double l2 = mx((n.max_gr_car_ana + n.mgrCarAnas) * fCgr_ana - n.mgrCarAnas, 0.0);
-        double l3 = mx((n.max_gr_ace_aer + n.mgrAceAers) * fAgr - n.mgrAceAers, 0.0);
-        double qO = (n.q_o2_car * l1 * fCgr_aer + n.q_o2_ace * l3 * (1 - fCgr_aer)) * fOgr * mx(1 - fIgr, 0.0) + n.q_o2_car_nt * mn((Cgr * n.inv_g1s), 1.0) * fCgr_aer * fOgr + n.q_o2_ace_nt * mn((Agr * n.inv_g3s), 1.0) * (1 - fCgr_aer) * fOgr;
-        double qC = (n.q_car_aer * l1 * fCgr_aer * fOgr + n.q_car_ana * l2 * (1 - fOgr)) * mx(1 - fIgr, 0.0) + n.q_car_aer_nt * mn((Cgr * n.inv_g1s), 1.0) * fCgr_aer * fOgr + n.q_car_ana_nt * mn((Cgr * n.inv_g2s), 1.0) * (1 - fOgr);
-        double qA = (n.q_ace_aer * l3 * (1 - fCgr_aer) * fOgr) * mx(1 - fIgr, 0.0) + n.q_ace_aer_nt * mn((Agr * n.inv_g3s), 1.0) * (1 - fCgr_aer) * fOgr;
-        double pA = (n.p_ace_aer * l1 * fCgr_aer * fOgr + n.p_ace_ana * l2 * (1 - fOgr)) * mx(1 - fIgr, 0.0) + n.p_ace_ana_nt * mn((Cgr * n.inv_g2s), 1.0) * (1 - fOgr);
-        double pW = n.carbon_to_waste * qC, qW = 0.0;
-        double GrCarAer = l1 * fCgr_aer * fOgr * mx(1 - fIgr, 0.0);
-        double GrCarAna = l2 * (1 - fOgr) * mx(1 - fIgr, 0.0);
-        double GrAceAer = l3 * (1 - fCgr_aer) * fOgr * mx(1 - fIgr, 0.0);
-        double gr = GrCarAer + GrCarAna + GrAceAer;
+        const Rates rt = point_rates(n, Cgr, Ogr, Agr);
+        const double gr = rt.gca + rt.gcn + rt.gaa;
         cur.gr1[id] = gr;
         cur.gr2[id] = gr;
         if (EXTRA && ex.gca) {
-            ex.qcm[id] = n.q_car_aer_nt * mn((Cgr * n.inv_g1s), 1.0) * fCgr_aer * fOgr + n.q_car_ana_nt * mn((Cgr * n.inv_g2s), 1.0) * (1 - fOgr);
-            ex.qam[id] = n.q_ace_aer_nt * mn((Agr * n.inv_g3s), 1.0) * (1 - fCgr_aer) * fOgr;
-            ex.pam[id] = n.p_ace_ana_nt * mn((Cgr * n.inv_g2s), 1.0) * (1 - fOgr);
-            ex.qom[id] = n.q_o2_car_nt * mn((Cgr * n.inv_g1s), 1.0) * fCgr_aer * fOgr + n.q_o2_ace_nt * mn((Agr * n.inv_g3s), 1.0) * (1 - fCgr_aer) * fOgr;
-            ex.gca[id] = GrCarAer; ex.gcn[id] = GrCarAna; ex.gaa[id] = GrAceAer;
+            ex.qcm[id] = n.q_car_aer_nt * mn((Cgr * n.inv_g1s), 1.0) * rt.fC * rt.fO + n.q_car_ana_nt * mn((Cgr * n.inv_g2s), 1.0) * (1 - rt.fO);
+            ex.qam[id] = n.q_ace_aer_nt * mn((Agr * n.inv_g3s), 1.0) * (1 - rt.fC) * rt.fO;
+            ex.pam[id] = n.p_ace_ana_nt * mn((Cgr * n.inv_g2s), 1.0) * (1 - rt.fO);
+            ex.qom[id] = n.q_o2_car_nt * mn((Cgr * n.inv_g1s), 1.0) * rt.fC * rt.fO + n.q_o2_ace_nt * mn((Agr * n.inv_g3s), 1.0) * (1 - rt.fC) * rt.fO;
+            ex.gca[id] = rt.gca; ex.gcn[id] = rt.gcn; ex.gaa[id] = rt.gaa;
         }
         if (!(x > 2)) { dev_error(st, BCG_E_NEED_MORE_BOXES, x); return; }
-        const double c0C = prev.C[id], c0W = prev.W[id], c0A = prev.A[id], c0O = prev.O[id];
-        const size_t up = IXZ(x, z + 1);
-        double Czz, Wzz, Azz, Ozz;
-        if (z == 0) {
-            Wzz = (prev.W[up] + pw0.W[x] - 2.0 * c0W) * n.inv_bl2;
-            Czz = (prev.C[up] + pw0.C[x] - 2.0 * c0C) * n.inv_bl2;
-            Azz = (prev.A[up] + pw0.A[x] - 2.0 * c0A) * n.inv_bl2;
-            Ozz = (prev.O[up] + pw0.O[x] - 2.0 * c0O) * n.inv_bl2;
-        } else {
-            const size_t dn = IXZ(x, z - 1);
-            Wzz = (prev.W[up] + prev.W[dn] - 2.0 * c0W) * n.inv_bl2;
-            Czz = (prev.C[up] + prev.C[dn] - 2.0 * c0C) * n.inv_bl2;
-            Azz = (prev.A[up] + prev.A[dn] - 2.0 * c0A) * n.inv_bl2;
-            Ozz = (prev.O[up] + prev.O[dn] - 2.0 * c0O) * n.inv_bl2;
-        }
-        const size_t xp = IXZ(x + 1, z), xm = IXZ(x - 1, z);
-        double Cxx = (prev.C[xp] + prev.C[xm] - 2.0 * c0C) * n.inv_bl2;
-        double Wxx = (prev.W[xp] + prev.W[xm] - 2.0 * c0W) * n.inv_bl2;
-        double Axx = (prev.A[xp] + prev.A[xm] - 2.0 * c0A) * n.inv_bl2;
-        double Oxx = (prev.O[xp] + prev.O[xm] - 2.0 * c0O) * n.inv_bl2;
-        double DS = ds[id];
-        double Cnew = c0C + (n.dcc * (Cxx + Czz) - qC * 0.25 * DS) * n.cdt;
-        double CAcenew = c0A + (n.dca * (Axx + Azz) + pA * 0.25 * DS - qA * 0.25 * DS) * n.cdt;
-        double Onew = c0O + (n.dco * (Oxx + Ozz) - qO * 0.25 * DS) * n.cdt;
-        cur.C[id] = mx(0.0, mn(Cnew, n.max_carbon));
-        cur.O[id] = mx(0.0, mn(Onew, n.max_o2));
-        cur.A[id] = mx(0.0, CAcenew);
-        double Wnew = c0W + (n.dcw * (Wxx + Wzz) + pW * DS - qW * DS) * n.cdt;
-        cur.W[id] = mx(0.0, Wnew);
+        const Sp4 dn = z == 0 ? Sp4{pw0.C[x], pw0.W[x], pw0.A[x], pw0.O[x]} : env_at(prev, IXZ(x, z - 1));
+        const Sp4 v = inside_step(n, rt, env_at(prev, id), env_at(prev, IXZ(x, z + 1)), dn, env_at(prev, IXZ(x + 1, z)),
+                                  env_at(prev, IXZ(x - 1, z)), ds[id]);
+        cur.C[id] = v.C; cur.O[id] = v.O; cur.A[id] = v.A; cur.W[id] = v.W;
     } else if (ins > 0.3) {
-        const size_t ixp = IXZ(x + 1, z), ixm = IXZ(x - 1, z), iu = IXZ(x, z + 1);
-        int bp = inside[ixp] > 0.5, bm = inside[ixm] > 0.5, bu = inside[iu] > 0.5;
-        double Cnew, Wnew, CAcenew;
-        if (z > 0) {
-            const size_t id_ = IXZ(x, z - 1);
-            int bd = inside[id_] > 0.5;
-            int den = bp + bm + bu + bd;
-            Cnew = (prev.C[ixp] * bp + prev.C[ixm] * bm + prev.C[iu] * bu + prev.C[id_] * bd) / den;
-            Wnew = (prev.W[ixp] * bp + prev.W[ixm] * bm + prev.W[iu] * bu + prev.W[id_] * bd) / den;
-            CAcenew = (prev.A[ixp] * bp + prev.A[ixm] * bm + prev.A[iu] * bu + prev.A[id_] * bd) / den;
-        } else {
-            int den = bp + bm + bu;
-            Cnew = (prev.C[ixp] * bp + prev.C[ixm] * bm + prev.C[iu] * bu) / den;
-            Wnew = (prev.W[ixp] * bp + prev.W[ixm] * bm + prev.W[iu] * bu) / den;
-            CAcenew = (prev.A[ixp] * bp + prev.A[ixm] * bm + prev.A[iu] * bu) / den;
-        }
-        cur.C[id] = mx(0.0, mn(Cnew, n.max_carbon));
-        cur.O[id] = mx(0.0, mn(n.max_o2, n.max_o2));
-        cur.A[id] = mx(0.0, CAcenew);
-        cur.W[id] = mx(0.0, Wnew);
+        const size_t ixp = IXZ(x + 1, z), ixm = IXZ(x - 1, z), iu = IXZ(x, z + 1), id_ = z > 0 ? IXZ(x, z - 1) : id;
+        const int bp = inside[ixp] > 0.5, bm = inside[ixm] > 0.5, bu = inside[iu] > 0.5, bd = z > 0 && inside[id_] > 0.5;
+        const Sp4 v = ring_step(n, bp, bm, bu, bd, env_at(prev, ixp), env_at(prev, ixm), env_at(prev, iu), env_at(prev, id_));
+        cur.C[id] = v.C; cur.O[id] = v.O; cur.A[id] = v.A; cur.W[id] = v.W;
     }
 #undef IXZ
 }
@@ -264,69 +329,15 @@ struct AgarRow { const double *C[BCG_MAX_AGAR_LEVELS], *O[BCG_MAX_AGAR_LEVELS], 
 __device__ __forceinline__ void wall_point(const NutConst& n, int level, int x, const EnvP& curenv, const AgarRow& ag,
                                            const WallAll& cw, const WallAll& pw, const double* __restrict__ inside)
 {
-    const int X = n.X;
-    if (level == 0 && inside[(size_t)x * n.Z] > 0.5) {
-        size_t i0 = (size_t)x * n.Z;
-        double gC = ag.C[0][x], gO = ag.O[0][x], gA = ag.A[0][x], gW = ag.W[0] ? ag.W[0][x] : 0.0;
-        double Cnew = (n.dcc * curenv.C[i0] + n.dac * gC) / (n.dcc + n.dac);
-        double Onew = (n.dco * curenv.O[i0] + n.dao * gO) / (n.dco + n.dao);
-        cw.C[0][x] = mx(0.0, mn(Cnew, n.max_carbon));
-        cw.O[0][x] = mx(0.0, mn(Onew, n.max_o2));
-        double CAcenew = (n.dca * curenv.A[i0] + n.daa * gA) / (n.dca + n.daa);
-        cw.A[0][x] = mx(0.0, CAcenew);
-        double Wnew = (n.dcw * curenv.W[i0] + n.daw * gW) / (n.dcw + n.daw);
-        cw.W[0][x] = mx(0.0, Wnew);
-        return;
+    const Sp4 g = {ag.C[level][x], ag.W[level] ? ag.W[level][x] : 0.0, ag.A[level][x], ag.O[level] ? ag.O[level][x] : 0.0};
+    Sp4 v;
+    if (level == 0 && inside[(size_t)x * n.Z] > 0.5) v = wall_inside(n, env_at(curenv, (size_t)x * n.Z), g);
+    else {
+        auto at = [&](int l, int i) { return Sp4{pw.C[l][i], pw.W[l][i], pw.A[l][i], 0.0}; };
+        const Sp4 p = at(level, x);
+        v = wall_diffuse(n, n.inv_h2[level], p, wall_along(n, level, x, p, at), g);
     }
-    const double* pC = pw.C[level];
-    const double* pW = pw.W[level];
-    const double* pA = pw.A[level];
-    double h2l = n.BL * n.BL * pow(4.0, (double)level);
-    double Cxx = 0, Wxx = 0, Axx = 0;
-    if (level > 0 && (x >= X / 4 - 1) && x <= X * 3 / 4) {
-        if (x == X / 4 - 1) {
-            Wxx = (pW[x - 1] + pw.W[level - 1][0] - 2 * pW[x]) / h2l;
-            Cxx = (pC[x - 1] + pw.C[level - 1][0] - 2 * pC[x]) / h2l;
-            Axx = (pA[x - 1] + pw.A[level - 1][0] - 2 * pA[x]) / h2l;
-        } else if (x == X * 3 / 4) {
-            Wxx = (pW[x + 1] + pw.W[level - 1][X - 2] - 2 * pW[x]) / h2l;
-            Cxx = (pC[x + 1] + pw.C[level - 1][X - 2] - 2 * pC[x]) / h2l;
-            Axx = (pA[x + 1] + pw.A[level - 1][X - 2] - 2 * pA[x]) / h2l;
-        }
-    } else if (level < n.A - 1 && (x == 0 || x == X - 1)) {
-        const int ly = 0;
-        if (x == 0) {
-            const int q = X / 4 - 1;
-            Wxx = (pW[x + 2] + 1.0 / (ly + 1) * pw.W[level + 1][q] + ly * 1.0 / (ly + 1) * pw.W[level + 1][q] - 2 * pW[x]) / 4 / h2l;
-            Cxx = (pC[x + 2] + 1.0 / (ly + 1) * pw.C[level + 1][q] + ly * 1.0 / (ly + 1) * pw.C[level + 1][q] - 2 * pC[x]) / 4 / h2l;
-            Axx = (pA[x + 2] + 1.0 / (ly + 1) * pw.A[level + 1][q] + ly * 1.0 / (ly + 1) * pw.A[level + 1][q] - 2 * pA[x]) / 4 / h2l;
-        } else {
-            const int q = X * 3 / 4;
-            Wxx = (pW[x - 1] + 1.0 / (ly + 1) * pw.W[level + 1][q] + ly * 1.0 / (ly + 1) * pw.W[level + 1][q] - 2 * pW[x]) / h2l;
-            Cxx = (pC[x - 1] + 1.0 / (ly + 1) * pw.C[level + 1][q] + ly * 1.0 / (ly + 1) * pw.C[level + 1][q] - 2 * pC[x]) / h2l;
-            Axx = (pA[x - 1] + 1.0 / (ly + 1) * pw.A[level + 1][q] + ly * 1.0 / (ly + 1) * pw.A[level + 1][q] - 2 * pA[x]) / h2l;
-        }
-    } else if (level == n.A - 1 && (x == 0 || x == X - 1)) {
-        int s1 = (x == 0) ? 1 : X - 2;
-        Wxx = (pW[s1] - 1.0 * pW[x]) / h2l;
-        Cxx = (pC[s1] - 1.0 * pC[x]) / h2l;
-        Axx = (pA[s1] - 1.0 * pA[x]) / h2l;
-    } else {
-        Wxx = (pW[x - 1] + pW[x + 1] - 2 * pW[x]) / h2l;
-        Cxx = (pC[x - 1] + pC[x + 1] - 2 * pC[x]) / h2l;
-        Axx = (pA[x - 1] + pA[x + 1] - 2 * pA[x]) / h2l;
-    }
-    double gC = ag.C[level][x], gA = ag.A[level][x], gW = ag.W[level] ? ag.W[level][x] : 0.0;
-    double Wzz = 2.0 * (gW - pW[x]) / h2l;
-    double Czz = 2.0 * (gC - pC[x]) / h2l;
-    double Azz = 2.0 * (gA - pA[x]) / h2l;
-    double Cnew = pC[x] + n.dac * (Cxx + Czz) * n.cdt;
-    cw.C[level][x] = mx(0.0, mn(Cnew, n.max_carbon));
-    cw.O[level][x] = mx(0.0, mn(n.max_o2, n.max_o2));
-    double CAcenew = pA[x] + n.daa * (Axx + Azz) * n.cdt;
-    cw.A[level][x] = mx(0.0, CAcenew);
-    double Wnew = pW[x] + n.daw * (Wxx + Wzz) * n.cdt;
-    cw.W[level][x] = mx(0.0, Wnew);
+    cw.C[level][x] = v.C; cw.W[level][x] = v.W; cw.A[level][x] = v.A; cw.O[level][x] = v.O;
 }
 
 static AgarRow agar_rows(bcg_ctx* c)
@@ -375,6 +386,322 @@ static void sweep_launch(dim3 grid, dim3 block, bcg_ctx* c, const NutConst& n, E
 #undef SWEEP
 }
 
+/* ---- several sweeps in one launch ----------------------------------------- */
+/* A launch a sweep is bound by its chain at small colonies (dependent loads, three
+ * quotients, the wall: 8 to 9 us whatever the size) and by instructions at large
+ * ones (19 us at a million cells).  Here a block
+ * keeps a tile of both environment buffers in shared memory with a halo of
+ * SW_K points and runs SW_K sweeps on it, each recomputing the halo as far as
+ * the next one needs it; in both buffers the points that no sweep writes keep
+ * their own values.  The level-0 wall over the tile is its row below z = 0 and
+ * runs along.  The rest of the wall (level 0 beside the bounding box, the other
+ * levels) depends on nothing in the colony for SW_K sweeps, since the box is
+ * wider than the colony by 5: blocks of its own take it.  Results go
+ * to a second set of buffers, which the next launch reads.
+ * Measured a sweep, launches included: 33 thousand cells 8.9 -> 3.1 us (tiles of
+ * 4), a million 19 -> 14.6 us (tiles of 16).  It is bound by instruction issue: 0.64
+ * a cycle and scheduler at a million cells, 1.6 points computed for one owned. */
+#define SW_K 4               /* sweeps a launch, even: the buffers' roles return */
+#define SW_RZ 40             /* rows of a tile with its halo */
+#define SW_OWN0 (SW_RZ - 1 - SW_K)        /* rows z = 0 .. of the bottom tile where others follow */
+#define SW_OWN (SW_RZ - 2 * SW_K)         /* rows of the tiles above it */
+/* A tile's columns.  16 recompute least (1.6 points for one) and fill the SMs
+ * from about 150 tiles on; fewer tiles leave SMs idle and a block's own chain of
+ * instructions is what counts, so smaller tiles with a thread a point. */
+template <int TX> struct SwTile {
+    static constexpr int RX = TX + 2 * SW_K, PTS = RX * SW_RZ, THREADS = TX == 16 ? 480 : PTS;
+    static constexpr int SMEM = PTS * (8 * 8 + 8 + 1) + RX * 3 * 8;
+};
+/* types of a point: 1 inside and swept, 2 ring and swept; bits 2..5 the ring's
+ * inside neighbours (x+1, x-1, z+1, z-1); bit 6 inside (the wall's test) */
+struct SweepSet { EnvP e[2]; WallAll w[2]; };
+
+/* the points' types, and the second set's points as the first has them (those
+ * no sweep writes must hold the same in both) */
+__global__ void k_sweep_types(NutConst n, const int* __restrict__ bbox, SweepSet a, SweepSet b, const double* __restrict__ inside,
+                              const double* __restrict__ ds, unsigned char* __restrict__ type)
+{
+    const int X = n.X, Z = n.Z, id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= X * Z) return;
+    const int x = id / Z, z = id - x * Z;
+    int t = inside[id] > 0.5 ? 64 : 0;
+    if (x >= bbox[0] && x <= bbox[1] && z <= bbox[2] && ds[id] > DBL_EPSILON && x >= 1 && x <= X - 2 && z <= Z - 2) {
+        if (t) t |= 1;
+        else if (inside[id] > 0.3)
+            t |= 2 | (inside[id + Z] > 0.5 ? 4 : 0) | (inside[id - Z] > 0.5 ? 8 : 0) | (inside[id + 1] > 0.5 ? 16 : 0) |
+                 (z > 0 && inside[id - 1] > 0.5 ? 32 : 0);
+    }
+    type[id] = (unsigned char)t;
+    for (int q = 0; q < 2; q++) {
+        b.e[q].C[id] = a.e[q].C[id]; b.e[q].W[id] = a.e[q].W[id]; b.e[q].A[id] = a.e[q].A[id]; b.e[q].O[id] = a.e[q].O[id];
+    }
+}
+
+/* The wall outside the tiles: level 0 left of minx and right of maxx, all of the
+ * other levels.  Joined where the levels couple, the points whose second
+ * difference is not 0 form one line:
+ *   level A-1: x = 0 .. X/4-1, ..., level 1: 0 .. X/4-1, level 0: 0 .. X-1,
+ *   level 1: 3X/4 .. X-1, ..., level A-1: 3X/4 .. X-1,
+ * a point's neighbours being the line's, but for a level's x = 0, which takes
+ * the second one to the right, and its x = 3X/4, the second one to the left.  A
+ * block carries SW_LINE of them, with a halo on both sides, through the SW_K
+ * sweeps in shared memory.  Level-0 columns under the box belong to the tiles;
+ * those next to its edges are carried as halo (they are no colony columns),
+ * and what the others get here stays too far off to be read.  The points between
+ * X/4 and 3X/4 of the upper levels depend on themselves alone. */
+#define SW_LINE 256
+#define SW_LHALO (2 * SW_K)
+__device__ void sweep_walls(const NutConst& n, int block, int minx, int maxx, const SweepSet& src, const SweepSet& dst,
+                            const AgarRow& ag, int b0, double* sm, int threads)
+{
+    const int X = n.X, A = n.A, nl = X / 4, x3 = X * 3 / 4, nr = X - x3, L0 = (A - 1) * nl, total = L0 + X + (A - 1) * nr;
+    const int lines = (total + SW_LINE - 1) / SW_LINE;
+    if (block >= lines) {
+        const int f = (block - lines) * threads + threadIdx.x, nm = x3 - nl;
+        if (f >= (A - 1) * nm) return;
+        const int l = 1 + f / nm, x = nl + f % nm;
+        const Sp4 g = {ag.C[l][x], 0.0, ag.A[l][x], 0.0}, none = {0.0, 0.0, 0.0, 0.0};
+        const WallAll& w = src.w[b0 ^ 1];
+        Sp4 v = {w.C[l][x], w.W[l][x], w.A[l][x], 0.0};
+        for (int s = 0; s < SW_K; s++) {
+            v = wall_diffuse(n, n.inv_h2[l], v, none, g);
+            if (s >= SW_K - 2) {
+                const WallAll& d = dst.w[b0 ^ (s & 1)];
+                d.C[l][x] = v.C; d.W[l][x] = v.W; d.A[l][x] = v.A; d.O[l][x] = v.O;
+            }
+        }
+        return;
+    }
+    constexpr int N = SW_LINE + 2 * SW_LHALO;
+    static_assert(N <= SwTile<16>::THREADS && N <= SwTile<4>::THREADS, "a thread a point");
+    const int q = threadIdx.x, pos = block * SW_LINE - SW_LHALO + q;
+    const bool on = q < N && pos >= 0 && pos < total;
+    int l = 0, x = 0, left = q - 1, right = q + 1;
+    double f = 0.0;
+    bool first = false, end = false;
+    Sp4 g = {0.0, 0.0, 0.0, 0.0};
+    if (on) {
+        if (pos < L0) { l = A - 1 - pos / nl; x = pos % nl; }
+        else if (pos < L0 + X) x = pos - L0;
+        else { const int r = pos - L0 - X; l = 1 + r / nr; x = x3 + r % nr; }
+        f = n.inv_h2[l];
+        if (x == 0 && l < A - 1) { right = q + 2; f *= 0.25; }
+        if (l > 0 && x == x3) left = q - 2;
+        first = l == A - 1 && x == 0; end = l == A - 1 && x == X - 1;
+        g.C = ag.C[l][x]; g.A = ag.A[l][x];
+        for (int b = 0; b < 2; b++) {
+            const WallAll& w = src.w[b];
+            double* m = sm + 3 * b * N + q;
+            m[0] = w.C[l][x]; m[N] = w.W[l][x]; m[2 * N] = w.A[l][x];
+        }
+    }
+    const bool mine = on && q >= SW_LHALO && q < SW_LHALO + SW_LINE && !(l == 0 && x >= minx && x <= maxx);
+    /* the halo's outer points go stale two at a time */
+    const bool step = on && (first || left >= 0) && (end || right < N) && (first || pos > 0) && (end || pos + 1 < total);
+    __syncthreads();
+    for (int s = 0; s < SW_K; s++) {
+        const int b = b0 ^ (s & 1);
+        if (step) {
+            const double* m = sm + 3 * (b ^ 1) * N;
+            const Sp4 p = {m[q], m[N + q], m[2 * N + q], 0.0};
+            Sp4 xx;
+            if (first || end) {
+                const int o = first ? q + 1 : q - 1;
+                xx.C = (m[o] - p.C) * f; xx.W = (m[N + o] - p.W) * f; xx.A = (m[2 * N + o] - p.A) * f;
+            } else {
+                xx.C = (m[left] + m[right] - 2 * p.C) * f; xx.W = (m[N + left] + m[N + right] - 2 * p.W) * f;
+                xx.A = (m[2 * N + left] + m[2 * N + right] - 2 * p.A) * f;
+            }
+            const Sp4 v = wall_diffuse(n, n.inv_h2[l], p, xx, g);
+            double* c = sm + 3 * b * N + q;
+            c[0] = v.C; c[N] = v.W; c[2 * N] = v.A;
+            if (mine && s >= SW_K - 2) {
+                const WallAll& d = dst.w[b];
+                d.C[l][x] = v.C; d.W[l][x] = v.W; d.A[l][x] = v.A; d.O[l][x] = v.O;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+/* b0: the buffer the first sweep writes; even: the first sweep's count is even */
+template <int TX>
+__global__ void __launch_bounds__(SwTile<TX>::THREADS, TX == 16 ? 2 : 1) k_sweep_block(const __grid_constant__ NutConst n, const int* __restrict__ bbox,
+                                                            const __grid_constant__ SweepSet src, const __grid_constant__ SweepSet dst,
+                                                            const unsigned char* __restrict__ type, const double* __restrict__ ds,
+                                                            const __grid_constant__ AgarRow ag, int b0, int even)
+{
+    constexpr int RX = SwTile<TX>::RX, P = SwTile<TX>::PTS, R = SW_RZ, THREADS = SwTile<TX>::THREADS;
+    const int minx = bbox[0], maxx = bbox[1], maxz = bbox[2], X = n.X, Z = n.Z, th = threadIdx.x;
+    extern __shared__ __align__(16) unsigned char sw_smem[];
+    if (blockIdx.y == 0) {
+        sweep_walls(n, blockIdx.x, minx, maxx, src, dst, ag, b0, reinterpret_cast<double*>(sw_smem), THREADS);
+        return;
+    }
+    const int zt = blockIdx.y - 1, x0 = minx + blockIdx.x * TX;
+    const bool floor_ = zt == 0;
+    const int z0 = floor_ ? 0 : SW_OWN0 + (zt - 1) * SW_OWN;
+    if (x0 > maxx || z0 > maxz) return;
+    /* a bottom tile that reaches over the box's top has no tile above */
+    const int z1 = floor_ ? (maxz + 2 < SW_RZ ? maxz + 1 : SW_OWN0) : z0 + SW_OWN;
+    const int zb = floor_ ? -1 : z0 - SW_K, xb = x0 - SW_K;       /* of row and column 0 */
+    double* v = reinterpret_cast<double*>(sw_smem);              /* [buffer][species][column][row] */
+    double* sds = v + 8 * P;
+    double* sag = sds + P;                                  /* [carbon, acetate, oxygen][column] */
+    unsigned char* st = reinterpret_cast<unsigned char*>(sag + 3 * RX);
+#pragma unroll 3
+    for (int q = th; q < P; q += THREADS) {
+        const int xi = q / R, r = q - xi * R, x = xb + xi, z = zb + r;
+        double e[8] = {0, 0, 0, 0, 0, 0, 0, 0}, d = 0.0;
+        int t = 0;
+        if (x >= 0 && x < X && z < Z) {
+            if (z >= 0) {
+                const size_t id = (size_t)x * Z + z;
+#pragma unroll
+                for (int b = 0; b < 2; b++) { e[4 * b] = src.e[b].C[id]; e[4 * b + 1] = src.e[b].W[id]; e[4 * b + 2] = src.e[b].A[id]; e[4 * b + 3] = src.e[b].O[id]; }
+                d = ds[id];
+                t = type[id];
+            } else {
+#pragma unroll
+                for (int b = 0; b < 2; b++) { e[4 * b] = src.w[b].C[0][x]; e[4 * b + 1] = src.w[b].W[0][x]; e[4 * b + 2] = src.w[b].A[0][x]; e[4 * b + 3] = src.w[b].O[0][x]; }
+                sag[xi] = ag.C[0][x]; sag[RX + xi] = ag.A[0][x]; sag[2 * RX + xi] = ag.O[0][x];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k * P + q] = e[k];
+        sds[q] = d;
+        st[q] = (unsigned char)t;
+    }
+    __syncthreads();
+    for (int s = 0; s < SW_K; s++) {
+        const int b = b0 ^ (s & 1);
+        const bool wall_first = (even != 0) == ((s & 1) == 0);
+        double* cur = v + 4 * b * P;
+        const double* prev = v + 4 * (b ^ 1) * P;
+        auto at = [&](int i) { return Sp4{prev[i], prev[P + i], prev[2 * P + i], prev[3 * P + i]}; };
+        auto put = [&](int i, const Sp4& a) { cur[i] = a.C; cur[P + i] = a.W; cur[2 * P + i] = a.A; cur[3 * P + i] = a.O; };
+        for (int q = th; q < P; q += THREADS) {
+            const int xi = q / R, r = q - xi * R, t = st[q];
+            if (xi == 0 || xi == RX - 1 || r == R - 1) continue;
+            if (r == 0) {
+                /* the wall beside the colony's columns */
+                if (floor_ && !(st[q + 1] & 64) && xb + xi >= 1 && xb + xi <= X - 2) {
+                    const Sp4 p = at(q), a = at(q - R), c = at(q + R), g = {sag[xi], 0.0, sag[RX + xi], 0.0};
+                    const double f = n.inv_h2[0];
+                    const Sp4 xx = {(a.C + c.C - 2 * p.C) * f, (a.W + c.W - 2 * p.W) * f, (a.A + c.A - 2 * p.A) * f, 0.0};
+                    put(q, wall_diffuse(n, f, p, xx, g));
+                }
+                continue;
+            }
+            /* the wall of a colony column, in the order of its z = 0 point */
+            auto wall = [&]() {
+                const Sp4 e = {cur[q], cur[P + q], cur[2 * P + q], cur[3 * P + q]};
+                const Sp4 g = {sag[xi], 0.0, sag[RX + xi], sag[2 * RX + xi]};
+                put(q - 1, wall_inside(n, e, g));
+            };
+            const bool own_wall = floor_ && r == 1 && (t & 64);
+            if (own_wall && wall_first) wall();
+            if (t & 1) {
+                const Sp4 c = at(q), dn = at(q - 1), xm = at(q - R);
+                const double dC = prev[q - R - 1], dA = prev[2 * P + q - R - 1], dO = prev[3 * P + q - R - 1];
+                const double Cgr = (dC + xm.C + dn.C + c.C) * 0.25, Ogr = (dO + xm.O + dn.O + c.O) * 0.25, Agr = (dA + xm.A + dn.A + c.A) * 0.25;
+                put(q, inside_step(n, point_rates(n, Cgr, Ogr, Agr), c, at(q + 1), dn, at(q + R), xm, sds[q]));
+            } else if (t & 2) {
+                put(q, ring_step(n, t >> 2 & 1, t >> 3 & 1, t >> 4 & 1, t >> 5 & 1, at(q + R), at(q - R), at(q + 1), at(q - 1)));
+            }
+            if (own_wall && !wall_first) wall();
+        }
+        __syncthreads();
+    }
+#pragma unroll 3
+    for (int q = th; q < P; q += THREADS) {
+        const int xi = q / R, r = q - xi * R, x = xb + xi, z = zb + r;
+        if (xi < SW_K || xi >= SW_K + TX || x > maxx) continue;
+        if (z < 0) {
+            if (!floor_) continue;
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+                dst.w[b].C[0][x] = v[4 * b * P + q]; dst.w[b].W[0][x] = v[(4 * b + 1) * P + q];
+                dst.w[b].A[0][x] = v[(4 * b + 2) * P + q]; dst.w[b].O[0][x] = v[(4 * b + 3) * P + q];
+            }
+        } else if (z >= z0 && z < z1 && (st[q] & 3)) {
+            const size_t id = (size_t)x * Z + z;
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+                dst.e[b].C[id] = v[4 * b * P + q]; dst.e[b].W[id] = v[(4 * b + 1) * P + q];
+                dst.e[b].A[id] = v[(4 * b + 2) * P + q]; dst.e[b].O[id] = v[(4 * b + 3) * P + q];
+            }
+        }
+    }
+}
+
+/* Whether the box is the deposition's (its margin keeps the colony off the
+ * columns that the tiles and the wall block share) and the tiles with their halos
+ * keep off the grid's sides, where the wall couples to the next level. */
+static bool sweeps_block(const bcg_ctx* c)
+{
+    const int* b = c->host_bbox;
+    return b[0] >= SW_K + 2 && b[1] <= c->P.box_x - SW_K - 3 && b[1] - b[0] >= 2 * SW_K && b[2] >= 0 && b[2] < c->P.box_z;
+}
+static SweepSet sweep_set(bcg_ctx* c, int second)
+{
+    SweepSet s;
+    for (int b = 0; b < 2; b++) {
+        s.e[b] = envp(c, b);
+        s.w[b] = wall_all(c, b);
+        if (second) {
+            const SweepBuf& t = c->sweep2[b];
+            s.e[b].C = t.C; s.e[b].W = t.W; s.e[b].A = t.A; s.e[b].O = t.O;
+            for (int l = 0; l < c->P.max_levels_mg; l++) {
+                double* w = t.wall + (size_t)l * 4 * c->P.box_x;
+                s.w[b].C[l] = w; s.w[b].W[l] = w + c->P.box_x; s.w[b].A[l] = w + 2 * (size_t)c->P.box_x; s.w[b].O[l] = w + 3 * (size_t)c->P.box_x;
+            }
+        }
+    }
+    return s;
+}
+/* columns of a tile for the box the host knows: 0 for single sweeps */
+static int sweep_tile(const bcg_ctx* c)
+{
+    if (!sweeps_block(c)) return 0;
+    const int* b = c->host_bbox;
+    const int w = b[1] - b[0] + 1, zt = b[2] + 2 < SW_RZ ? 1 : 1 + (b[2] + 1 - SW_OWN0 + SW_OWN - 1) / SW_OWN;
+    for (int tx = 4; tx < 16; tx *= 2) if ((w + tx - 1) / tx * zt <= 148) return tx;
+    return 16;
+}
+template <int TX>
+static void launch_sweep_block(bcg_ctx* c, const NutConst& nc, const SweepSet& from, const SweepSet& to, const AgarRow& ag, int ce, int even)
+{
+    const int X = nc.X, Z = nc.Z;
+    const dim3 grid((unsigned)((X + TX - 1) / TX), (unsigned)(2 + (Z > SW_OWN0 ? (Z - SW_OWN0 + SW_OWN - 1) / SW_OWN : 0)));
+    k_sweep_block<TX><<<grid, SwTile<TX>::THREADS, SwTile<TX>::SMEM, c->stream>>>(nc, c->bbox, from, to, c->sweep_type, c->ds, ag, ce, even);
+}
+/* as many of the next `n` sweeps as fit an even number of launches */
+static int run_sweep_blocks(bcg_ctx* c, const NutConst& nc, const AgarRow& ag, int n, int ce, int count)
+{
+    const int launches = n / SW_K & ~1, tx = sweep_tile(c);
+    if (launches <= 0 || !tx) return 0;
+    const SweepSet a = sweep_set(c, 0), b = sweep_set(c, 1);
+    const int X = nc.X, Z = nc.Z;
+    k_sweep_types<<<(unsigned)((X * Z + 255) / 256), 256, 0, c->stream>>>(nc, c->bbox, a, b, c->inside, c->ds, c->sweep_type);
+    for (int j = 0; j < launches; j++) {
+        const SweepSet &from = j & 1 ? b : a, &to = j & 1 ? a : b;
+        if (tx == 4) launch_sweep_block<4>(c, nc, from, to, ag, ce, count % 2 == 0);
+        else if (tx == 8) launch_sweep_block<8>(c, nc, from, to, ag, ce, count % 2 == 0);
+        else launch_sweep_block<16>(c, nc, from, to, ag, ce, count % 2 == 0);
+    }
+    c->launches += launches + 1;
+    return launches * SW_K;
+}
+int sweep_kernel_attributes()
+{
+    if (cudaFuncSetAttribute(k_sweep_block<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SwTile<4>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(k_sweep_block<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, SwTile<8>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(k_sweep_block<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, SwTile<16>::SMEM) != cudaSuccess)
+        return BCG_E_CUDA;
+    return BCG_OK;
+}
+
 /* `nsweeps` sweeps with the local buffer indices (ce = current colony
  * buffer, cw = current wall buffer) and sweep counter, as the reference's
  * loop keeps them (Multigrid.cpp:1017-1120); diag_from = first sweep index
@@ -386,7 +713,13 @@ static void run_sweeps(bcg_ctx* c, int nsweeps, int& ce, int& cwb, int& count, i
     AgarRow ag = agar_rows(c);
     /* at least one z block: its first A lanes carry the wall rows */
     const dim3 gcol((unsigned)((Z + 31) / 32), (unsigned)((X + COLONY_COLS - 1) / COLONY_COLS)), bcol(32, COLONY_COLS);
-    for (int j = 0; j < nsweeps; j++) {
+    int j0 = 0;
+    if (c->P.nutrient_gsi == 0) {
+        const int plain = diag_from < nsweeps ? diag_from : nsweeps;
+        if (ce == cwb) j0 = run_sweep_blocks(c, n, ag, plain, ce, count);
+        count += j0;
+    }
+    for (int j = j0; j < nsweeps; j++) {
         EnvP cur = envp(c, ce), prev = envp(c, ce ^ 1);
         WallAll cw = wall_all(c, cwb), pw = wall_all(c, cwb ^ 1);
         WallP pw0 = {pw.C[0], pw.W[0], pw.O[0], pw.A[0]};
@@ -434,9 +767,11 @@ void nutrient_graphs_drop(bcg_ctx* c)
 
 static int nutrient_unit_graph(bcg_ctx* c, int sweeps, int last, cudaGraphExec_t* out)
 {
-    if (c->nutrient_graph_sweeps != sweeps) {
+    const int blocked = sweep_tile(c);
+    if (c->nutrient_graph_sweeps != sweeps || c->nutrient_graph_blocked != blocked) {
         nutrient_graphs_drop(c);
         c->nutrient_graph_sweeps = sweeps;
+        c->nutrient_graph_blocked = blocked;
     }
     if (!c->nutrient_graph[last]) {
         cudaGraph_t g;
