@@ -34,6 +34,17 @@ struct DevStatus {
     int info;         /* index of the offending cell / box */
 };
 
+/* What the host reads each step, in one piece: the error word, the division
+ * loop's counts, and MoveCell/GrowCell's two counters, which its last block
+ * hands over and clears for the next launch. */
+struct DevStep {
+    DevStatus status;
+    int n_done[4];                /* divisions done, cells after them, groups */
+    unsigned long long fcw;       /* F_cw calls */
+    int div_count;                /* cells with Length >= Ldiv */
+    unsigned blocks;              /* blocks that have finished */
+};
+
 /* Parameters the kernels read, copied by value into each launch. */
 /* divisions per step handled by bcg_divide, and the footprint-overlap
  * pairs its planner records before falling back to one sequential group */

@@ -61,17 +61,20 @@ int ctx_check_status(bcg_ctx* c)
         cudaStreamSynchronize(c->stream);
         return rc;
     }
-    cudaError_t e = cudaStreamSynchronize(c->stream);
+    cudaError_t e = cudaMemcpyAsync(&c->step_host->status, c->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) { g_last_cuda = e; return BCG_E_CUDA; }
-    DevStatus st;
-    e = cudaMemcpy(&st, c->status, sizeof(st), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) { g_last_cuda = e; return BCG_E_CUDA; }
-    if (st.code) {
+    return ctx_take_status(c);
+}
+/* the status word a synchronised copy left in step_host; an error is cleared */
+int ctx_take_status(bcg_ctx* c)
+{
+    const int code = c->step_host->status.code;
+    if (code) {
         DevStatus z = {0, 0};
         cudaMemcpy(c->status, &z, sizeof(z), cudaMemcpyHostToDevice);
-        return st.code;
     }
-    return BCG_OK;
+    return code;
 }
 
 int ctx_check_status_bbox(bcg_ctx* c)
@@ -255,13 +258,11 @@ extern "C" int bcg_create(const bcg_params* p, bcg_ctx** out)
     DALLOC(c->cell_box, cap * 4);
     DALLOC(c->scan_tmp, 4096 * 4 + 64);
     DALLOC(c->div_list, cap * 4);
-    DALLOC(c->div_count, 64);
     DALLOC(c->fcw_count, 64);
     DALLOC(c->moved, cap * 4);
     DALLOC(c->delta_ids, 2 * cap * 4);
     DALLOC(c->delta_box, 2 * cap * 4);
     DALLOC(c->lineage, 2 * cap * 4);
-    DALLOC(c->n_done_dev, 64);
     DALLOC(c->draws_dev, 9 * cap * 4);
     DALLOC(c->div_rec, 2 * (size_t)DIV_SORT_MAX * sizeof(CellRec));
     DALLOC(c->div_box, 2 * (size_t)DIV_SORT_MAX * 4);
@@ -270,8 +271,12 @@ extern "C" int bcg_create(const bcg_params* p, bcg_ctx** out)
     DALLOC(c->div_par, (size_t)DIV_SORT_MAX * 4);
     DALLOC(c->div_order, (size_t)DIV_SORT_MAX * 4);
     DALLOC(c->div_grp, 2 * (size_t)DIV_SORT_MAX * 4);
-    DALLOC(c->status, sizeof(DevStatus));
-    BCG_CUDA_TRY(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
+    DALLOC(c->step, sizeof(DevStep));
+    c->status = &c->step->status;
+    if (cudaMallocHost((void**)&c->step_host, sizeof(DevStep)) != cudaSuccess ||
+        cudaMallocHost((void**)&c->lineage_host, 2 * DIV_SORT_MAX * sizeof(int)) != cudaSuccess) { bcg_destroy(c); return BCG_E_CUDA; }
+    BCG_CUDA_TRY(cudaMemsetAsync(c->step, 0, sizeof(DevStep), c->stream));
+    BCG_CUDA_TRY(cudaMemsetAsync(c->box_cnt, 0, (size_t)c->nbox * 4, c->stream));
     BCG_CUDA_TRY(cudaMemsetAsync(c->moved, 0, cap * 4, c->stream));
     BCG_CUDA_TRY(cudaMemsetAsync(c->ncount, 0, cap * 4, c->stream));
     BCG_CUDA_TRY(cudaMemsetAsync(c->box_start, 0, ((size_t)c->nbox + 1) * 4, c->stream));
@@ -354,9 +359,9 @@ extern "C" int bcg_destroy(bcg_ctx* c)
     void* ptrs[] = {c->rec[0], c->rec[1], c->stage, c->soa.ldiv, c->soa.gr, c->soa.tp, c->soa.tq, c->soa.ap, c->soa.aq,
                     c->soa.dfx, c->soa.dfy, c->soa.dfz, c->soa.sfx, c->soa.sfy, c->soa.sfz, c->soa.type, c->soa.anc,
                     c->nbr, c->ncount, c->box_cnt, c->box_start, c->box_ids, c->cell_box, c->scan_tmp,
-                    c->div_list, c->div_count, c->fcw_count, c->moved, c->delta_ids, c->delta_box, c->lineage,
-                    c->n_done_dev, c->draws_dev, c->div_rec, c->div_box, c->div_rect, c->div_pairs, c->div_par,
-                    c->div_order, c->div_grp, c->status, c->height, c->rough_height, c->nrm_x, c->nrm_y, c->nrm_z,
+                    c->div_list, c->step, c->fcw_count, c->moved, c->delta_ids, c->delta_box, c->lineage,
+                    c->draws_dev, c->div_rec, c->div_box, c->div_rect, c->div_pairs, c->div_par,
+                    c->div_order, c->div_grp, c->height, c->rough_height, c->nrm_x, c->nrm_y, c->nrm_z,
                     c->wall, c->rd, c->inside, c->rds, c->ds, c->dens, c->rws, c->wds, c->rw, c->wd, c->bbox, c->mg_scratch, c->sweep_type};
     for (void* q : ptrs) if (q) cudaFree(q);
     for (int b = 0; b < 2; b++) {
@@ -385,6 +390,8 @@ extern "C" int bcg_destroy(bcg_ctx* c)
     for (int g = 0; g < 2; g++) if (c->nutrient_graph[g]) cudaGraphExecDestroy(c->nutrient_graph[g]);
     if (c->solve_graph) cudaGraphExecDestroy(c->solve_graph);
     if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->step_host) cudaFreeHost(c->step_host);
+    if (c->lineage_host) cudaFreeHost(c->lineage_host);
     timeline_free(c);
     for (int t = 0; t < BCG_T_COUNT; t++) { if (c->ev[t][0]) cudaEventDestroy(c->ev[t][0]); if (c->ev[t][1]) cudaEventDestroy(c->ev[t][1]); }
     if (c->aux_stream) { cudaStreamSynchronize(c->aux_stream); cudaStreamDestroy(c->aux_stream); }

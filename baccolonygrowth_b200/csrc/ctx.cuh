@@ -69,13 +69,14 @@ struct bcg_ctx {
     int* scan_tmp;         /* block sums */
     /* divisions */
     int* div_list;         /* cap */
-    int* div_count;        /* device counter */
-    unsigned long long* fcw_count;
+    unsigned long long* fcw_count;      /* mean_stress's */
+    DevStep* step;         /* device */
+    DevStep* step_host;    /* pinned, written by kernels and copies */
     int* moved;            /* cap, per-step division bookkeeping */
     int* delta_ids;        /* 2*cap */
     int* delta_box;
     int* lineage;          /* 2*cap */
-    int* n_done_dev;
+    int* lineage_host;     /* pinned, 2*DIV_SORT_MAX: the plan kernel writes it too */
     float* draws_dev;      /* 9*cap */
     /* division planning (DIV_SORT_MAX divisions per step at most) */
     CellRec* div_rec;      /* 2 per division: new mother, daughter */
@@ -90,7 +91,7 @@ struct bcg_ctx {
      * moved, grown records (the reference's new_cells) are rec[cur ^ 1] */
     int move_pending;
     /* status */
-    DevStatus* status;     /* device */
+    DevStatus* status;     /* device: step->status */
     /* pinned host staging */
     void* pinned;
     size_t pinned_bytes;
@@ -166,6 +167,7 @@ struct bcg_ctx {
 MechParams mech_params(const bcg_ctx* c);
 FieldPtrs field_ptrs(const bcg_ctx* c);
 int ctx_check_status(bcg_ctx* c);   /* syncs, reads the device status word */
+int ctx_take_status(bcg_ctx* c);    /* the word as the last synchronised read left it */
 void timer_begin(bcg_ctx* c, int t);
 void timer_end(bcg_ctx* c, int t, int launches);
 int ensure_pinned(bcg_ctx* c, size_t bytes);

@@ -8,6 +8,7 @@
 #include "ctx.cuh"
 #include "cellmath.cuh"
 #include "internal.h"
+#include <stddef.h>
 #include <string.h>
 
 /* ======================================================================= */
@@ -80,7 +81,29 @@ __global__ void k_scan_blocks(int nb, int* __restrict__ block_sums)
         pre += v[j];
     }
 }
-__global__ void k_scan_apply(int n, const int* __restrict__ in, const int* __restrict__ block_sums, int* __restrict__ out)
+/* the whole scan in one block, for up to SCAN_SMALL boxes: a thread takes up to
+ * 32 counts side by side, so that one round of loads covers them all (4 us;
+ * the three launches of the general form 10 us and their gaps).  Both forms
+ * leave the counts 0 for the next binning. */
+#define SCAN_SMALL 32768
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_small(int n, int* __restrict__ in, int* __restrict__ out)
+{
+    __shared__ int sh[32];
+    const int per = (n + SCAN_BLOCK - 1) / SCAN_BLOCK, base = threadIdx.x * per;
+    int v[SCAN_SMALL / SCAN_BLOCK], s = 0;
+#pragma unroll
+    for (int j = 0; j < SCAN_SMALL / SCAN_BLOCK; j++) {
+        v[j] = j < per && base + j < n ? in[base + j] : 0;
+        s += v[j];
+    }
+    int total;
+    int pre = block_excl_scan(s, sh, total);
+#pragma unroll
+    for (int j = 0; j < SCAN_SMALL / SCAN_BLOCK; j++)
+        if (j < per && base + j < n) { out[base + j] = pre; in[base + j] = 0; pre += v[j]; }
+    if (threadIdx.x == 0) out[n] = total;
+}
+__global__ void k_scan_apply(int n, int* __restrict__ in, const int* __restrict__ block_sums, int* __restrict__ out)
 {
     __shared__ int sh[32];
     long base = (long)blockIdx.x * SCAN_BLOCK * SCAN_ITEMS;
@@ -94,7 +117,7 @@ __global__ void k_scan_apply(int n, const int* __restrict__ in, const int* __res
     int pre = block_excl_scan(s, sh, total) + block_sums[blockIdx.x];
     for (int j = 0; j < SCAN_ITEMS; j++) {
         long idx = base + (long)threadIdx.x * SCAN_ITEMS + j;
-        if (idx < n) out[idx] = pre;
+        if (idx < n) { out[idx] = pre; in[idx] = 0; }
         pre += v[j];
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[n] = pre;
@@ -125,8 +148,13 @@ __global__ void k_bin_sort(int nbox, const int* __restrict__ box_start, int* __r
     }
 }
 
-static int scan_exclusive(bcg_ctx* c, const int* in, int* out, int n)
+static int scan_exclusive(bcg_ctx* c, int* in, int* out, int n)
 {
+    if (n <= SCAN_SMALL) {
+        k_scan_small<<<1, SCAN_BLOCK, 0, c->stream>>>(n, in, out);
+        c->launches++;
+        return BCG_OK;
+    }
     int nb = (n + SCAN_BLOCK * SCAN_ITEMS - 1) / (SCAN_BLOCK * SCAN_ITEMS);
     if (nb < 1) nb = 1;
     if (nb > SCAN_BLOCK * SCAN_ITEMS) return BCG_E_ARG;
@@ -142,7 +170,6 @@ int bin_cells(bcg_ctx* c, int buf)
 {
     MechParams mp = mech_params(c);
     int n = c->n;
-    BCG_CUDA_TRY(cudaMemsetAsync(c->box_cnt, 0, sizeof(int) * (size_t)c->nbox, c->stream));
     int* slot = c->delta_ids;   /* scratch: cap ints, unused outside divisions */
     if (n > 0) {
         k_bin_count<<<(n + 255) / 256, 256, 0, c->stream>>>(n, c->rec[buf], mp, c->cell_box, slot, c->box_cnt, c->status);
@@ -333,9 +360,9 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
         const CellRec* __restrict__ old, CellRec* __restrict__ nw,
         const int* __restrict__ nbr, const int* __restrict__ ncount,
         CellSoA soa, FieldPtrs fp, MechParams mp, double dt,
-        int* __restrict__ div_list, int* __restrict__ div_count,
-        unsigned long long* __restrict__ fcw_count, DevStatus* st)
+        int* __restrict__ div_list, DevStep* step, DevStep* host)
 {
+    DevStatus* st = &step->status;
     int t = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const int gl = threadIdx.x & (G - 1);
     /* Lanes past the last cell run the body on cell 0 and write nothing:
@@ -392,7 +419,7 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
             soa.dfx[me] = df.x; soa.dfy[me] = df.y; soa.dfz[me] = df.z;
             soa.sfx[me] = sf.x; soa.sfy[me] = sf.y; soa.sfz[me] = sf.z;
             if (nc.L >= __ldg(&soa.ldiv[me])) {
-                int k = atomicAdd(div_count, 1);
+                int k = atomicAdd(&step->div_count, 1);
                 div_list[k] = me;
             }
             if (!isfinite(nc.p.x) || !isfinite(nc.p.z) || !isfinite(nc.q.x) || !isfinite(nc.q.z))
@@ -408,7 +435,19 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
     if (threadIdx.x == 0) {
         unsigned long long s = 0;
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += wsum[w];
-        if (s) atomicAdd(fcw_count, s);
+        if (s) atomicAdd(&step->fcw, s);
+        /* the last block hands the step's counters and the error word to the
+         * host (pinned memory: no copies) and clears the counters */
+        __threadfence();
+        if (atomicAdd(&step->blocks, 1u) == gridDim.x - 1) {
+            __threadfence();
+            volatile DevStep* d = step;
+            volatile DevStep* h = host;
+            h->status.code = d->status.code; h->status.info = d->status.info;
+            h->div_count = d->div_count; h->fcw = d->fcw;
+            d->div_count = 0; d->fcw = 0; d->blocks = 0;
+            __threadfence_system();
+        }
     }
 }
 
@@ -430,8 +469,6 @@ extern "C" int bcg_set_force_group(bcg_ctx* c, int g)
 int launch_move_grow(bcg_ctx* c, double dt, int group, int occ)
 {
     int n = c->n;
-    BCG_CUDA_TRY(cudaMemsetAsync(c->div_count, 0, sizeof(int), c->stream));
-    BCG_CUDA_TRY(cudaMemsetAsync(c->fcw_count, 0, sizeof(unsigned long long), c->stream));
     if (n > 0) {
         MechParams mp = mech_params(c);
         FieldPtrs fp = field_ptrs(c);
@@ -442,7 +479,7 @@ int launch_move_grow(bcg_ctx* c, double dt, int group, int occ)
         const CellRec* old = c->rec[c->cur];
         CellRec* nw = c->rec[c->cur ^ 1];
 #define MG_ARGS(G, M, B) k_move_grow<G, M, B><<<blocks, threads, 0, c->stream>>>(n, nb, c->box_ids, old, nw, c->nbr, c->ncount, \
-            c->soa, fp, mp, dt, c->div_list, c->div_count, c->fcw_count, c->status)
+            c->soa, fp, mp, dt, c->div_list, c->step, c->step_host)
 #define MG_GROUPS(M, B) switch (group) { \
             case 1: MG_ARGS(1, M, B); break; case 2: MG_ARGS(2, M, B); break; case 4: MG_ARGS(4, M, B); break; \
             case 8: MG_ARGS(8, M, B); break; default: MG_ARGS(16, M, B); break; }
@@ -457,26 +494,27 @@ int launch_move_grow(bcg_ctx* c, double dt, int group, int occ)
 }
 
 /* split halves of bcg_move_grow (used by the ensemble runner to overlap
- * colonies): the launch queues the kernel and the two counter reads, the
- * finish waits for them */
+ * colonies): the launch, and the wait for what its last block hands over */
 int move_grow_launch(bcg_ctx* c, double dt)
 {
-    int rc = launch_move_grow(c, dt, force_group_of(c), force_occ_of(c));
-    if (rc) return rc;
-    int* hp = (int*)c->pinned;
-    BCG_CUDA_TRY(cudaMemcpyAsync(hp, c->div_count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    BCG_CUDA_TRY(cudaMemcpyAsync(hp + 2, c->fcw_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-    return BCG_OK;
+    return launch_move_grow(c, dt, force_group_of(c), force_occ_of(c));
 }
 int move_grow_finish(bcg_ctx* c, int* n_div, int64_t* fcw_calls)
 {
-    int rc = ctx_check_status(c);
+    int rc;
+    if (c->n > 0 && !c->pending_error) {
+        BCG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+        rc = ctx_take_status(c);
+    } else {
+        c->step_host->div_count = 0;
+        c->step_host->fcw = 0;
+        rc = ctx_check_status(c);
+    }
     if (rc) return rc;
     c->move_pending = 1;
-    int* hp = (int*)c->pinned;
-    c->last_ndiv = hp[0];
-    if (n_div) *n_div = hp[0];
-    if (fcw_calls) *fcw_calls = (int64_t)(*(unsigned long long*)(hp + 2));
+    c->last_ndiv = c->step_host->div_count;
+    if (n_div) *n_div = c->last_ndiv;
+    if (fcw_calls) *fcw_calls = (int64_t)c->step_host->fcw;
     return BCG_OK;
 }
 
@@ -487,10 +525,6 @@ extern "C" int bcg_move_grow(bcg_ctx* c, double dt, int* n_div, int64_t* fcw_cal
     int rc = launch_move_grow(c, dt, force_group_of(c), force_occ_of(c));
     if (rc) return rc;
     timer_end(c, BCG_T_MOVE_GROW, c->n > 0 ? 1 : 0);
-    /* the two counters are the only values the host needs this step */
-    int* hp = (int*)c->pinned;
-    BCG_CUDA_TRY(cudaMemcpyAsync(hp, c->div_count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    BCG_CUDA_TRY(cudaMemcpyAsync(hp + 2, c->fcw_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
     return move_grow_finish(c, n_div, fcw_calls);
 }
 
@@ -651,7 +685,7 @@ __global__ void __launch_bounds__(1024) k_div_plan(int n_start, int ndiv, int ca
         const int* __restrict__ nbr, const int* __restrict__ ncount,
         CellRec* __restrict__ new_rec, int* __restrict__ new_box, int4* __restrict__ rect,
         int2* __restrict__ pairs, int* __restrict__ par_out, int* __restrict__ order, int* __restrict__ grp,
-        int* __restrict__ lineage, int* __restrict__ out, DevStatus* st)
+        int* __restrict__ lineage, int* __restrict__ lineage_host, int* __restrict__ out, DevStatus* st)
 {
     /* dynamic shared memory: the sorted parents (later the group of each
      * root), the union-find parents, the groups' fill counters */
@@ -695,6 +729,7 @@ __global__ void __launch_bounds__(1024) k_div_plan(int n_start, int ndiv, int ca
         if (bd < 0) { dev_error(st, BCG_E_OUT_OF_GRID, N); bd = 0; }
         new_box[2 * d] = bm; new_box[2 * d + 1] = bd;
         lineage[2 * d] = m; lineage[2 * d + 1] = N;
+        *reinterpret_cast<int2*>(lineage_host + 2 * d) = make_int2(m, N);
         int b0 = cell_box[m];
         int x0 = b0 / YZ, z0 = b0 % mp.box_z;
         int xlo = x0, xhi = x0, zlo = z0, zhi = z0;
@@ -919,18 +954,24 @@ int divide_launch(bcg_ctx* c, const float* draws, int n_draw_sets, double t)
     rc = ensure_pinned(c, db + 64);
     if (rc) return rc;
     memcpy(c->pinned, draws, db);
-    BCG_CUDA_TRY(cudaMemcpyAsync(c->draws_dev, c->pinned, db, cudaMemcpyHostToDevice, c->stream));
+    /* a few draws are read from the pinned memory as they are; more are worth
+     * the copy, since the kernel's threads would fetch them word by word */
+    const float* src = (const float*)c->pinned;
+    if (ndiv > 64) {
+        BCG_CUDA_TRY(cudaMemcpyAsync(c->draws_dev, c->pinned, db, cudaMemcpyHostToDevice, c->stream));
+        src = c->draws_dev;
+    }
     MechParams mp = mech_params(c);
-    k_div_plan<<<1, 1024, DIV_PLAN_SMEM, c->stream>>>(c->n, ndiv, c->cap, t, c->draws_dev, c->rec[nb], c->soa, mp,
+    k_div_plan<<<1, 1024, DIV_PLAN_SMEM, c->stream>>>(c->n, ndiv, c->cap, t, src, c->rec[nb], c->soa, mp,
         c->div_list, c->cell_box, c->nbr, c->ncount, c->div_rec, c->div_box, c->div_rect, c->div_pairs,
-        c->div_par, c->div_order, c->div_grp, c->lineage, c->n_done_dev, c->status);
-    k_div_groups<<<ndiv, 32 * DIV_GROUP_WARPS, 0, c->stream>>>(c->n, c->n_done_dev, c->div_grp, c->div_order,
+        c->div_par, c->div_order, c->div_grp, c->lineage, c->lineage_host, c->step->n_done, c->status);
+    k_div_groups<<<ndiv, 32 * DIV_GROUP_WARPS, 0, c->stream>>>(c->n, c->step->n_done, c->div_grp, c->div_order,
         c->lineage, c->div_rec, c->div_box, c->rec[nb], mp, c->nbr, c->ncount, c->box_start, c->box_ids,
         c->moved, c->delta_ids, c->delta_box, c->status);
     c->launches += 2;
     BCG_CUDA_TRY(cudaGetLastError());
-    int* hp = (int*)c->pinned;
-    BCG_CUDA_TRY(cudaMemcpyAsync(hp, c->n_done_dev, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    /* the error word and the counts, in one copy */
+    BCG_CUDA_TRY(cudaMemcpyAsync(c->step_host, c->step, offsetof(DevStep, fcw), cudaMemcpyDeviceToHost, c->stream));
     return BCG_OK;
 }
 int divide_finish(bcg_ctx* c, int* n_done, int* lineage)
@@ -938,10 +979,11 @@ int divide_finish(bcg_ctx* c, int* n_done, int* lineage)
     const int ndiv = c->last_ndiv;
     int done = 0, rc = BCG_OK;
     if (ndiv > 0) {
-        rc = ctx_check_status(c);
-        done = ((int*)c->pinned)[0];
-        if (lineage && done > 0)
-            BCG_CUDA_TRY(cudaMemcpy(lineage, c->lineage, sizeof(int) * 2 * (size_t)done, cudaMemcpyDeviceToHost));
+        BCG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+        if (c->pending_error) rc = ctx_check_status(c);
+        else rc = ctx_take_status(c);
+        done = c->step_host->n_done[0];
+        if (lineage && done > 0) memcpy(lineage, c->lineage_host, sizeof(int) * 2 * (size_t)done);
         c->n += done;
     }
     c->cur ^= 1;
