@@ -125,15 +125,13 @@ __device__ __forceinline__ void relax_point(const MgConst& m, const MgLvlT<T>& L
 template <class T>
 __device__ __forceinline__ double relax_eval(const MgConst& m, const MgLvlT<T>& L, const double* __restrict__ R64,
                                              int l, int sp, int i, int k,
-                                             const double* __restrict__ inside0, int& kind, double& cfac)
+                                             const double* __restrict__ inside0, int& kind, const RelaxK<double>& K)
 {
     const int nx = L.nx, nz = L.nz;
-    const RelaxK<double> K = relax_k<double>(m, l, sp);
     const T* E = SP(L.e);
     const double r = AT(R64, L, i, k);
     const bool oxy = (sp == 1);
     const bool top_levels = l >= m.A - 1;
-    cfac = K.cf;
     kind = 2;
     if (k == 0) {
         int d = 1 << l;
@@ -1715,38 +1713,42 @@ extern "C" int bcg_mg_solve(bcg_ctx* c, int vcycles)
  * for E = (R c + N(E)) / (c + 2) points it is R - ((c+2) E - N(E)) / c, for
  * Dirichlet points R - E.  Computed in FP64 from the FP64 right-hand side
  * and the current correction (FP64 or FP32 storage).  Max-norms of the
- * defect and of R go to out[0], out[1] as ordered bit patterns. */
+ * defect and of R go to out[0], out[1] as ordered bit patterns.
+ * The relaxation constants come from the host and a block takes DEFECT_ROWS
+ * rows before it touches the two words: with three divisions a point and
+ * an atomic a warp it took 64 us (FP32) and 73 us (FP64) at 2305 x 513 points. */
+#define DEFECT_ROWS 16
+struct DefectConst { RelaxK<double> k[3]; double scale[3]; int nxp, nzp; };
 template <class T>
-__global__ void k_mg_defect(MgConst m, MgLvlT<T> L, MgLvl L64, int l, const double* __restrict__ inside0,
-                            unsigned long long* out)
+__global__ void __launch_bounds__(256) k_mg_defect(MgConst m, MgLvlT<T> L, MgLvl L64, int l, DefectConst dc,
+                                                   const double* __restrict__ inside0, unsigned long long* out)
 {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    int sp = blockIdx.y;
+    const int i = blockIdx.x * 256 + threadIdx.x, sp = blockIdx.z;
+    const int k0 = blockIdx.y * DEFECT_ROWS, k1 = min(k0 + DEFECT_ROWS, L.nz + 1);
+    const RelaxK<double> K = SP(dc.k);
+    const double scale = SP(dc.scale);
     double dmax = 0.0, rmax = 0.0;
-    if (idx < (L.nx + 1) * (L.nz + 1)) {
-        int i = idx % (L.nx + 1), k = idx / (L.nx + 1);
-        const int X = m.box_x, ZA = m.box_z_agar;
-        int d = 1 << l, d0 = 1 << m.A;
-        int nxp = X * d0 / d < X ? X * d0 / d : X;
-        int nzp = ZA * d0 / d < ZA ? ZA * d0 / d : ZA;
-        int ip = 2 * i - L.nx + nxp / 2, kp = 2 * k;
-        bool uncovered = (l == 0 || ip <= 0 || ip >= nxp || kp >= nzp);
-        if (uncovered) {
-            int kind; double cfac;
-            double v = relax_eval<T>(m, L, SP(L64.r), l, sp, i, k, inside0, kind, cfac);
-            if (kind != 0) {
-                double e = (double)AT(SP(L.e), L, i, k);
-                double def = (kind == 1) ? (v - e) : (v - e) * (cfac + 2) / cfac;
-                dmax = fabs(def);
-                rmax = fabs(AT(SP(L64.r), L64, i, k));
-            }
+    if (i <= L.nx) {
+        const int ip = 2 * i - L.nx + dc.nxp / 2;
+        const bool column = l == 0 || ip <= 0 || ip >= dc.nxp;
+        for (int k = column ? k0 : max(k0, (dc.nzp + 1) / 2); k < k1; k++) {
+            int kind;
+            const double v = relax_eval<T>(m, L, SP(L64.r), l, sp, i, k, inside0, kind, K);
+            if (kind == 0) continue;
+            const double d = v - (double)AT(SP(L.e), L, i, k);
+            dmax = fmax(dmax, fabs(kind == 1 ? d : d * scale));
+            rmax = fmax(rmax, fabs(AT(SP(L64.r), L64, i, k)));
         }
     }
     for (int o = 16; o >= 1; o >>= 1) {
         dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
         rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
     }
-    if ((threadIdx.x & 31) == 0) {
+    __shared__ double sd[8], sr[8];
+    if ((threadIdx.x & 31) == 0) { sd[threadIdx.x >> 5] = dmax; sr[threadIdx.x >> 5] = rmax; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) { dmax = fmax(dmax, sd[w]); rmax = fmax(rmax, sr[w]); }
         /* non-negative doubles order like their bit patterns */
         if (dmax > 0) atomicMax(&out[0], (unsigned long long)__double_as_longlong(dmax));
         if (rmax > 0) atomicMax(&out[1], (unsigned long long)__double_as_longlong(rmax));
@@ -1754,10 +1756,14 @@ __global__ void k_mg_defect(MgConst m, MgLvlT<T> L, MgLvl L64, int l, const doub
 }
 
 template <class A, class B>
-__global__ void k_mg_convert(const A* __restrict__ in, B* __restrict__ out, size_t n)
+__global__ void k_mg_convert(const A* __restrict__ in0, const A* __restrict__ in1, const A* __restrict__ in2,
+                             B* __restrict__ out0, B* __restrict__ out1, B* __restrict__ out2, size_t n)
 {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = (B)in[i];
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (blockIdx.y == 0) out0[i] = (B)in0[i];
+    else if (blockIdx.y == 1) out1[i] = (B)in1[i];
+    else out2[i] = (B)in2[i];
 }
 
 /* relative defect over the composite levels; syncs the stream */
@@ -1768,7 +1774,16 @@ static int mg_rel_defect(bcg_ctx* c, const MgConst& m, double* rel, double* rhs_
     BCG_CUDA_TRY(cudaMemsetAsync(d, 0, 2 * sizeof(unsigned long long), c->stream));
     for (int l = 0; l < m.A; l++) {
         MgLvlT<T> L = lvl<T>(c, l);
-        k_mg_defect<T><<<grid2((L.nx + 1) * (L.nz + 1), 256), 256, 0, c->stream>>>(m, L, mg_lvl(c, l), l, c->inside, d);
+        DefectConst dc;
+        const ResConst rc = res_const(m, l);
+        dc.nxp = rc.nxp; dc.nzp = rc.nzp;
+        for (int sp = 0; sp < 3; sp++) {
+            const double cf = m.bl2 * (double)(1 << (2 * l)) / m.dt / m.D[sp], inv = 1.0 / (cf + 2.0);
+            dc.k[sp].cf = cf; dc.k[sp].inv = inv; dc.k[sp].c = cf * inv; dc.k[sp].w = 0.5 * inv;
+            dc.scale[sp] = (cf + 2.0) / cf;
+        }
+        const dim3 grid((unsigned)((L.nx + 1 + 255) / 256), (unsigned)((L.nz + 1 + DEFECT_ROWS - 1) / DEFECT_ROWS), 3);
+        k_mg_defect<T><<<grid, 256, 0, c->stream>>>(m, L, mg_lvl(c, l), l, dc, c->inside, d);
         c->launches++;
     }
     unsigned long long h[2];
@@ -1787,18 +1802,12 @@ static void mg_convert_levels(bcg_ctx* c, bool to_float, bool res)
     for (int l = 0; l < c->mg_levels; l++) {
         MgLevel& L = c->mg[l];
         size_t n = (size_t)L.pitch * (L.nz + 1);
-        for (int sp = 0; sp < 3; sp++) {
-            if (to_float) {
-                const double* src = res ? L.res[sp] : L.err[sp];
-                float* dst = res ? L.resf[sp] : L.errf[sp];
-                k_mg_convert<double, float><<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(src, dst, n);
-            } else {
-                const float* src = res ? L.resf[sp] : L.errf[sp];
-                double* dst = res ? L.res[sp] : L.err[sp];
-                k_mg_convert<float, double><<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(src, dst, n);
-            }
-            c->launches++;
-        }
+        const dim3 grid((unsigned)((n + 255) / 256), 3);
+        double* const* d = res ? L.res : L.err;
+        float* const* f = res ? L.resf : L.errf;
+        if (to_float) k_mg_convert<double, float><<<grid, 256, 0, c->stream>>>(d[0], d[1], d[2], f[0], f[1], f[2], n);
+        else k_mg_convert<float, double><<<grid, 256, 0, c->stream>>>(f[0], f[1], f[2], d[0], d[1], d[2], n);
+        c->launches++;
     }
 }
 
