@@ -2,8 +2,8 @@
  * fields.cu -- cell-to-grid deposition and the surface fields
  * (AgentBasedModel-BacColonyGrowth/Compute.cpp:120-738).
  *
- * GetDensity / GetHeight walk the bins of the current record buffer (one
- * thread per x column, boxes bottom to top); ShiftDensity, BoxAverage,
+ * GetDensity / GetHeight walk the bins of the current record buffer (a block
+ * or a warp per x column, a thread per box); ShiftDensity, BoxAverage,
  * Height_Average, Smooth and GetSurfaceNormal are stencil kernels bounded by
  * the device-resident bounding box, so the chain runs without host syncs.
  */
@@ -19,21 +19,37 @@ __global__ void k_bbox_reset(int* bbox, int X)
     if (threadIdx.x == 0) { bbox[0] = X; bbox[1] = 0; bbox[2] = 0; }
 }
 
+/* one box's share of the column's heights: the highest top among the cells
+ * over each of the rgh sub-columns.  h starts from the cell radius, so only
+ * positive tops count, and positive doubles order as their bit patterns. */
+__device__ __forceinline__ void raise_height(long long* h, int i_ht, int rgh, double top)
+{
+    if (i_ht < 0) i_ht = 0;
+    if (i_ht > rgh - 1) i_ht = rgh - 1;
+    if (i_ht < 8 && top > __longlong_as_double(h[i_ht])) atomicMax(&h[i_ht], __double_as_longlong(top));
+}
+
 /* GetDensity (Compute.cpp:120-227): per box sum of Length*Radius, the
  * inside flag, and per column the max top of the cells (starting from the
- * cell radius).  One thread per column. */
-__global__ void k_get_density(int X, int Z, int rgh, double box_length, double cell_radius,
+ * cell radius).  One block per column and one thread per box: what bounds it
+ * is the chain of loads start -> id -> record of each box, so a box's cells
+ * are the only ones walked in series (their sum keeps its order).  One thread
+ * per column, over all its boxes, took 95 us at 4096 cells (256 columns), 411
+ * at 262144 (2304) and 772 at 1048576 (4608); this form 10, 16 and 43. */
+#define COLUMN_THREADS 128
+__global__ void __launch_bounds__(COLUMN_THREADS) k_get_density(int X, int Z, int rgh, double box_length, double cell_radius,
                               const CellRec* __restrict__ rec, const int* __restrict__ box_start,
                               const int* __restrict__ box_ids, double* __restrict__ rd,
                               double* __restrict__ inside, double* __restrict__ height, int* bbox)
 {
-    int bx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (bx >= X) return;
-    double h[8];
-    for (int i = 0; i < rgh && i < 8; i++) h[i] = cell_radius;
+    __shared__ long long h[8];
+    __shared__ int top_z;
+    const int bx = blockIdx.x;
+    if (threadIdx.x < 8) h[threadIdx.x] = __double_as_longlong(cell_radius);
+    if (threadIdx.x == 0) top_z = -1;
+    __syncthreads();
     const double Vbox = box_length * box_length;
-    int any = 0, top_z = 0;
-    for (int bz = 0; bz < Z; bz++) {
+    for (int bz = threadIdx.x; bz < Z; bz += COLUMN_THREADS) {
         int b = bx * Z + bz;
         int s = box_start[b], e = box_start[b + 1];
         double den = 0;
@@ -41,19 +57,16 @@ __global__ void k_get_density(int X, int Z, int rgh, double box_length, double c
             const CellRec& r = rec[box_ids[t]];
             double4 pl = r.pL, qr = r.qR;
             double cmx = (pl.x + qr.x) * 0.5;
-            int i_ht = (int)((cmx / box_length - (bx - X / 2)) * rgh);
-            if (i_ht < 0) i_ht = 0;
-            if (i_ht > rgh - 1) i_ht = rgh - 1;
-            double top = pl.z > qr.z ? pl.z : qr.z;
-            if (i_ht < 8) h[i_ht] = h[i_ht] > top ? h[i_ht] : top;
+            raise_height(h, (int)((cmx / box_length - (bx - X / 2)) * rgh), rgh, pl.z > qr.z ? pl.z : qr.z);
             den += pl.w * qr.w;
         }
-        if (e > s) { any = 1; top_z = bz; }
+        if (e > s) atomicMax(&top_z, bz);
         if (den == 0) { rd[IX(bx, bz)] = 0; inside[IX(bx, bz)] = 0; }
         else { rd[IX(bx, bz)] = den / Vbox; inside[IX(bx, bz)] = 1.0; }
     }
-    for (int i = 0; i < rgh && i < 8; i++) height[bx * rgh + i] = h[i];
-    if (any) { atomicMin(&bbox[0], bx); atomicMax(&bbox[1], bx); atomicMax(&bbox[2], top_z); }
+    __syncthreads();
+    if (threadIdx.x < rgh && threadIdx.x < 8) height[bx * rgh + threadIdx.x] = __longlong_as_double(h[threadIdx.x]);
+    if (threadIdx.x == 0 && top_z >= 0) { atomicMin(&bbox[0], bx); atomicMax(&bbox[1], bx); atomicMax(&bbox[2], top_z); }
 }
 
 /* the boundary ring of insideColonyDen, Compute.cpp:228-249 (reads only
@@ -74,34 +87,39 @@ __global__ void k_inside_ring(int X, int Z, double* inside)
     }
 }
 
-/* GetHeight (Compute.cpp:256-340): top four occupied boxes per column */
-__global__ void k_get_height(int X, int Z, int rgh, double box_length, double cell_radius,
+/* GetHeight (Compute.cpp:256-340): top four occupied boxes per column.  One
+ * warp per column looks at 32 boxes at a time from the top; a lane walks its
+ * own box if it is among the first four (8.6 us at 4096 cells; one thread per
+ * column 78). */
+__global__ void __launch_bounds__(COLUMN_THREADS) k_get_height(int X, int Z, int rgh, double box_length, double cell_radius,
                              const CellRec* __restrict__ rec, const int* __restrict__ box_start,
                              const int* __restrict__ box_ids, double* __restrict__ height, int* bbox)
 {
-    int bx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (bx >= X) return;
-    double h[8];
-    for (int i = 0; i < rgh && i < 8; i++) h[i] = cell_radius;
-    int pos_ct = 0, top_z = -1;
-    for (int bz = Z - 1; bz >= 0; bz--) {
-        int b = bx * Z + bz;
-        int s = box_start[b], e = box_start[b + 1];
-        if (e > s) { pos_ct++; if (top_z < 0) top_z = bz; }
-        for (int t = s; t < e; t++) {
-            const CellRec& r = rec[box_ids[t]];
-            double4 pl = r.pL, qr = r.qR;
-            double cmx = (pl.x + qr.x) * 0.5;
-            int i_ht = (int)((cmx - (bx - X / 2) * box_length) / (box_length / rgh));
-            if (i_ht < 0) i_ht = 0;
-            if (i_ht > rgh - 1) i_ht = rgh - 1;
-            double top = pl.z > qr.z ? pl.z : qr.z;
-            if (i_ht < 8) h[i_ht] = h[i_ht] > top ? h[i_ht] : top;
-        }
-        if (pos_ct > 3) break;
+    __shared__ long long hs[COLUMN_THREADS / 32][8];
+    const int lane = threadIdx.x & 31, bx = blockIdx.x * (COLUMN_THREADS / 32) + (threadIdx.x >> 5);
+    if (bx >= X) return;                       /* whole warp */
+    long long* h = hs[threadIdx.x >> 5];
+    if (lane < 8) h[lane] = __double_as_longlong(cell_radius);
+    __syncwarp();
+    int found = 0, top_z = -1;
+    for (int z0 = Z - 1; z0 >= 0 && found < 4; z0 -= 32) {
+        const int bz = z0 - lane;
+        int s = 0, e = 0;
+        if (bz >= 0) { s = box_start[bx * Z + bz]; e = box_start[bx * Z + bz + 1]; }
+        const unsigned occ = __ballot_sync(0xffffffffu, e > s);
+        if (top_z < 0 && occ) top_z = z0 - (__ffs(occ) - 1);
+        if (found + __popc(occ & ((1u << lane) - 1)) < 4)
+            for (int t = s; t < e; t++) {
+                const CellRec& r = rec[box_ids[t]];
+                double4 pl = r.pL, qr = r.qR;
+                double cmx = (pl.x + qr.x) * 0.5;
+                raise_height(h, (int)((cmx - (bx - X / 2) * box_length) / (box_length / rgh)), rgh, pl.z > qr.z ? pl.z : qr.z);
+            }
+        found += __popc(occ);
     }
-    for (int i = 0; i < rgh && i < 8; i++) height[bx * rgh + i] = h[i];
-    if (top_z >= 0) { atomicMin(&bbox[0], bx); atomicMax(&bbox[1], bx); atomicMax(&bbox[2], top_z); }
+    __syncwarp();
+    if (lane < rgh && lane < 8) height[bx * rgh + lane] = __longlong_as_double(h[lane]);
+    if (lane == 0 && top_z >= 0) { atomicMin(&bbox[0], bx); atomicMax(&bbox[1], bx); atomicMax(&bbox[2], top_z); }
 }
 
 /* minx-5, maxx+5, maxz+5 (Compute.cpp:250-252) and the range the stencils
@@ -238,7 +256,7 @@ static int deposit(bcg_ctx* c, bool smooth)
     if (rc) return rc;
     const int X = P.box_x, Z = P.box_z;
     k_bbox_reset<<<1, 32, 0, c->stream>>>(c->bbox, X);
-    k_get_density<<<(X + 127) / 128, 128, 0, c->stream>>>(X, Z, P.refinement_grid_height, P.box_length, P.cell_radius,
+    k_get_density<<<X, COLUMN_THREADS, 0, c->stream>>>(X, Z, P.refinement_grid_height, P.box_length, P.cell_radius,
         c->rec[c->cur], c->box_start, c->box_ids, c->rd, c->inside, c->height, c->bbox);
     k_inside_ring<<<(X * Z + 255) / 256, 256, 0, c->stream>>>(X, Z, c->inside);
     k_bbox_finish<<<1, 32, 0, c->stream>>>(c->bbox, X, Z, P.filter_len / 2, c->status);
@@ -270,7 +288,7 @@ extern "C" int bcg_update_height(bcg_ctx* c)
     if (rc) return rc;
     const int X = P.box_x, Z = P.box_z;
     k_bbox_reset<<<1, 32, 0, c->stream>>>(c->bbox, X);
-    k_get_height<<<(X + 127) / 128, 128, 0, c->stream>>>(X, Z, P.refinement_grid_height, P.box_length, P.cell_radius,
+    k_get_height<<<(X + 3) / 4, COLUMN_THREADS, 0, c->stream>>>(X, Z, P.refinement_grid_height, P.box_length, P.cell_radius,
         c->rec[c->cur], c->box_start, c->box_ids, c->height, c->bbox);
     k_bbox_finish<<<1, 32, 0, c->stream>>>(c->bbox, X, Z, P.filter_len / 2, c->status);
     c->launches += 3;
