@@ -81,27 +81,40 @@ __global__ void k_scan_blocks(int nb, int* __restrict__ block_sums)
         pre += v[j];
     }
 }
-/* the whole scan in one block, for up to SCAN_SMALL boxes: a thread takes up to
- * 32 counts side by side, so that one round of loads covers them all (4 us;
- * the three launches of the general form 10 us and their gaps).  Both forms
- * leave the counts 0 for the next binning. */
+/* the whole scan in one block, for up to SCAN_SMALL boxes (6 us at 12800; the
+ * three launches of the general form 12 and their gaps): tiles of 4 counts a
+ * thread, all loaded before the first is scanned.  Both forms leave the counts 0 for the
+ * next binning. */
 #define SCAN_SMALL 32768
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_small(int n, int* __restrict__ in, int* __restrict__ out)
 {
     __shared__ int sh[32];
-    const int per = (n + SCAN_BLOCK - 1) / SCAN_BLOCK, base = threadIdx.x * per;
-    int v[SCAN_SMALL / SCAN_BLOCK], s = 0;
+    constexpr int TILE = SCAN_BLOCK * SCAN_ITEMS, TILES = SCAN_SMALL / TILE;
+    int4 v[TILES];
+    const int at = threadIdx.x * SCAN_ITEMS;
 #pragma unroll
-    for (int j = 0; j < SCAN_SMALL / SCAN_BLOCK; j++) {
-        v[j] = j < per && base + j < n ? in[base + j] : 0;
-        s += v[j];
+    for (int t = 0; t < TILES; t++) {
+        const int i = t * TILE + at;
+        v[t] = make_int4(0, 0, 0, 0);
+        if (i + 3 < n) v[t] = *reinterpret_cast<const int4*>(in + i);
+        else { if (i < n) v[t].x = in[i]; if (i + 1 < n) v[t].y = in[i + 1]; if (i + 2 < n) v[t].z = in[i + 2]; }
     }
-    int total;
-    int pre = block_excl_scan(s, sh, total);
+    int carry = 0;
 #pragma unroll
-    for (int j = 0; j < SCAN_SMALL / SCAN_BLOCK; j++)
-        if (j < per && base + j < n) { out[base + j] = pre; in[base + j] = 0; pre += v[j]; }
-    if (threadIdx.x == 0) out[n] = total;
+    for (int t = 0; t < TILES; t++) {
+        if (t * TILE >= n) break;
+        int total;
+        const int i = t * TILE + at, a = carry + block_excl_scan(v[t].x + v[t].y + v[t].z + v[t].w, sh, total);
+        const int4 o = make_int4(a, a + v[t].x, a + v[t].x + v[t].y, a + v[t].x + v[t].y + v[t].z);
+        if (i + 3 < n) { *reinterpret_cast<int4*>(out + i) = o; *reinterpret_cast<int4*>(in + i) = make_int4(0, 0, 0, 0); }
+        else {
+            if (i < n) { out[i] = o.x; in[i] = 0; }
+            if (i + 1 < n) { out[i + 1] = o.y; in[i + 1] = 0; }
+            if (i + 2 < n) { out[i + 2] = o.z; in[i + 2] = 0; }
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
 }
 __global__ void k_scan_apply(int n, int* __restrict__ in, const int* __restrict__ block_sums, int* __restrict__ out)
 {
@@ -307,6 +320,58 @@ extern "C" int bcg_rebuild_neighbours(bcg_ctx* c)
 /* ======================================================================= */
 /* MoveCell + GrowCell                                                      */
 /* ======================================================================= */
+/* One lane per cell (G = 1): the neighbours' records pass through shared memory.
+ * A lane that gathers its own neighbour's 128 bytes touches a line of its own
+ * with each of eight loads and waits for them; here the warp fetches its 32
+ * neighbours together, eight lanes a record, asynchronously, the next neighbour
+ * while it works on this one.  A record's 16-byte pieces are rotated by its lane,
+ * so that the lanes' reads of one piece meet no bank twice.  Two slots a warp.
+ * The cells' own records come and go the same way.  What remains is the FP64
+ * chain of a pair's force: a scheduler issues an instruction every 2 cycles
+ * (before, every 5), its FP64 pipe is 40% busy.  262144 cells with 6 neighbours:
+ * 145 us, gathered 167. */
+#define STAGE_BYTES (32 * 128)
+__device__ __forceinline__ void stage_fetch(unsigned char* slot, const CellRec* __restrict__ rec, int id)
+{
+    const int lane = threadIdx.x & 31, piece = lane & 7;
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        const int who = (lane >> 3) + 4 * r, nid = __shfl_sync(0xffffffffu, id, who);
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(slot + who * 128 + ((piece ^ (who & 7)) << 4));
+        if (nid >= 0)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(reinterpret_cast<const unsigned char*>(rec + nid) + piece * 16));
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+/* one lane's record as eight pieces, and the warp's store of its 32 records */
+__device__ __forceinline__ void stage_store(unsigned char* slot, CellRec* __restrict__ rec, int id, const CellRec& r)
+{
+    const int lane = threadIdx.x & 31, piece = lane & 7;
+    const double2 p[8] = {make_double2(r.pL.x, r.pL.y), make_double2(r.pL.z, r.pL.w), make_double2(r.qR.x, r.qR.y), make_double2(r.qR.z, r.qR.w),
+                          make_double2(r.v.x, r.v.y), make_double2(r.v.z, r.v.w), make_double2(r.w.x, r.w.y), make_double2(r.w.z, r.w.w)};
+#pragma unroll
+    for (int i = 0; i < 8; i++) *reinterpret_cast<double2*>(slot + lane * 128 + ((i ^ piece) << 4)) = p[i];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int who = (lane >> 3) + 4 * i, nid = __shfl_sync(0xffffffffu, id, who);
+        if (nid >= 0)
+            reinterpret_cast<double2*>(rec + nid)[piece] = *reinterpret_cast<const double2*>(slot + who * 128 + ((piece ^ (who & 7)) << 4));
+    }
+}
+__device__ __forceinline__ Cst stage_read(const unsigned char* slot)
+{
+    const int lane = threadIdx.x & 31, x = lane & 7;
+    const unsigned char* r = slot + lane * 128;
+    auto at = [&](int piece) { return *reinterpret_cast<const double2*>(r + ((piece ^ x) << 4)); };
+    const double2 a0 = at(0), a1 = at(1), b0 = at(2), b1 = at(3), c0 = at(4), c1 = at(5), d0 = at(6), d1 = at(7);
+    Cst s;
+    s.p = mk(a0.x, a0.y, a1.x); s.L = a1.y;
+    s.q = mk(b0.x, b0.y, b1.x); s.R = b1.y;
+    s.v = mk(c0.x, c0.y, c1.x); s.w = mk(d0.x, d0.y, d1.x);
+    return s;
+}
+
 /* Forces on `a` from its neighbour list (lanes of a G-wide group split the
  * list; the group reduces with a fixed butterfly), plus the wall, drag and
  * surface-tension terms (sum_forces, Forces.cpp:332-381). */
@@ -314,12 +379,35 @@ template <int G, bool GEOM32>
 __device__ __forceinline__ void sum_forces_group(const Cst& a, int me, const CellRec* __restrict__ old,
                                                  const int* __restrict__ list, int cnt, double wall_z,
                                                  const FieldPtrs& fp, const MechParams& mp,
-                                                 V3& Fnet, V3& Tnet, V3& sf, V3& df, int& near_wall)
+                                                 V3& Fnet, V3& Tnet, V3& sf, V3& df, int& near_wall, unsigned char* stage, bool again)
 {
     const int gl = threadIdx.x & (G - 1);
     V3 cm = avg_pq(a.p, a.q);
     V3 F = mk(0, 0, 0), T = mk(0, 0, 0);
-    for (int j = gl; j < cnt; j += G) {
+    if (G == 1) {
+        /* the caller has fetched the first neighbours into slot 0 */
+        const int most = __reduce_max_sync(0xffffffffu, cnt);
+        int next = 1 < cnt ? __ldg(&list[1]) : -1;
+        for (int j = 0; j < most; j++) {
+            stage_fetch(stage + ((j + 1) & 1) * STAGE_BYTES, old, next);
+            next = j + 2 < cnt ? __ldg(&list[j + 2]) : -1;
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            if (j < cnt) {
+                const Cst b = stage_read(stage + (j & 1) * STAGE_BYTES);
+                V3 f, r;
+                if (GEOM32 ? pair_force_f32geom(a, cm, b, mp, f, r) : pair_force(a, cm, b, mp, f, r)) {
+                    F = add3(F, f);
+                    T = add3(T, cross3(sub3(r, cm), f));
+                }
+            }
+            __syncwarp();
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        /* the next pass begins with the same neighbours */
+        if (again) stage_fetch(stage, old, 0 < cnt ? __ldg(&list[0]) : -1);
+    } else for (int j = gl; j < cnt; j += G) {
         int id = __ldg(&list[j]);
         Cst b = load_cst(&old[id]);
         V3 f, r;
@@ -371,18 +459,31 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
     const bool active = t < n;
     int me = active ? (t < nbinned ? __ldg(&order[t]) : t) : 0;
     int near1 = 0, near2 = 0;
+    bool told = false;             /* this lane left something for the last block to read */
+    constexpr int SLOTS = G == 1 ? 4 * 2 : 0;        /* two a warp of 128 threads */
+    __shared__ __align__(128) unsigned char stages[SLOTS ? SLOTS * STAGE_BYTES : 16];
+    unsigned char* stage = stages + (G == 1 ? (threadIdx.x >> 5) * 2 * STAGE_BYTES : 0);
     {
-        Cst o = load_cst(&old[me]);
+        const int* list = nbr + (size_t)me * mp.kmax;
+        const int cnt = active || G > 1 ? __ldg(&ncount[me]) : 0;
+        Cst o;
+        if (G == 1) {
+            /* the cells' own records by the same way, then the first neighbours */
+            stage_fetch(stage + STAGE_BYTES, old, me);
+            stage_fetch(stage, old, cnt > 0 ? __ldg(&list[0]) : -1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            o = stage_read(stage + STAGE_BYTES);
+            __syncwarp();
+        } else o = load_cst(&old[me]);
         V3 ocm = avg_pq(o.p, o.q);
         int xi, yi, zi;
         int obox = box_address(ocm, mp, xi, yi, zi);
-        if (obox < 0) { if (gl == 0 && active) dev_error(st, BCG_E_OUT_OF_GRID, me); xi = 0; yi = 0; }
+        if (obox < 0) { if (gl == 0 && active) { dev_error(st, BCG_E_OUT_OF_GRID, me); told = true; } xi = 0; yi = 0; }
         double wall_z = __ldg(&fp.wall[xi * mp.box_y + yi]);
-        const int* list = nbr + (size_t)me * mp.kmax;
-        int cnt = __ldg(&ncount[me]);
         V3 F, T, sf, df;
         /* integrate, Integrate.cpp:11-32 */
-        sum_forces_group<G, GEOM32>(o, me, old, list, cnt, wall_z, fp, mp, F, T, sf, df, near1);
+        sum_forces_group<G, GEOM32>(o, me, old, list, cnt, wall_z, fp, mp, F, T, sf, df, near1, stage, true);
         Cst tmp = o;
         half_kick(dt, F, T, o, tmp.v, tmp.w);
         V3 rcmp = sub3(o.p, ocm), rcmq = sub3(o.q, ocm);
@@ -390,14 +491,14 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
         tmp.p = add3(o.p, scl3(vp, dt));
         tmp.q = add3(o.q, scl3(vq, dt));
         tmp.p.y = 0; tmp.q.y = 0;
-        sum_forces_group<G, GEOM32>(tmp, me, old, list, cnt, wall_z, fp, mp, F, T, sf, df, near2);
+        sum_forces_group<G, GEOM32>(tmp, me, old, list, cnt, wall_z, fp, mp, F, T, sf, df, near2, stage, false);
         Cst nc = tmp;
         half_kick(dt, F, T, tmp, nc.v, nc.w);
         nc.v.y = 0;
         /* grow, grow.cpp:17-102 */
         V3 ncm = avg_pq(nc.p, nc.q);
         int nbox = box_address(ncm, mp, xi, yi, zi);
-        if (nbox < 0) { if (gl == 0 && active) dev_error(st, BCG_E_OUT_OF_GRID, me); nbox = 0; }
+        if (nbox < 0) { if (gl == 0 && active) { dev_error(st, BCG_E_OUT_OF_GRID, me); told = true; } nbox = 0; }
         double g;
         if (mp.cross_feeding && __ldg(&soa.type[me]) != 1) g = __ldg(&fp.gr2[nbox]);
         else g = __ldg(&fp.gr1[nbox]);
@@ -408,22 +509,26 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
         nc.L += dL;
         nc.p = sub3(nc.p, dv);
         nc.q = add3(nc.q, dv);
+        CellRec r;
+        r.pL = make_double4(nc.p.x, nc.p.y, nc.p.z, nc.L);
+        r.qR = make_double4(nc.q.x, nc.q.y, nc.q.z, nc.R);
+        r.v = make_double4(nc.v.x, nc.v.y, nc.v.z, 0.0);
+        r.w = make_double4(nc.w.x, nc.w.y, nc.w.z, 0.0);
+        if (G == 1) stage_store(stage, nw, active ? me : -1, r);
         if (gl == 0 && active) {
-            CellRec r;
-            r.pL = make_double4(nc.p.x, nc.p.y, nc.p.z, nc.L);
-            r.qR = make_double4(nc.q.x, nc.q.y, nc.q.z, nc.R);
-            r.v = make_double4(nc.v.x, nc.v.y, nc.v.z, 0.0);
-            r.w = make_double4(nc.w.x, nc.w.y, nc.w.z, 0.0);
-            nw[me] = r;
+            if (G > 1) nw[me] = r;
             soa.gr[me] = g;
             soa.dfx[me] = df.x; soa.dfy[me] = df.y; soa.dfz[me] = df.z;
             soa.sfx[me] = sf.x; soa.sfy[me] = sf.y; soa.sfz[me] = sf.z;
             if (nc.L >= __ldg(&soa.ldiv[me])) {
                 int k = atomicAdd(&step->div_count, 1);
                 div_list[k] = me;
+                told = true;
             }
-            if (!isfinite(nc.p.x) || !isfinite(nc.p.z) || !isfinite(nc.q.x) || !isfinite(nc.q.z))
+            if (!isfinite(nc.p.x) || !isfinite(nc.p.z) || !isfinite(nc.q.x) || !isfinite(nc.q.z)) {
                 dev_error(st, BCG_E_NAN, me);
+                told = true;
+            }
         }
     }
     /* F_cw calls (one rand() each, Forces.cpp:102): block-reduce then one atomic */
@@ -431,14 +536,17 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
     for (int o = 16; o >= 1; o >>= 1) calls += __shfl_xor_sync(0xffffffffu, calls, o);
     __shared__ unsigned long long wsum[8];
     if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = calls;
-    __syncthreads();
+    told = __syncthreads_or(told);
     if (threadIdx.x == 0) {
         unsigned long long s = 0;
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += wsum[w];
         if (s) atomicAdd(&step->fcw, s);
         /* the last block hands the step's counters and the error word to the
-         * host (pinned memory: no copies) and clears the counters */
-        __threadfence();
+         * host (pinned memory: no copies) and clears the counters.  A block
+         * that changed none of them has nothing to publish: its fence would
+         * wait for its records' stores and hold its place on the SM (at
+         * 262144 cells, 16 lanes each, 24 us of 562). */
+        if (told || s) __threadfence();
         if (atomicAdd(&step->blocks, 1u) == gridDim.x - 1) {
             __threadfence();
             volatile DevStep* d = step;

@@ -53,6 +53,45 @@ def step_both(p, orc, col, rng):
     return len(lin)
 
 
+@pytest.mark.parametrize("group", [1, 16])
+@pytest.mark.parametrize("n", [31, 129, 4097])
+def test_lanes_on_partial_warps(gpu, n, group):
+    p, orc, col, rng = make(n)
+    assert _abi.load().bcg_set_force_group(col.h, group) == 0
+    step_both(p, orc, col, rng)
+
+
+def test_one_cell(gpu):
+    """A lone cell's wall torques cancel, so its angular velocity is rounding
+    (nothing to compare with the oracle's): all lane counts do the same
+    arithmetic on it and agree in every bit."""
+    out = []
+    for group in (1, 2, 16):
+        p, _, col, rng = make(1)
+        assert _abi.load().bcg_set_force_group(col.h, group) == 0
+        col.step(p.dt, 0.0, rng)
+        out.append(col.cells())
+    assert out[0].tobytes() == out[1].tobytes() == out[2].tobytes()
+
+
+# 256 x 128 boxes are the last that one block scans
+@pytest.mark.parametrize("box_z", [16, 127, 128, 129])
+def test_scan_sizes(gpu, box_z):
+    p, orc, col, rng = make(1025, box_x=256, box_z=box_z)
+    assert nbr_sets(orc.neighbours()) == nbr_sets(col.neighbours())
+    step_both(p, orc, col, rng)
+
+
+# up to 64 divisions read their draws where the host wrote them
+@pytest.mark.parametrize("count", [1, 63, 64, 65])
+def test_division_counts(gpu, count):
+    def mutate(cells):
+        cells["ldiv"] = 10.0
+        pick = np.random.default_rng(3).permutation(len(cells))[:count]
+        cells["ldiv"][pick] = cells["length"][pick]
+    assert step_both(*make(3000, mutate=mutate)) == count
+
+
 @pytest.mark.parametrize("n,box_z", [(1, None), (700, 33), (20000, None), (60000, 131)])
 def test_deposition_sizes(gpu, n, box_z):
     p, orc, col, _ = make(n, box_z=box_z, phi=0.45)
