@@ -50,35 +50,49 @@ __device__ __forceinline__ Cst load_cst_coh(const CellRec* r)
 __device__ __forceinline__ V3 avg_pq(V3 p, V3 q) { return scl3(add3(p, q), 0.5); }
 
 /* min_distance, Neighbours.cpp:107-160 */
-__device__ __forceinline__ double seg_distance(V3 p1, V3 q1, V3 p2, V3 q2, V3& c1, V3& c2)
+/* its square */
+__device__ __forceinline__ double seg_distance2(V3 p1, V3 q1, V3 p2, V3 q2, V3& c1, V3& c2)
 {
     V3 v1 = sub3(q1, p1), v2 = sub3(q2, p2), r = sub3(p1, p2);
     double l1 = dot3(v1, v1), l2 = dot3(v2, v2), f = dot3(v2, r), c = dot3(v1, r), b = dot3(v1, v2);
     double denom = l1 * l2 - b * b, s, t;
     if (denom != 0) s = clamp01((b * f - c * l2) / denom);
     else s = 0;
-    double tnom = b * s + f;
-    if (tnom < 0) { t = 0; s = clamp01(-c / l1); }
-    else if (tnom > l2) { t = 1; s = clamp01((b - c) / l1); }
-    else t = tnom / l2;
+    /* the three cases share one division, whose operands each lane selects: a
+     * warp meets all three, and took as many divisions */
+    const double tnom = b * s + f;
+    const bool low = tnom < 0, high = tnom > l2;
+    const double quo = (low ? -c : high ? b - c : tnom) / (low || high ? l1 : l2);
+    t = low ? 0 : high ? 1 : quo;
+    if (low || high) s = clamp01(quo);
     c1 = add3(p1, scl3(v1, s));
     c2 = add3(p2, scl3(v2, t));
     V3 cv = sub3(c1, c2);
-    return sqrt(dot3(cv, cv));
+    return dot3(cv, cv);
+}
+__device__ __forceinline__ double seg_distance(V3 p1, V3 q1, V3 p2, V3 q2, V3& c1, V3& c2) { return sqrt(seg_distance2(p1, q1, p2, q2, c1, c2)); }
+
+/* sqrt(sq) < lim, with the root only where rounding could decide: outside a
+ * band of 2^-49 around lim^2 (the square's and the root's roundings together
+ * are below 2^-51) the squares tell */
+__device__ __forceinline__ bool root_below(double sq, double lim)
+{
+    const double l2 = lim * lim;
+    if (lim > 1e-100) {
+        if (sq < l2 * (1 - 0x1p-49)) return true;
+        if (sq > l2 * (1 + 0x1p-49)) return false;
+    }
+    return sqrt(sq) < lim;
 }
 
 /* reduceNeighbours test, Neighbours.cpp:74-88: keep j for cell a */
 __device__ __forceinline__ bool keep_neighbour(V3 ap, V3 aq, double aL, double aR, V3 acm, V3 bp, V3 bq, double rc)
 {
-    V3 v = sub3(bp, acm);
-    double dp = sqrt(dot3(v, v));
-    v = sub3(bq, acm);
-    double dq = sqrt(dot3(v, v));
+    V3 v = sub3(bp, acm), w = sub3(bq, acm);
     double lim = aL / 2.0 + rc * aR;
-    if ((dp < lim) || (dq < lim)) {
+    if (root_below(dot3(v, v), lim) || root_below(dot3(w, w), lim)) {
         V3 c1, c2;
-        double d = seg_distance(ap, aq, bp, bq, c1, c2);
-        return d < rc * aR;
+        return root_below(seg_distance2(ap, aq, bp, bq, c1, c2), rc * aR);
     }
     return false;
 }
@@ -228,10 +242,16 @@ __device__ __forceinline__ double height_interp(const double* __restrict__ h, in
 __device__ __forceinline__ void surface_tension(const Cst& c, V3 cm, const FieldPtrs& fp, const MechParams& mp, V3& F, V3& T)
 {
     const int rgh = mp.rgh;
-    const double hb = mp.box_length / rgh;
+    const double hb = mp.height_step;
     const int half = mp.box_x / 2 * rgh;
-    int xa = (int)((cm.x + mp.box_x / 2 * mp.box_length) / (mp.box_length / rgh));
-    int i_ht = (int)(c.p.x / hb + half);
+    /* inside the colony (most cells of a large one) nothing else is needed */
+    int i_ht = (int)(cm.x / hb + half);
+    double dxc = cm.x / hb - (i_ht - half + 0.5);
+    i_ht = (int)ceil(dxc) + i_ht - 1;
+    double height_cm = height_interp(fp.height, i_ht, dxc, mp.xh);
+    if (height_cm > (cm.z + mp.box_length)) { F = mk(0, 0, 0); T = mk(0, 0, 0); return; }
+    int xa = (int)((cm.x + mp.box_x / 2 * mp.box_length) / hb);
+    i_ht = (int)(c.p.x / hb + half);
     double dxp = c.p.x / hb - (i_ht - half + 0.5);
     i_ht = (int)ceil(dxp) + i_ht - 1;
     double height_p = height_interp(fp.height, i_ht, dxp, mp.xh);
@@ -239,11 +259,6 @@ __device__ __forceinline__ void surface_tension(const Cst& c, V3 cm, const Field
     double dxq = c.q.x / hb - (i_ht - half + 0.5);
     i_ht = (int)ceil(dxq) + i_ht - 1;
     double height_q = height_interp(fp.height, i_ht, dxq, mp.xh);
-    i_ht = (int)(cm.x / hb + half);
-    double dxc = cm.x / hb - (i_ht - half + 0.5);
-    i_ht = (int)ceil(dxc) + i_ht - 1;
-    double height_cm = height_interp(fp.height, i_ht, dxc, mp.xh);
-    if (height_cm > (cm.z + mp.box_length)) { F = mk(0, 0, 0); T = mk(0, 0, 0); return; }
     xa = xa < 0 ? 0 : (xa > mp.xh - 1 ? mp.xh - 1 : xa);
     V3 N = mk(fp.nx[xa], fp.ny[xa], fp.nz[xa]);
     V3 F1 = mk(0, 0, 0), F2 = mk(0, 0, 0);

@@ -56,7 +56,7 @@ struct MechParams {
     int box_x, box_y, box_z, rgh;
     int xh;             /* Height/Normal length, box_x*rgh */
     int kmax, box_cap;
-    double box_length, rc, cell_radius, l_divide;
+    double box_length, height_step, rc, cell_radius, l_divide;   /* height_step = box_length / rgh */
     double k_cc, k_wc, var_l, var_angle, var_pos, viscosity, gamma_t, cell_mu, wall_mu;
     double tension, delta_h;
     int cross_feeding;

@@ -204,99 +204,123 @@ int bin_cells(bcg_ctx* c, int buf)
 /* ======================================================================= */
 /* neighbour lists                                                          */
 /* ======================================================================= */
-/* Rebuild the reduced list of cell `me` with one warp: gather the 3x3x3
- * box stencil (UniformGrid.h:141-170, z outer, y, x inner), apply the
+/* Rebuild the reduced list of cell `me` with L lanes of a warp: gather the
+ * 3x3x3 box stencil (UniformGrid.h:141-170, z outer, y, x inner), apply the
  * reduceNeighbours filter (Neighbours.cpp:57-93).  Candidates come from the
  * bins; when `moved` is given, binned cells flagged as moved are skipped
- * and the (ids, boxes) of the delta list are gathered instead. */
-template <bool COH>
-__device__ void warp_rebuild_one(int me, const CellRec* rec, MechParams mp,
+ * and the (ids, boxes) of the delta list are gathered instead (they follow
+ * the binned cells of their box).
+ *
+ * The warp's groups run the same trips (whole-warp collectives).  Each lane
+ * writes the ids of its boxes to the group's list in shared memory, where the
+ * candidates are then read side by side: to find a candidate's box by shuffles
+ * cost more instructions than the test itself (all lists of 262144 cells: 440 us
+ * with 32 lanes a cell and shuffles, 248 so). */
+#define REBUILD_LIST 64
+template <int L, bool COH>
+__device__ __forceinline__ void rebuild_list(int me, int* __restrict__ cand, const CellRec* rec, const MechParams& mp,
                                  const int* __restrict__ box_start, const int* __restrict__ box_ids,
                                  const int* moved, const int* delta_ids,
                                  const int* delta_box, int ndelta,
                                  int* nbr, int* ncount, DevStatus* st)
 {
-    const int lane = threadIdx.x & 31;
-    Cst a = COH ? load_cst_coh(&rec[me]) : load_cst(&rec[me]);
+    constexpr int PER = (27 + L - 1) / L;
+    const unsigned all = 0xffffffffu, DELTA = 0x80000000u;
+    const int lane = threadIdx.x & 31, gl = lane & (L - 1), g0 = lane & ~(L - 1);
+    const bool valid = me >= 0;
+    Cst a = COH ? load_cst_coh(&rec[valid ? me : 0]) : load_cst(&rec[valid ? me : 0]);
     V3 acm = avg_pq(a.p, a.q);
     int xi, yi, zi;
     int abox = box_address(acm, mp, xi, yi, zi);
-    if (abox < 0) { if (lane == 0) dev_error(st, BCG_E_OUT_OF_GRID, me); return; }
+    const bool here = valid && abox >= 0;
+    if (valid && abox < 0 && gl == 0) dev_error(st, BCG_E_OUT_OF_GRID, me);
     int* out = nbr + (size_t)me * mp.kmax;
     const int YZ = mp.box_y * mp.box_z;
-    /* the stencil's boxes in scan order, one a lane: lane i takes
-     * (dz, dy, dx) = i / 9, i / 3 % 3, i % 3 around the cell's box, boxes
-     * off the grid counting nothing.  Each box contributes its binned cells
-     * (in bin order), then the delta cells listed in it. */
-    int bs = 0, nbin = 0, ndel = 0, b = -1;
-    if (lane < 27) {
-        const int za = zi - 1 + lane / 9, ya = yi - 1 + (lane / 3) % 3, xa = xi - 1 + lane % 3;
-        if (za >= 0 && za < mp.box_z && ya >= 0 && ya < mp.box_y && xa >= 0 && xa < mp.box_x) {
-            b = xa * YZ + ya * mp.box_z + za;
-            bs = box_start[b];
-            int e = box_start[b + 1];
-            if (e - bs > mp.box_cap) e = bs + mp.box_cap;   /* overfull: error already raised by the binning */
-            nbin = e - bs;
-            for (int t = 0; t < ndelta; t++) ndel += (delta_box[t] == b);
-        }
-    }
-    /* exclusive prefix of the boxes' candidate counts */
-    const int tot_i = nbin + ndel;
-    int incl = tot_i;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    const int off = incl - tot_i;
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    int cnt = 0;
-    for (int t0 = 0; t0 < total; t0 += 32) {
-        const int f = t0 + lane;
-        /* the box holding candidate f: the last lane whose offset is <= f */
-        int box = 0;
-        for (int q = 1; q < 27; q++) {
-            const int oq = __shfl_sync(0xffffffffu, off, q), tq = __shfl_sync(0xffffffffu, tot_i, q);
-            if (tq > 0 && oq <= f) box = q;
-        }
-        const int ob = __shfl_sync(0xffffffffu, off, box), nb_ = __shfl_sync(0xffffffffu, nbin, box);
-        const int sb = __shfl_sync(0xffffffffu, bs, box), bb = __shfl_sync(0xffffffffu, b, box);
-        int j = -1;
-        bool from_delta = false;
-        if (f < total) {
-            const int r = f - ob;
-            if (r < nb_) {
-                j = box_ids[sb + r];
-            } else {
-                /* the (r - nb_)-th delta cell listed in this box */
-                int k = r - nb_;
-                for (int t = 0; t < ndelta; t++)
-                    if (delta_box[t] == bb) { if (k == 0) { j = delta_ids[t]; break; } k--; }
-                from_delta = true;
+    /* the stencil's boxes in scan order, `per` a lane side by side; layers of
+     * y off the grid (all but one where the grid has one) are not counted */
+    const int y0 = max(yi - 1, 0), ny = min(yi + 1, mp.box_y - 1) - y0 + 1;
+    const int nb = here ? 9 * ny : 0, per = (nb + L - 1) / L;
+    int box[PER], bs[PER], num[PER], tot_i = 0;
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int q = gl * per + i;
+        box[i] = -1; bs[i] = 0; num[i] = 0;
+        if (i < per && q < nb) {
+            const int za = zi - 1 + q / (3 * ny), ya = y0 + (q / 3) % ny, xa = xi - 1 + q % 3;
+            if (za >= 0 && za < mp.box_z && xa >= 0 && xa < mp.box_x) {
+                const int b = xa * YZ + ya * mp.box_z + za;
+                box[i] = b;
+                bs[i] = box_start[b];
+                num[i] = min(box_start[b + 1] - bs[i], mp.box_cap);   /* overfull: error already raised by the binning */
+                tot_i += num[i];
+                for (int t = 0; t < ndelta; t++) tot_i += (delta_box[t] == b);
             }
         }
-        bool keep = false;
-        if (j >= 0 && j != me && (from_delta || !(moved && moved[j]))) {
-            Cst bj = COH ? load_cst_coh(&rec[j]) : load_cst(&rec[j]);
-            keep = keep_neighbour(a.p, a.q, a.L, a.R, acm, bj.p, bj.q, mp.rc);
-        }
-        unsigned m = __ballot_sync(0xffffffffu, keep);
-        int pos = cnt + __popc(m & ((1u << lane) - 1));
-        if (keep && pos < mp.kmax) out[pos] = j;
-        cnt += __popc(m);
     }
-    if (cnt > mp.kmax) { if (lane == 0) dev_error(st, BCG_E_NEIGH_OVERFLOW, me); cnt = mp.kmax; }
-    if (lane == 0) ncount[me] = cnt;
+    /* exclusive prefix of the lanes' candidate counts */
+    int incl = tot_i;
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) {
+        const int v = __shfl_up_sync(all, incl, o, L);
+        if (gl >= o) incl += v;
+    }
+    const int off = incl - tot_i;
+    const int total = __shfl_sync(all, incl, L - 1, L);
+    const int most = L == 32 ? total : __reduce_max_sync(all, total);
+    int cnt = 0;
+    for (int w0 = 0; w0 < most; w0 += REBUILD_LIST) {
+        int at = off - w0;
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            for (int k = 0; k < num[i]; k++, at++)
+                if (at >= 0 && at < REBUILD_LIST) cand[at] = box_ids[bs[i] + k];
+            if (box[i] >= 0)
+                for (int t = 0; t < ndelta; t++)
+                    if (delta_box[t] == box[i]) {
+                        if (at >= 0 && at < REBUILD_LIST) cand[at] = (int)((unsigned)delta_ids[t] | DELTA);
+                        at++;
+                    }
+        }
+        __syncwarp();
+        const int end = min(most - w0, REBUILD_LIST);
+        for (int t0 = 0; t0 < end; t0 += L) {
+            bool keep = false;
+            int j = -1;
+            if (w0 + t0 + gl < total) {
+                const unsigned e = (unsigned)cand[t0 + gl];
+                j = (int)(e & ~DELTA);
+                if (j != me && ((e & DELTA) || !(moved && moved[j]))) {
+                    Cst bj = COH ? load_cst_coh(&rec[j]) : load_cst(&rec[j]);
+                    keep = keep_neighbour(a.p, a.q, a.L, a.R, acm, bj.p, bj.q, mp.rc);
+                }
+            }
+            const unsigned m = (__ballot_sync(all, keep) >> g0) & (L == 32 ? all : (1u << (L & 31)) - 1);
+            const int pos = cnt + __popc(m & ((1u << gl) - 1));
+            if (keep && pos < mp.kmax) out[pos] = j;
+            cnt += __popc(m);
+        }
+        __syncwarp();
+    }
+    if (here && gl == 0) {
+        if (cnt > mp.kmax) { dev_error(st, BCG_E_NEIGH_OVERFLOW, me); cnt = mp.kmax; }
+        ncount[me] = cnt;
+    }
 }
 
-__global__ void k_rebuild_all(int n, const CellRec* __restrict__ rec, MechParams mp,
+/* Eight lanes a cell: nine boxes (one layer in y) of a few cells each are 30 to
+ * 50 candidates, which leave less of the last trip idle than on 32 lanes, and
+ * four cells share what a warp does once. */
+#define REBUILD_LANES 8
+#define REBUILD_THREADS 128
+__global__ void __launch_bounds__(REBUILD_THREADS) k_rebuild_all(int n, const CellRec* __restrict__ rec, MechParams mp,
                               const int* __restrict__ box_start, const int* __restrict__ box_ids,
                               int* __restrict__ nbr, int* __restrict__ ncount, DevStatus* st)
 {
-    int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (w >= n) return;
-    /* walk the cells in bin order so that consecutive warps share boxes */
-    int me = box_ids[w];
-    warp_rebuild_one<false>(me, rec, mp, box_start, box_ids, nullptr, nullptr, nullptr, 0, nbr, ncount, st);
+    __shared__ int cand[REBUILD_THREADS / REBUILD_LANES][REBUILD_LIST];
+    const int w = (blockIdx.x * REBUILD_THREADS + threadIdx.x) / REBUILD_LANES;
+    /* walk the cells in bin order so that consecutive groups share boxes */
+    rebuild_list<REBUILD_LANES, false>(w < n ? box_ids[w] : -1, cand[threadIdx.x / REBUILD_LANES], rec, mp, box_start, box_ids,
+                                       nullptr, nullptr, nullptr, 0, nbr, ncount, st);
 }
 
 extern "C" int bcg_rebuild_neighbours(bcg_ctx* c)
@@ -306,9 +330,8 @@ extern "C" int bcg_rebuild_neighbours(bcg_ctx* c)
     int rc = bin_cells(c, c->cur);
     if (rc) return rc;
     if (c->n > 0) {
-        int threads = 256;
-        long warps = c->n;
-        k_rebuild_all<<<(unsigned)((warps * 32 + threads - 1) / threads), threads, 0, c->stream>>>(
+        const long lanes = (long)c->n * REBUILD_LANES;
+        k_rebuild_all<<<(unsigned)((lanes + REBUILD_THREADS - 1) / REBUILD_THREADS), REBUILD_THREADS, 0, c->stream>>>(
             c->n, c->rec[c->cur], mech_params(c), c->box_start, c->box_ids, c->nbr, c->ncount, c->status);
         c->launches++;
     }
@@ -560,8 +583,23 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
 }
 
 /* lanes per cell in the force loop: the context's choice (bcg_autotune or
- * bcg_set_force_group), else 4 */
-static int force_group_of(const bcg_ctx* c) { return c->force_group ? c->force_group : 4; }
+ * bcg_set_force_group), else as many (up to 8) as keep the launch in one wave
+ * of 4 blocks of 128 on 148 SMs, and one where a lane a cell fills more than
+ * that.  Below the line more lanes shorten the walk over a cell's neighbours;
+ * above it they only add what each lane does again.  Dense colonies (6
+ * neighbours), us a launch:
+ *   cells      1000  4096  16384  32768  65536  262144
+ *   8 lanes    18.8  21.2   32.5   48.0   77.9   268
+ *   4          21.0  21.4   26.9   40.5   61.1   191
+ *   2          24.9  24.7   28.0   34.2   56.0   160
+ *   1          31.0  32.0   31.9   34.8   42.9   134 */
+static int force_group_of(const bcg_ctx* c)
+{
+    if (c->force_group) return c->force_group;
+    int g = 8;
+    while (g > 1 && (long)c->n * g > 148L * 4 * 128) g >>= 1;
+    return g;
+}
 static int force_occ_of(const bcg_ctx* c) { return c->force_occ ? c->force_occ : 4; }
 extern "C" int bcg_set_force_group(bcg_ctx* c, int g)
 {
@@ -981,7 +1019,7 @@ __global__ void __launch_bounds__(1024) k_div_plan(int n_start, int ndiv, int ca
  * lists one division rebuilds (the mother's, her listed neighbours', the
  * daughter's) each depend only on the records and the boxes, which the
  * rebuilds do not change, so the block's warps share them out. */
-#define DIV_GROUP_WARPS 4
+#define DIV_GROUP_WARPS 8
 __global__ void __launch_bounds__(32 * DIV_GROUP_WARPS) k_div_groups(int n_start, const int* __restrict__ div_out,
         const int* __restrict__ grp, const int* __restrict__ order, const int* __restrict__ lineage,
         const CellRec* __restrict__ new_rec, const int* __restrict__ new_box,
@@ -990,6 +1028,7 @@ __global__ void __launch_bounds__(32 * DIV_GROUP_WARPS) k_div_groups(int n_start
         int* moved, int* delta_ids, int* delta_box, DevStatus* st)
 {
     __shared__ int idl[1 + 1024 + 1];
+    __shared__ int cand[DIV_GROUP_WARPS][REBUILD_LIST];
     const int w = threadIdx.x >> 5;
     const int g = blockIdx.x;
     if (g >= div_out[2]) return;                       /* whole block */
@@ -1015,7 +1054,7 @@ __global__ void __launch_bounds__(32 * DIV_GROUP_WARPS) k_div_groups(int n_start
         /* every thread has read the mother's old list before a warp rewrites it */
         __syncthreads();
         for (int k = w; k < cnt + 2; k += DIV_GROUP_WARPS)
-            warp_rebuild_one<true>(idl[k], rec, mp, box_start, box_ids, moved, dids, dbox, 2 * (j + 1), nbr, ncount, st);
+            rebuild_list<32, true>(idl[k], cand[w], rec, mp, box_start, box_ids, moved, dids, dbox, 2 * (j + 1), nbr, ncount, st);
     }
     __syncthreads();
     for (int j = threadIdx.x; j < gl; j += blockDim.x) moved[lineage[2 * order[gs + j]]] = 0;

@@ -53,6 +53,12 @@ def step_both(p, orc, col, rng):
     return len(lin)
 
 
+# one wave of 75776 lanes holds 8, 4 and 2 lanes for 9472, 18944 and 37888 cells
+@pytest.mark.parametrize("n", [33, 9472, 9473, 18945, 37889])
+def test_default_lanes(gpu, n):
+    step_both(*make(n))
+
+
 @pytest.mark.parametrize("group", [1, 16])
 @pytest.mark.parametrize("n", [31, 129, 4097])
 def test_lanes_on_partial_warps(gpu, n, group):
@@ -80,6 +86,21 @@ def test_scan_sizes(gpu, box_z):
     p, orc, col, rng = make(1025, box_x=256, box_z=box_z)
     assert nbr_sets(orc.neighbours()) == nbr_sets(col.neighbours())
     step_both(p, orc, col, rng)
+
+
+def squeeze(f):
+    def mutate(cells):
+        for q in ("p", "q"):
+            cells[q] *= f      # shorter cells, closer together: more of them in a box
+        cells["length"] *= f
+    return mutate
+
+
+# a lane group's candidate list holds 64: fewer, and several windows of it
+@pytest.mark.parametrize("f", [1.0, 0.7, 0.5])
+def test_candidate_windows(gpu, f):
+    p, orc, col, rng = make(2000, mutate=squeeze(f))
+    assert nbr_sets(orc.neighbours()) == nbr_sets(col.neighbours())
 
 
 # up to 64 divisions read their draws where the host wrote them
