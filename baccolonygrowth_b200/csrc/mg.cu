@@ -21,22 +21,6 @@ namespace cg = cooperative_groups;
 __device__ __forceinline__ double dmaxd(double a, double b) { return a > b ? a : b; }
 __device__ __forceinline__ double dmind(double a, double b) { return a < b ? a : b; }
 
-#define AT(arr, L, i, k) (arr)[(size_t)(k) * (L).pitch + (i)]
-
-/* Read (i, k) with the reference's flat index i*(nz+1)+k: on levels with
- * nz <= 1 the stencils reach k = -1 or k = nz+1, which the reference's
- * Array3D maps onto the neighbouring column; an index past either end of
- * the array (undefined in the reference) reads as 0.  In range it is AT. */
-template <class P, class LV>
-__device__ __forceinline__ P at_ref(const P* a, const LV& L, int i, int k)
-{
-    if (k >= 0 && k <= L.nz) return AT(a, L, i, k);
-    long f = (long)i * (L.nz + 1) + k;
-    long n = (long)(L.nx + 1) * (L.nz + 1);
-    if (f < 0 || f >= n) return P(0);
-    int i2 = (int)(f / (L.nz + 1)), k2 = (int)(f % (L.nz + 1));
-    return AT(a, L, i2, k2);
-}
 
 MgConst mg_const(const bcg_ctx* c, double dt)
 {
@@ -931,13 +915,7 @@ __global__ void k_mg_reset_zero(MgLvlT<T> L, int zero_res)
 }
 
 /* updateSolAgaElementwise, Multigrid.cpp:544-568 */
-/* With `nest` set it also does NestSolAgaElementwise
- * (Multigrid.cpp:724-737) for level l+1 (Ln): a point (i, k) of this level
- * that level l+1 nests, Sol_{l+1}(i', k') = Sol_l(2i' - nx' + nxp'/2, 2k'),
- * writes its updated value there.  That is the value the separate pass
- * would copy: between the two only the boundary rewrite and Res change,
- * and neither touches a nested point. */
-__global__ void k_mg_update_sol(MgConst m, MgLvl L, int l, MgLvl Ln, int nest)
+__global__ void k_mg_update_sol(MgConst m, MgLvl L, int l)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y, sp = blockIdx.z;
     const int nx = L.nx;
@@ -958,15 +936,6 @@ __global__ void k_mg_update_sol(MgConst m, MgLvl L, int l, MgLvl Ln, int nest)
         else a = dmaxd(a, 0.0);
     }
     e = 0;
-    if (nest) {
-        const int nxpn = (X * d0) >> (l + 1) < X ? (X * d0) >> (l + 1) : X;
-        const int nzpn = (ZA * d0) >> (l + 1) < ZA ? (ZA * d0) >> (l + 1) : ZA;
-        const int t = i + Ln.nx - nxpn / 2;
-        if ((k & 1) == 0 && (t & 1) == 0 && i > 0 && i < nxpn && k < nzpn) {
-            const int in = t >> 1, kn = k >> 1;
-            if (in >= 0 && in <= Ln.nx && kn <= Ln.nz) AT(SP(Ln.s), Ln, in, kn) = a;
-        }
-    }
 }
 
 /* per-level constants of the residual pass, worked out on the host with
@@ -1079,58 +1048,119 @@ __global__ void k_mg_update_res(MgConst m, MgLvl L, MgLvl Lp, int l, ResConst rc
     }
 }
 
-/* rewriteSolBdryAga, Multigrid.cpp:469-503 (top row, then the side columns) */
-__global__ void k_mg_rewrite_bdry(MgConst m, MgLvl L, MgLvl Lc, int l)
+/* All levels as one launch sees them (a parameter the kernels index where it
+ * lies); first[l]: level l's first block of FINISH_COLS columns and FINISH_ROWS
+ * rows of a species.  The wall rows that copyFromMG fills, by level and species:
+ * the current buffer's and the other's. */
+#define FINISH_COLS 128
+#define FINISH_ROWS 8
+struct MgAll {
+    int levels, first[BCG_MAX_MG_LEVELS + 1], across[BCG_MAX_MG_LEVELS];
+    MgLvl lv[BCG_MAX_MG_LEVELS];
+    double* wall[BCG_MAX_MG_LEVELS][2][3];
+};
+
+/* reset(), Multigrid.cpp:827-841, in one pass over all levels: updateSolAga
+ * (544-568), NestSolAga (724-737) and resetZero (47-82).  A point that no finer
+ * level covers is updated by its thread, which also writes it where coarser
+ * levels nest it, one after another; the covered points are just those.
+ * (Between the reference's separate passes only the boundary rewrite and Res
+ * change, and neither touches a nested point.)  What bounds the large levels is
+ * their five passes over memory (4609 x 1025 points, three composite levels: 251 us,
+ * 6.8 TB/s; a launch a level 272); on small ones it was the launches
+ * (with the boundary and wall copies eleven of 2 to 4 us at
+ * 257 x 33 points, two composite levels; now two of 6 and 4). */
+__global__ void __launch_bounds__(256) k_mg_finish(const __grid_constant__ MgConst m, const __grid_constant__ MgAll a)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    int sp = blockIdx.y;
-    const int X = m.box_x;
-    int d = 1 << l, d0 = 1 << m.A;
-    const int nx = L.nx, nz = L.nz;
-    int nx2 = X * d0 / d / 4 < X ? X * d0 / d / 4 : X;
+    int l = 0;
+    while ((int)blockIdx.x >= a.first[l + 1]) l++;
+    const MgLvl& L = a.lv[l];
+    const int nx = L.nx, X = m.box_x, ZA = m.box_z_agar, d0 = 1 << m.A;
+    int b = blockIdx.x - a.first[l];
+    const int sp = b % 3;
+    b /= 3;
+    const int k = b / a.across[l] * FINISH_ROWS + (threadIdx.x >> 5);
+    const int i0 = b % a.across[l] * FINISH_COLS + (threadIdx.x & 31);
+    if (k > L.nz) return;
+    double* __restrict__ e = SP(L.e) + (size_t)k * L.pitch;
+    double* __restrict__ r = SP(L.r) + (size_t)k * L.pitch;
+    double* s = SP(L.s) + (size_t)k * L.pitch;
+    /* X d0 / 2^l, as a shift */
+    const int nxp = (X * d0) >> l < X ? (X * d0) >> l : X, nzp = (ZA * d0) >> l < ZA ? (ZA * d0) >> l : ZA;
+    /* the points updated, all loaded before the first store */
+    double sv[FINISH_COLS / 32], ev[FINISH_COLS / 32];
+    bool own[FINISH_COLS / 32];
+#pragma unroll
+    for (int c = 0; c < FINISH_COLS / 32; c++) {
+        const int i = i0 + 32 * c, ip = 2 * i - nx + nxp / 2;
+        own[c] = i <= nx && l < m.A && (l == 0 || ip <= 0 || ip >= nxp || 2 * k >= nzp);
+        if (own[c]) { sv[c] = s[i]; ev[c] = e[i]; }
+    }
+#pragma unroll
+    for (int c = 0; c < FINISH_COLS / 32; c++) {
+        const int i = i0 + 32 * c;
+        if (i > nx) break;
+        if (own[c]) {
+            double v = sv[c] + ev[c];
+            if (sp == 0) v = dmaxd(dmind(v, m.max_carbon), 0.0);
+            else if (sp == 1) v = dmaxd(dmind(v, m.max_o2_agar), 0.0);
+            else v = dmaxd(v, 0.0);
+            s[i] = v;
+            for (int q = l + 1, in = i, kn = k; q < m.A; q++) {
+                const MgLvl& N = a.lv[q];
+                const int nxpn = (X * d0) >> q < X ? (X * d0) >> q : X, nzpn = (ZA * d0) >> q < ZA ? (ZA * d0) >> q : ZA;
+                const int t = in + N.nx - nxpn / 2;
+                if ((kn & 1) || (t & 1) || in <= 0 || in >= nxpn || kn >= nzpn) break;
+                in = t >> 1; kn >>= 1;
+                if (in < 0 || in > N.nx || kn > N.nz) break;
+                AT(SP(N.s), N, in, kn) = v;
+            }
+        }
+        r[i] = 0;
+        e[i] = 0;
+    }
+}
+
+/* rewriteSolBdryAga, Multigrid.cpp:469-503 (top row, then the side columns), of
+ * all levels but the last, and copyFromMG (958-981) of all: the wall rows of both
+ * buffers (the agar field is read straight from the solution rows
+ * 1..BoxZAgar).  A level's boundary takes inner values of the next, which keep
+ * theirs; the one wall value that is rewritten here, column 0's, is worked out
+ * again for the copy. */
+__global__ void k_mg_walls(const __grid_constant__ MgConst m, const __grid_constant__ MgAll a)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, sp = blockIdx.y, l = blockIdx.z;
+    const MgLvl& L = a.lv[l];
+    const int X = m.box_x, nx = L.nx, nz = L.nz, d0 = 1 << m.A;
+    const bool rewritten = l < m.A - 1;
+    const MgLvl& Lc = a.lv[rewritten ? l + 1 : l];
     const double* C = SP(Lc.s);
+    double* s = SP(L.s);
+    const int nx2 = min((X * d0) >> (l + 2), X), col = nx2 / 2 - nx / 4;
+    if (t < X) {
+        const double v = rewritten && t == 0 ? (AT(C, Lc, col, 0) + AT(C, Lc, col, 0)) / 2 : AT(s, L, t, 0);
+        SP(a.wall[l][0])[t] = v;
+        SP(a.wall[l][1])[t] = v;
+    }
+    if (!rewritten) return;
     if (t < nx + 1) {
-        int i = t, k2 = nz / 2;
-        int i2 = nx2 / 2 + i / 2 - nx / 4, i2p1 = nx2 / 2 + (i + 1) / 2 - nx / 4;
-        AT(SP(L.s), L, i, nz) = (AT(C, Lc, i2, k2) + AT(C, Lc, i2p1, k2)) / 2;
+        const int i2 = col + t / 2, i2p1 = col + (t + 1) / 2, k2 = nz / 2;
+        AT(s, L, t, nz) = (AT(C, Lc, i2, k2) + AT(C, Lc, i2p1, k2)) / 2;
     } else if (t < nx + 1 + 2 * nz) {
-        int u = t - (nx + 1);
-        int k = u >> 1, side = u & 1;
-        int i = side ? nx : 0;
-        int i2 = nx2 / 2 + i / 2 - nx / 4;
-        AT(SP(L.s), L, i, k) = (AT(C, Lc, i2, k / 2) + AT(C, Lc, i2, (k + 1) / 2)) / 2;
+        const int u = t - (nx + 1), k = u >> 1, i = u & 1 ? nx : 0, i2 = col + i / 2;
+        AT(s, L, i, k) = (AT(C, Lc, i2, k / 2) + AT(C, Lc, i2, (k + 1) / 2)) / 2;
     }
 }
 
 /* copyToMG, Multigrid.cpp:891-907: wall-under-colony values into level 0,
  * then the periodic copy of column 0 into column BoxX on the last
  * composite level */
-__global__ void k_mg_copy_to(MgConst m, MgLvl L0, const double* __restrict__ wC, const double* __restrict__ wO,
+__global__ void k_mg_copy_to(MgConst m, MgLvl L0, MgLvl La, const double* __restrict__ wC, const double* __restrict__ wO,
                              const double* __restrict__ wA, const double* __restrict__ inside0)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 1 && i <= m.box_x - 1 && inside0[(size_t)i * m.box_z] > 0) {
-        AT(L0.s[0], L0, i, 0) = wC[i];
-        AT(L0.s[1], L0, i, 0) = wO[i];
-        AT(L0.s[2], L0, i, 0) = wA[i];
-    }
-}
-__global__ void k_mg_copy_edge(MgLvl L)
-{
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    int sp = blockIdx.y;
-    if (k > L.nz) return;
-    AT(SP(L.s), L, L.nx, k) = AT(SP(L.s), L, 0, k);
-}
-/* copyFromMG, Multigrid.cpp:958-981: wall rows of both buffers (the agar
- * field is read straight from the solution rows 1..BoxZAgar) */
-__global__ void k_mg_copy_from(MgLvl L, int X, double* cC, double* cO, double* cA, double* pC, double* pO, double* pA)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= X) return;
-    double c = AT(L.s[0], L, i, 0), o = AT(L.s[1], L, i, 0), a = AT(L.s[2], L, i, 0);
-    cC[i] = c; cO[i] = o; cA[i] = a;
-    pC[i] = c; pO[i] = o; pA[i] = a;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, sp = blockIdx.y;
+    if (i >= 1 && i <= m.box_x - 1 && inside0[(size_t)i * m.box_z] > 0) AT(SP(L0.s), L0, i, 0) = pick3(wC, wO, wA, sp)[i];
+    if (i <= La.nz) AT(SP(La.s), La, La.nx, i) = AT(SP(La.s), La, 0, i);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1225,8 +1255,20 @@ static int warm_rows(const MgConst& m, int l)
 #define TILE_POINTS 1800000
 static bool tile_takes(const MgLevel& L) { return (long)(L.nx + 1) * (L.nz + 1) <= TILE_POINTS; }
 
+/* levels whose smoothing adds the prolongation as it reads: those of the tile
+ * form, unless their last odd row lies beside the coarse level's rows (at_ref) or
+ * the column beside the coarse level's last one beyond its pitch */
 template <class T>
-static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps)
+static bool smooth_interpolates(const bcg_ctx* c, const MgConst& m, int l)
+{
+    if (sizeof(T) != 8 || c->relax_mode != 3) return false;
+    const MgLevel &F = c->mg[l], &C = c->mg[l + 1];
+    const int nxp = (m.box_x << m.A) >> (l + 2) < m.box_x ? (m.box_x << m.A) >> (l + 2) : m.box_x;
+    return F.nz + 1 >= 3 && tile_takes(F) && (F.nz + 1) / 2 <= C.nz && nxp / 2 - F.nx / 4 + F.nx / 2 + 1 < C.pitch;
+}
+
+template <class T>
+static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps, bool interpolate = false)
 {
     const int rows = c->mg[l].nz + 1;
     /* levels of 0-1 interior rows read across columns through the flat
@@ -1240,8 +1282,10 @@ static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps)
             const int warm = warm_rows(m, l);
             while (sweeps > 0) {
                 const int S = sweeps >= 3 ? 3 : sweeps;
-                const int rc = mg_smooth_tile(c, m, mg_lvl(c, l), l, S, warm);
+                const MgLvl coarse = mg_lvl(c, interpolate ? l + 1 : l);
+                const int rc = mg_smooth_tile(c, m, mg_lvl(c, l), l, S, warm, interpolate ? &coarse : nullptr);
                 if (rc) { c->pending_error = rc; return; }
+                interpolate = false;
                 swap_err<T>(c, l);
                 sweeps -= S;
             }
@@ -1506,9 +1550,12 @@ void mg_vcycle_t(bcg_ctx* c, const MgConst& m, int mu1, int mu2)
     } else relax_coarsest<T>(c, m, Lv - 1, mu2);
     for (int l = down - 1; l >= 0; l--) {
         MgLvlT<T> Lf = lvl<T>(c, l), Lc = lvl<T>(c, l + 1);
-        k_mg_interp<T><<<grid_rows(Lf.nx / 2 + 1, Lf.nz + 1, 128), 128, 0, c->stream>>>(m, Lf, Lc, l);
-        c->launches++;
-        smooth_level<T>(c, m, l, mu1);
+        const bool interpolates = mu1 > 0 && smooth_interpolates<T>(c, m, l);
+        if (!interpolates) {
+            k_mg_interp<T><<<grid_rows(Lf.nx / 2 + 1, Lf.nz + 1, 128), 128, 0, c->stream>>>(m, Lf, Lc, l);
+            c->launches++;
+        }
+        smooth_level<T>(c, m, l, mu1, interpolates);
     }
 }
 template void mg_vcycle_t<double>(bcg_ctx*, const MgConst&, int, int);
@@ -1516,20 +1563,18 @@ template void mg_vcycle_t<float>(bcg_ctx*, const MgConst&, int, int);
 
 void mg_vcycle(bcg_ctx* c, const MgConst& m, int mu1, int mu2) { mg_vcycle_t<double>(c, m, mu1, mu2); }
 
-static void reset_zero(bcg_ctx* c, int from_level = 0)
+static void reset_zero(bcg_ctx* c)
 {
-    for (int l = from_level; l < c->mg_levels; l++) {
+    for (int l = 0; l < c->mg_levels; l++) {
         MgLvl L = mg_lvl(c, l);
         k_mg_reset_zero<double><<<grid_rows(L.nx + 1, L.nz + 1, 256), 256, 0, c->stream>>>(L, l > 0);
         c->launches++;
     }
 }
-static void update_sol(bcg_ctx* c, const MgConst& m, int l, bool nest = false)
+static void update_sol(bcg_ctx* c, const MgConst& m, int l)
 {
     MgLvl L = mg_lvl(c, l);
-    const bool n = nest && l + 1 < m.A;
-    MgLvl Ln = n ? mg_lvl(c, l + 1) : L;
-    k_mg_update_sol<<<grid_rows(L.nx + 1, L.nz + 1, 256), 256, 0, c->stream>>>(m, L, l, Ln, n ? 1 : 0);
+    k_mg_update_sol<<<grid_rows(L.nx + 1, L.nz + 1, 256), 256, 0, c->stream>>>(m, L, l);
     c->launches++;
 }
 static void update_res(bcg_ctx* c, const MgConst& m, int l, bool setup_clean = false)
@@ -1562,27 +1607,37 @@ void mg_setup(bcg_ctx* c, const MgConst& m)
     for (int l = 0; l <= m.A - 1; l++) update_res(c, m, l);
 }
 
-/* reset(), Multigrid.cpp:827-841 (evalUpdateRes's result is discarded there).
- * updateSolAga and NestSolAga run as one pass per level (update_sol with
- * nest).  Level 0's Res, which reset() recomputes last, is read by nothing
- * before the next setup() recomputes it: it is computed only when a caller
- * reads a multigrid array or changes its inputs (mg_res0_materialise). */
-void mg_reset(bcg_ctx* c, const MgConst& m)
+/* reset(), Multigrid.cpp:827-841 (evalUpdateRes's result is discarded there),
+ * and copyFromMG (958-981) into the wall buffers: two launches over all
+ * levels.  The reference recomputes Res on every composite level in reset(), and
+ * its resetZero clears it again on levels > 0; level 0's is read by nothing before
+ * the next setup() recomputes it: it is computed only when a caller reads a
+ * multigrid array or changes its inputs (mg_res0_materialise). */
+void mg_finish(bcg_ctx* c, const MgConst& m, int cur_wall)
 {
-    for (int l = 0; l <= m.A - 1; l++) update_sol(c, m, l, true);
-    for (int l = 0; l < m.A - 1; l++) {
-        MgLvl L = mg_lvl(c, l), Lc = mg_lvl(c, l + 1);
-        int n = L.nx + 1 + 2 * L.nz;
-        k_mg_rewrite_bdry<<<grid2(n, 256), 256, 0, c->stream>>>(m, L, Lc, l);
-        c->launches++;
+    MgAll a;
+    memset(&a, 0, sizeof(a));
+    a.levels = c->mg_levels;
+    int most = 0;
+    for (int l = 0; l < a.levels; l++) {
+        const MgLvl L = a.lv[l] = mg_lvl(c, l);
+        a.across[l] = L.nx / FINISH_COLS + 1;
+        a.first[l + 1] = a.first[l] + 3 * a.across[l] * (L.nz / FINISH_ROWS + 1);
+        if (l >= m.A) continue;
+        for (int b = 0; b < 2; b++) {
+            const WallBuf& w = c->wal[cur_wall ^ b];
+            a.wall[l][b][0] = w.C[l]; a.wall[l][b][1] = w.O[l]; a.wall[l][b][2] = w.A[l];
+        }
+        const int n = L.nx + 1 + 2 * L.nz;
+        if (n > most) most = n;
     }
-    /* the reference recomputes Res on every composite level here, and the
-     * resetZero below clears it again on levels > 0: only level 0's stays,
-     * computed on demand */
+    if (m.box_x > most) most = m.box_x;
+    k_mg_finish<<<a.first[a.levels], 256, 0, c->stream>>>(m, a);
+    k_mg_walls<<<dim3((unsigned)((most + 255) / 256), 3, (unsigned)m.A), 256, 0, c->stream>>>(m, a);
+    c->launches += 2;
     c->mg_res0_stale = 1;
-    /* updateSolAga already zeroed Err and Res on the composite levels */
-    reset_zero(c, m.A);
     c->mg_clean = 1;
+    c->leg_old_stale = 1;        /* copyFromMG writes FieldAgar and oldFieldAgar alike */
 }
 
 /* level 0's Res as reset() leaves it, before a caller reads or writes a
@@ -1598,22 +1653,10 @@ void mg_copy_to(bcg_ctx* c, const MgConst& m, int wall_buf)
 {
     MgLvl L0 = mg_lvl(c, 0);
     const WallBuf& w = c->wal[wall_buf];
-    k_mg_copy_to<<<(m.box_x + 255) / 256, 256, 0, c->stream>>>(m, L0, w.C[0], w.O[0], w.A[0], c->inside);
     MgLvl La = mg_lvl(c, m.A - 1);
-    k_mg_copy_edge<<<grid2(La.nz + 1, 256), 256, 0, c->stream>>>(La);
-    c->launches += 2;
-}
-
-void mg_copy_from(bcg_ctx* c, const MgConst& m, int cur_wall)
-{
-    c->leg_old_stale = 1;        /* copyFromMG writes FieldAgar and oldFieldAgar alike */
-    for (int l = 0; l < m.A; l++) {
-        MgLvl L = mg_lvl(c, l);
-        const WallBuf& cw = c->wal[cur_wall];
-        const WallBuf& pw = c->wal[cur_wall ^ 1];
-        k_mg_copy_from<<<(m.box_x + 255) / 256, 256, 0, c->stream>>>(L, m.box_x, cw.C[l], cw.O[l], cw.A[l], pw.C[l], pw.O[l], pw.A[l]);
-        c->launches++;
-    }
+    const int n = m.box_x > La.nz + 1 ? m.box_x : La.nz + 1;
+    k_mg_copy_to<<<grid2(n, 256), 256, 0, c->stream>>>(m, L0, La, w.C[0], w.O[0], w.A[0], c->inside);
+    c->launches++;
 }
 
 /* Multigrid::solve (Multigrid.cpp:864-889) with the given V-cycle count;
@@ -1624,8 +1667,7 @@ int mg_solve_impl(bcg_ctx* c, int vcycles, int wall_buf)
     mg_copy_to(c, m, wall_buf);
     mg_setup(c, m);
     for (int v = 0; v < vcycles; v++) mg_vcycle(c, m, c->P.mg_mu1, c->P.mg_mu2);
-    mg_reset(c, m);
-    mg_copy_from(c, m, wall_buf);
+    mg_finish(c, m, wall_buf);
     if (c->pending_error) { const int rc = c->pending_error; c->pending_error = BCG_OK; return rc; }
     return cudaGetLastError() == cudaSuccess ? BCG_OK : BCG_E_CUDA;
 }
@@ -1680,7 +1722,7 @@ static int mg_solve_graphed(bcg_ctx* c, int vcycles, int wall_buf, cudaStream_t 
         }
         c->solve_graph_key = key;
     } else {
-        /* the host state a solve leaves (mg_setup, mg_reset, mg_copy_from) */
+        /* the host state a solve leaves (mg_setup, mg_finish) */
         c->mg_res0_stale = 1;
         c->mg_clean = 1;
         c->leg_old_stale = 1;
@@ -1852,8 +1894,7 @@ extern "C" int bcg_mg_solve_tol(bcg_ctx* c, double rel_tol, int precision, int m
             if ((rc = mg_rel_defect<double>(c, m, &rel, nullptr))) return rc;
         }
     } else rel = 0.0;
-    mg_reset(c, m);
-    mg_copy_from(c, m, 0);
+    mg_finish(c, m, 0);
     BCG_CUDA_TRY(cudaGetLastError());
     timer_end(c, BCG_T_MG_SOLVE, (int)(c->launches - l0));
     if (iters) *iters = it;

@@ -31,9 +31,8 @@ MgLvlF mg_lvl_f(const bcg_ctx* c, int l);
 template <class T> void mg_vcycle_t(bcg_ctx* c, const MgConst& m, int mu1, int mu2);
 void mg_vcycle(bcg_ctx* c, const MgConst& m, int mu1, int mu2);
 void mg_setup(bcg_ctx* c, const MgConst& m);
-void mg_reset(bcg_ctx* c, const MgConst& m);
 void mg_copy_to(bcg_ctx* c, const MgConst& m, int wall_buf);
-void mg_copy_from(bcg_ctx* c, const MgConst& m, int cur_wall);
+void mg_finish(bcg_ctx* c, const MgConst& m, int cur_wall);
 int mg_solve_impl(bcg_ctx* c, int vcycles, int wall_buf);
 /* the TMA-staged fused smoother (mg_smooth.cu): S sweeps of level L from
  * E into E2 with about `target_warps` warps (one row segment of one strip
@@ -48,8 +47,9 @@ int mg_smooth_tma_attributes();
 int mg_smooth_tma_fits(int nx);
 
 /* the register-tiled smoother and the one-launch coarsest levels (mg_tile.cu):
- * S sweeps of level L from E into E2; levels l0 .. of a V-cycle, in place */
-int mg_smooth_tile(bcg_ctx* c, const MgConst& m, const MgLvl& L, int l, int S, int warm);
+ * S sweeps of level L from E (plus the prolongation of `coarse`, if given) into
+ * E2; levels l0 .. of a V-cycle, in place */
+int mg_smooth_tile(bcg_ctx* c, const MgConst& m, const MgLvl& L, int l, int S, int warm, const MgLvl* coarse);
 int mg_tail_level(const bcg_ctx* c, const MgConst& m);
 int mg_tail(bcg_ctx* c, const MgConst& m, const MgLvl* lvls, int l0, int mu1, int mu2);
 int mg_tile_attributes();
@@ -62,6 +62,23 @@ template <class P>
 __device__ __forceinline__ P pick3(const P& a0, const P& a1, const P& a2, int i) { return i == 0 ? a0 : (i == 1 ? a1 : a2); }
 #define SP(arr) pick3((arr)[0], (arr)[1], (arr)[2], sp)
 
+
+#define AT(arr, L, i, k) (arr)[(size_t)(k) * (L).pitch + (i)]
+
+/* Read (i, k) with the reference's flat index i*(nz+1)+k: on levels with
+ * nz <= 1 the stencils reach k = -1 or k = nz+1, which the reference's
+ * Array3D maps onto the neighbouring column; an index past either end of
+ * the array (undefined in the reference) reads as 0.  In range it is AT. */
+template <class P, class LV>
+__device__ __forceinline__ P at_ref(const P* a, const LV& L, int i, int k)
+{
+    if (k >= 0 && k <= L.nz) return AT(a, L, i, k);
+    long f = (long)i * (L.nz + 1) + k;
+    long n = (long)(L.nx + 1) * (L.nz + 1);
+    if (f < 0 || f >= n) return P(0);
+    int i2 = (int)(f / (L.nz + 1)), k2 = (int)(f % (L.nz + 1));
+    return AT(a, L, i2, k2);
+}
 
 /* The relaxation update of relaxationAgarElementwise (Multigrid.cpp:160-249)
  *   E = (R h^2/(dt D) + sum of weighted neighbours) / (h^2/(dt D) + 2)

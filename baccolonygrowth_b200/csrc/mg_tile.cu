@@ -127,10 +127,10 @@ __device__ __forceinline__ void mt_sweeps(double (&Ee)[MT_ROWS], double (&Eo)[MT
 /* One smoothing of a strip: rows k0 .. k0 + MT_ROWS - 1 of columns ce, ce + 1
  * (lane order) read through ld(array, k), S sweeps, and the results left in Ee
  * and Eo.  kw: first row of the segment. */
-template <class SH, class Load>
+template <class SH, class Load, class Add>
 __device__ __forceinline__ void mt_strip(double (&Ee)[MT_ROWS], double (&Eo)[MT_ROWS], const MgConst& m, int l, int sp, int nx, int nz, int ce,
                                          int kw, int slot, int chunks, int S, SH& sh,
-                                         const double* __restrict__ inside0, const Load& ld)
+                                         const double* __restrict__ inside0, const Load& ld, const Add& add)
 {
     const int lane = threadIdx.x & 31, co = ce + 1, k0 = kw + MT_ROWS * slot;
     const RelaxK<double> K = relax_k<double>(m, l, sp);
@@ -147,6 +147,7 @@ __device__ __forceinline__ void mt_strip(double (&Ee)[MT_ROWS], double (&Eo)[MT_
         Ee[j] = Eo[j] = Re[j] = Ro[j] = 0.0;
         if (k0 + j <= nz) ld(k0 + j, Ee[j], Eo[j], &Re[j], &Ro[j]);
     }
+    add(k0, Ee, Eo);
     double ae = 0.0, ao = 0.0;
     if (slot == chunks - 1) {
         if (k0 + MT_ROWS <= nz) ld(k0 + MT_ROWS, ae, ao, (double*)nullptr, (double*)nullptr);
@@ -200,8 +201,12 @@ __device__ __forceinline__ void mt_strip(double (&Ee)[MT_ROWS], double (&Eo)[MT_
  * 1153 x 257 35 -> 12 us, 2305 x 513 57 -> 39 us.  What bounds
  * the small ones is the chain: loads 1.5 us, six half-sweeps of 0.7 us.  The
  * largest repeat 35 of 144 rows and 12 of 64 columns, and a block fills its
- * SM's registers, so loads and sweeps of different blocks do not overlap. */
-__global__ void __launch_bounds__(32 * MT_WARPS, 1) k_mg_tile(MgConst m, MgLvl L, int l, MtPlan plan,
+ * SM's registers, so loads and sweeps of different blocks do not overlap.
+ * INTERP: the values smoothed are E plus the next level's correction
+ * (interpolationAga, Multigrid.cpp:407-467), added as they are read; as a launch
+ * of its own it took 4.5 us on levels of 129 to 513 columns, so 1.5. */
+template <bool INTERP>
+__global__ void __launch_bounds__(32 * MT_WARPS, 1) k_mg_tile(MgConst m, MgLvl L, MgLvl Lc, int l, MtPlan plan,
                                                               const double* __restrict__ inside0)
 {
     __shared__ MtShare<MT_WARPS> sh;
@@ -215,15 +220,62 @@ __global__ void __launch_bounds__(32 * MT_WARPS, 1) k_mg_tile(MgConst m, MgLvl L
     const bool in = ce >= 0 && ce <= nx;
     const double* __restrict__ E = SP(L.e);
     const double* __restrict__ R = SP(L.r);
+    /* X 2^A / 2^l / 4, as a shift; the coarse column of the even column (the one
+     * beside a last even column is not used: it lies in the plane's padding) */
+    const int nxp = min((m.box_x << m.A) >> (l + 2), m.box_x);
+    const double* __restrict__ C = SP(Lc.e) + (nxp / 2 - nx / 4 + (ce >> 1));
     double Ee[MT_ROWS], Eo[MT_ROWS];
     auto ld = [&](int k, double& e, double& o, double* re, double* ro) {
         if (!in) return;
         const size_t at = (size_t)k * L.pitch + ce;
         const double2 v = *reinterpret_cast<const double2*>(E + at);
         e = v.x; o = v.y;
+        if (INTERP && !re) {
+            const double* c = C + (size_t)(k >> 1) * Lc.pitch;
+            const double* d = (k & 1) ? c + Lc.pitch : c;
+            const double c0 = c[0], c1 = c[1], d0 = d[0], d1 = d[1];
+            const double ie = (k & 1) ? 0.5 * (c0 + d0) : c0, io = (k & 1) ? 0.25 * (c0 + d0 + c1 + d1) : 0.5 * (c0 + c1);
+            e += ie;
+            if (ce < nx) o += io;
+        }
         if (re) { const double2 q = *reinterpret_cast<const double2*>(R + at); *re = q.x; *ro = q.y; }
     };
-    mt_strip(Ee, Eo, m, l, sp, nx, nz, ce, kw, threadIdx.y, blockDim.y, S, sh, inside0, ld);
+    /* the prolongation on a thread's 9 rows: one coarse column of the six rows
+     * they lie between (the next column is the next lane's), an odd row taking the
+     * mean of two */
+    auto add = [&](int k0, double (&e)[MT_ROWS], double (&o)[MT_ROWS]) {
+        if (!INTERP) return;
+        constexpr int ROWS = (MT_ROWS + 3) / 2;
+        const int p = k0 & 1;
+        double c[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const int kp = (k0 >> 1) + r;
+            c[r] = in && 2 * kp <= nz + 1 ? C[(size_t)kp * Lc.pitch] : 0.0;
+        }
+        double x[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const int kp = (k0 >> 1) + r;
+            x[r] = __shfl_down_sync(0xffffffffu, c[r], 1);
+            if ((lane == 31 || ce + 2 > nx) && in && 2 * kp <= nz + 1) x[r] = C[(size_t)kp * Lc.pitch + 1];
+        }
+        const bool odd = ce < nx;
+#pragma unroll
+        for (int j = 0; j < MT_ROWS; j++) {
+            const int a = j >> 1, b = (j + 1) >> 1;       /* the row's coarse row for an even k0, for an odd one */
+            const double c0 = p ? c[b] : c[a], c1 = p ? x[b] : x[a];
+            double ie = c0, io = 0.5 * (c0 + c1);
+            if ((p != 0) != (j & 1)) {
+                const double d0 = p ? c[b + 1 < ROWS ? b + 1 : b] : c[a + 1 < ROWS ? a + 1 : a];
+                const double d1 = p ? x[b + 1 < ROWS ? b + 1 : b] : x[a + 1 < ROWS ? a + 1 : a];
+                ie = 0.5 * (c0 + d0);
+                io = 0.25 * (c0 + d0 + c1 + d1);
+            }
+            if (in && k0 + j <= nz) { e[j] += ie; if (odd) o[j] += io; }
+        }
+    };
+    mt_strip(Ee, Eo, m, l, sp, nx, nz, ce, kw, threadIdx.y, blockDim.y, S, sh, inside0, ld, add);
     if (lane < S || lane > 31 - S || !in) return;
     double* __restrict__ EO = SP(L.e2);
 #pragma unroll
@@ -236,7 +288,7 @@ __global__ void __launch_bounds__(32 * MT_WARPS, 1) k_mg_tile(MgConst m, MgLvl L
     }
 }
 
-int mg_smooth_tile(bcg_ctx* c, const MgConst& m, const MgLvl& L, int l, int S, int warm)
+int mg_smooth_tile(bcg_ctx* c, const MgConst& m, const MgLvl& L, int l, int S, int warm, const MgLvl* coarse)
 {
     const int rows = L.nz + 1, cap = MT_ROWS * MT_WARPS - (S - 1);
     MtPlan p;
@@ -250,7 +302,9 @@ int mg_smooth_tile(bcg_ctx* c, const MgConst& m, const MgLvl& L, int l, int S, i
     const int held = nseg == 1 ? rows : p.n0 + S - 1;
     const int outp = 32 - 2 * S;
     const dim3 grid((unsigned)((L.nx + 1 + 2 * outp - 1) / (2 * outp)), (unsigned)nseg, 3);
-    k_mg_tile<<<grid, dim3(32, (unsigned)((held + MT_ROWS - 1) / MT_ROWS)), 0, c->stream>>>(m, L, l, p, c->inside);
+    const dim3 block(32, (unsigned)((held + MT_ROWS - 1) / MT_ROWS));
+    if (coarse) k_mg_tile<true><<<grid, block, 0, c->stream>>>(m, L, *coarse, l, p, c->inside);
+    else k_mg_tile<false><<<grid, block, 0, c->stream>>>(m, L, L, l, p, c->inside);
     c->launches++;
     return BCG_OK;
 }

@@ -1,0 +1,47 @@
+"""The passes that end a solve (update, nesting, boundary rewrite, zeroing, wall
+rows: two launches over all levels) against the C restatement in oracle/, by the
+number of composite levels: one (nothing nests), three and five (a point is
+nested several times).  Bars as test_gpu_fields.py's test_mg_solve."""
+import numpy as np
+import pytest
+
+from baccolonygrowth_b200 import _abi, params
+from baccolonygrowth_b200.colony import Colony, synth_colony
+
+import checkers as ck
+from test_gpu_fields import TOL, close, deplete, wall_mask
+from test_gpu_mg_tile import problem
+
+F = _abi.FIELDS
+SPECIES = ("CARBON", "OXYGEN", "ACETATE")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("box_x,rows,levels", [(256, 16, 1), (224, 36, 3), (992, 40, 5)])
+def test_solve_end_against_oracle(gpu, box_x, rows, levels):
+    p = problem(box_x, rows, levels)
+    w, h = params.dome_size(200, 1.0 / 10.0)
+    cells = synth_colony(200, w, h, seed=5)
+    orc = ck.Oracle(p, seed=12345)
+    orc.load(cells)
+    col = Colony(p, cells)
+    col.set_field("WALL", orc.field(F["WALL"]))
+    orc.update_density()
+    col.update_density()
+    deplete(p, orc, col)
+    for _ in range(2):
+        orc.mg_solve(2, p.mg_dt)
+        col.mg_solve(2)
+    for l in range(p.mg_levels):
+        for sp in SPECIES:
+            for kind in ("SOL", "RES", "ERR"):
+                f = "MG_%s_%s" % (kind, sp)
+                a, b = orc.field(F[f], l), col.field(f, l)
+                if kind == "SOL":
+                    assert close(a, b) <= TOL, (f, l)
+                else:
+                    assert np.abs(a - b).max() <= TOL * max(1.0, np.abs(a).max()), (f, l)
+    for l in range(p.max_levels_mg):
+        for sp in SPECIES:
+            f = "WALLF_" + sp
+            assert close(orc.field(F[f], l), col.field(f, l), mask=wall_mask(p, l)) <= TOL, (f, l)
