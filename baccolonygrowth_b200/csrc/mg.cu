@@ -350,16 +350,17 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_smem(MgConst m, MgLvlT<T> L,
 }
 
 /* Relaxation of point (i, k) of a level held in shared memory (row k at
- * offset k*(nx+1)), in place; the point code of k_mg_coarse_smem. */
+ * offset k*(nx+1)), in place; the point code of k_mg_coarse_smem.  Returns
+ * whether the value changed. */
 template <class T>
-__device__ __forceinline__ void relax_smem(const RelaxK<T>& K, bool oxy, bool top_levels,
+__device__ __forceinline__ bool relax_smem(const RelaxK<T>& K, bool oxy, bool top_levels,
                                            int nx, int nz, int i, int k, T* Es, const T* Rs,
                                            const unsigned char* ins_row0)
 {
     const int W = nx + 1;
     const bool side = (i == 0 || i == nx);
-    const T r = Rs[k * W + i];
-    T out = Es[k * W + i];
+    const T r = Rs[k * W + i], old = Es[k * W + i];
+    T out = old;
     if (k == 0) {
         if (ins_row0[i]) out = r;
         else if (side) {
@@ -379,6 +380,7 @@ __device__ __forceinline__ void relax_smem(const RelaxK<T>& K, bool oxy, bool to
         }
     }
     Es[k * W + i] = out;
+    return out != old;
 }
 
 /* All mu2 relaxations of a level of nz >= 1 held in shared memory, as a
@@ -473,7 +475,14 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_wave(MgConst m, MgLvlT<T> L,
  * block copies its halos from its neighbours' buffers.  Every block runs
  * the same barriers; the last one comes after every read of another
  * block's shared memory, so no block leaves while read.  H <= W / C keeps
- * a halo inside the neighbouring block's columns. */
+ * a halo inside the neighbouring block's columns.
+ *
+ * A sweep that leaves every value as it found it is reproduced by all later
+ * ones.  With its columns a block publishes the last sweep in which one of its
+ * own values changed; once that sweep, over all blocks, lies before one that is
+ * complete, the values are those that all `sweeps` sweeps give, and the cluster
+ * stops.  145 x 33 points, 100 sweeps: 161 us to 80; in
+ * FP32, whose fixed point is nearer, at 73 x 17 points 106 to 19. */
 template <class T>
 __global__ void __launch_bounds__(768) k_mg_coarse_cluster(MgConst m, MgLvlT<T> L, int l, int sweeps, int H,
                                                             const double* __restrict__ inside0)
@@ -492,6 +501,9 @@ __global__ void __launch_bounds__(768) k_mg_coarse_cluster(MgConst m, MgLvlT<T> 
     T* E = SP(L.e);
     const T* R = SP(L.r);
     const int nth = blockDim.x, th = threadIdx.x;
+    __shared__ int changed[2], all_changed;      /* last sweep that changed a value: published (by buffer), of the cluster */
+    if (th < 2) changed[th] = -1;
+    if (th == 2) all_changed = -1;
     for (int q = th; q < np; q += nth) {
         int i = q % W, k = q / W;
         Es[q] = AT(E, L, i, k);
@@ -519,6 +531,7 @@ __global__ void __launch_bounds__(768) k_mg_coarse_cluster(MgConst m, MgLvlT<T> 
     const int ncol = first < e1 ? (e1 - first + 1) / 2 : 0;
     const int a0 = ncol ? tl / ncol : 0x7fffffff, cc0 = ncol ? tl % ncol : 0;
     const int steps = nz + 1 + 2 * (sweeps - 1) + 1;
+    int last = -1;                         /* last sweep in which this thread changed a value of the block's own */
     for (int b = 0, t0 = 0; t0 < steps; b++, t0 += H) {
         const int t_end = min(steps, t0 + H);
         for (int t = t0; t < t_end; t++) {
@@ -527,10 +540,11 @@ __global__ void __launch_bounds__(768) k_mg_coarse_cluster(MgConst m, MgLvlT<T> 
                 const int s_lo = tp > nz ? (tp - nz + 1) / 2 : 0;
                 const int s_hi = min(sweeps - 1, tp / 2);
                 const int na = s_hi - s_lo + 1;
-                if (a0 < na)
-                    relax_smem<T>(K, oxy, top_levels, nx, nz, first + 2 * cc0, tp - 2 * (s_lo + a0), Es, Rs, ins);
-                for (int q = tl + nhalf; q < na * ncol; q += nhalf)
-                    relax_smem<T>(K, oxy, top_levels, nx, nz, first + 2 * (q % ncol), tp - 2 * (s_lo + q / ncol), Es, Rs, ins);
+                auto relax = [&](int i, int s) {
+                    if (relax_smem<T>(K, oxy, top_levels, nx, nz, i, tp - 2 * s, Es, Rs, ins) && i >= c0 && i < c1) last = max(last, s);
+                };
+                if (a0 < na) relax(first + 2 * cc0, s_lo + a0);
+                for (int q = tl + nhalf; q < na * ncol; q += nhalf) relax(first + 2 * (q % ncol), s_lo + q / ncol);
             }
             __syncthreads();
         }
@@ -542,7 +556,10 @@ __global__ void __launch_bounds__(768) k_mg_coarse_cluster(MgConst m, MgLvlT<T> 
                 mine[q] = Es[k * W + c0 + h];
                 mine[H * NZ + q] = Es[k * W + c1 - H + h];
             }
+            const int warp_last = __reduce_max_sync(0xffffffffu, last);
+            if ((th & 31) == 0) atomicMax(&changed[b & 1], warp_last);
             cluster.sync();
+            if (th < C) atomicMax(&all_changed, *cluster.map_shared_rank(&changed[b & 1], th));
             const T* lsrc = pubL_left + (b & 1) * 2 * H * NZ + H * NZ;   /* left neighbour's last H columns */
             const T* rsrc = pubR_right + (b & 1) * 2 * H * NZ;           /* right neighbour's first H columns */
             for (int q = th; q < H * NZ; q += nth) {
@@ -552,6 +569,8 @@ __global__ void __launch_bounds__(768) k_mg_coarse_cluster(MgConst m, MgLvlT<T> 
                 if (xr < e1) Es[k * W + xr] = rsrc[q];
             }
             __syncthreads();
+            /* sweep s has ended with step 2 s + nz + 1 (its odd columns' last row) */
+            if (all_changed < (t_end - 1 - (nz + 1)) / 2 && t_end > nz + 1) break;
         }
     }
     cluster.sync();              /* no block leaves while another may read its buffers */

@@ -10,7 +10,7 @@ from baccolonygrowth_b200.colony import Colony, synth_colony
 
 import checkers as ck
 from test_gpu_fields import TOL, close, deplete, wall_mask
-from test_gpu_mg_tile import problem
+from test_gpu_mg_tile import colony, problem, solutions
 
 F = _abi.FIELDS
 SPECIES = ("CARBON", "OXYGEN", "ACETATE")
@@ -45,3 +45,17 @@ def test_solve_end_against_oracle(gpu, box_x, rows, levels):
         for sp in SPECIES:
             f = "WALLF_" + sp
             assert close(orc.field(F[f], l), col.field(f, l), mask=wall_mask(p, l)) <= TOL, (f, l)
+
+
+# the cluster form of the coarsest level stops at its fixed point: sweeps that
+# end before a row's wavefront has, before the fixed point, and long after it
+@pytest.mark.gpu
+@pytest.mark.parametrize("mu2", [1, 2, 9, 40, 300])
+def test_coarsest_level_stops_at_fixed_point(gpu, mu2):
+    p = problem(4608, 24, 3, mg_levels=6, mg_mu2=mu2)
+    a, b = colony(p, 3), colony(p, 0)
+    for _ in range(2):
+        a.mg_solve()
+        b.mg_solve()
+    for x, y in zip(solutions(a), solutions(b)):
+        assert np.abs(x - y).max() <= 1e-12 * max(np.abs(y).max(), 1e-300)
