@@ -1777,8 +1777,13 @@ extern "C" int bcg_mg_solve(bcg_ctx* c, int vcycles)
  * defect and of R go to out[0], out[1] as ordered bit patterns.
  * The relaxation constants come from the host and a block takes DEFECT_ROWS
  * rows before it touches the two words: with three divisions a point and
- * an atomic a warp it took 64 us (FP32) and 73 us (FP64) at 2305 x 513 points. */
+ * an atomic a warp it took 64 us (FP32) and 73 us (FP64) at 2305 x 513 points.
+ * A thread knows its column's case and works out a point's on the first and
+ * last rows only, and loads DEFECT_AHEAD rows before it uses the first: with the
+ * choice at every point, which kept the rows' loads apart, it waited for memory,
+ * 36 and 39 us; so 15 and 19. */
 #define DEFECT_ROWS 16
+#define DEFECT_AHEAD 8
 struct DefectConst { RelaxK<double> k[3]; double scale[3]; int nxp, nzp; };
 template <class T>
 __global__ void __launch_bounds__(256) k_mg_defect(MgConst m, MgLvlT<T> L, MgLvl L64, int l, DefectConst dc,
@@ -1792,14 +1797,46 @@ __global__ void __launch_bounds__(256) k_mg_defect(MgConst m, MgLvlT<T> L, MgLvl
     if (i <= L.nx) {
         const int ip = 2 * i - L.nx + dc.nxp / 2;
         const bool column = l == 0 || ip <= 0 || ip >= dc.nxp;
-        for (int k = column ? k0 : max(k0, (dc.nzp + 1) / 2); k < k1; k++) {
+        const int kb = column ? k0 : max(k0, (dc.nzp + 1) / 2);
+        auto point = [&](int k) {
             int kind;
             const double v = relax_eval<T>(m, L, SP(L64.r), l, sp, i, k, inside0, kind, K);
-            if (kind == 0) continue;
+            if (kind == 0) return;
             const double d = v - (double)AT(SP(L.e), L, i, k);
             dmax = fmax(dmax, fabs(kind == 1 ? d : d * scale));
             rmax = fmax(rmax, fabs(AT(SP(L64.r), L64, i, k)));
+        };
+        const bool side = i == 0 || i == L.nx, top_levels = l >= m.A - 1, given = side && sp == 1;
+        const double sc = given ? 1.0 : scale;
+        const size_t P = L.pitch;
+        const ptrdiff_t left = i == 0 ? 1 : -1, right = i == L.nx ? -1 : 1;
+        const T* __restrict__ e = SP(L.e) + i;
+        const double* __restrict__ r = SP(L64.r) + i;
+        if (kb == 0 && k1 > 0) point(0);
+        if (!side || top_levels) {
+            const int ke = min(k1, L.nz);
+            for (int k = max(kb, 1); k < ke; k += DEFECT_AHEAD) {
+                T c[DEFECT_AHEAD + 2], xm[DEFECT_AHEAD], xp[DEFECT_AHEAD];
+                double rk[DEFECT_AHEAD];
+#pragma unroll
+                for (int j = 0; j < DEFECT_AHEAD + 2; j++) c[j] = e[min(k - 1 + j, L.nz) * P];
+#pragma unroll
+                for (int j = 0; j < DEFECT_AHEAD; j++) {
+                    const size_t at = min(k + j, L.nz) * P;
+                    xm[j] = e[at + left]; xp[j] = e[at + right]; rk[j] = r[at];
+                }
+#pragma unroll
+                for (int j = 0; j < DEFECT_AHEAD; j++) {
+                    const double b = (double)c[j], u = (double)c[j + 2], xl = (double)xm[j], xr = (double)xp[j];
+                    const double v = given ? rk[j] : side ? rx_side(rk[j], b, u, xl, K) : rx_in(rk[j], b, u, xl, xr, K);
+                    if (k + j < ke) {
+                        dmax = fmax(dmax, fabs((v - (double)c[j + 1]) * sc));
+                        rmax = fmax(rmax, fabs(rk[j]));
+                    }
+                }
+            }
         }
+        if (kb <= L.nz && k1 > L.nz && L.nz > 0) point(L.nz);
     }
     for (int o = 16; o >= 1; o >>= 1) {
         dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));

@@ -59,3 +59,23 @@ def test_coarsest_level_stops_at_fixed_point(gpu, mu2):
         b.mg_solve()
     for x, y in zip(solutions(a), solutions(b)):
         assert np.abs(x - y).max() <= 1e-12 * max(np.abs(y).max(), 1e-300)
+
+
+# blocks of 16 rows, eight loaded together; 37 rows of points.  Without sweeps the
+# correction stays zero, so the relaxation's defect is Res itself and the ratio 1
+# up to the rounding of c R (cf + 2) / cf; a row that were left out would give 0.
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("k", [1, 7, 8, 9, 14, 15, 16, 17, 24, 31, 32, 33, 35])
+def test_defect_sees_every_row(gpu, k, precision):
+    p = problem(256, 36, 2, mg_mu1=0, mg_mu2=0)
+    col = Colony(p, synth_colony(200, *params.dome_size(200, 1.0 / 10.0), seed=5))
+    for l in range(2):
+        n = len(col.field("MG_SOL_CARBON", l))
+        sol = np.full((n // 37, 37), 8.0)
+        if l == 0:
+            sol[101, k] = 7.0
+        col.set_field("MG_SOL_CARBON", sol.reshape(-1), l)
+    it, rel = col.mg_solve_tol(1e-300, precision, 1)
+    assert it == 1 and abs(rel - 1.0) <= 1e-14, (it, rel)
+    col.close()
