@@ -373,15 +373,17 @@ int bcg_autotune(bcg_ctx* ctx, int what, int* choice);
 
 /* Fixed kernel shapes for one context, for profiling and for tests of the
  * variants (each drops the context's captured graphs):
- *   bcg_set_force_group    lanes per cell in MoveCell+GrowCell: 1, 2, 4
- *                          (default), 8 or 16; the results do not depend
- *                          on it;
+ *   bcg_set_force_group    lanes per cell in MoveCell+GrowCell: 1, 2, 4,
+ *                          8 or 16 (unset: 8 for small colonies down to
+ *                          1 for large ones); the results differ by
+ *                          rounding only;
  *   bcg_set_relax_mode     agar smoother form: 0 = one thread per column
  *                          and half-sweep, 1 = half-sweeps with row
  *                          segments, 2 = fused sweeps with rows staged per
  *                          lane, 3 = fused sweeps with rows staged by the
- *                          tensor memory accelerator (default); the forms
- *                          agree to rounding;
+ *                          tensor memory accelerator, FP64 levels up to
+ *                          1.8 million points on register tiles
+ *                          (default); the forms agree to rounding;
  *   bcg_set_smoother_warps resident-warp target of the fused smoother
  *                          (0 = default or tuned);
  *   bcg_smoother_launch_ms device time of one finest-level launch of the
