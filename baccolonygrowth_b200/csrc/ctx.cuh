@@ -115,6 +115,7 @@ struct bcg_ctx {
     int nutrient_graph_sweeps;           /* 0: none captured (dropped whenever a kernel choice changes) */
     int nutrient_graph_launches[2];
     int nutrient_graph_blocked;          /* tile of the blocked sweeps they hold (0: single sweeps) */
+    int nutrient_graph_clean[2];         /* mg_clean when captured */
     /* the captured per-step solve (bcg_mg_solve): its key (V-cycles, wall
      * buffer, whether Err and Res were clean on entry; -1: none) */
     cudaGraphExec_t solve_graph;

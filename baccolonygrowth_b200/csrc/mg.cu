@@ -1654,6 +1654,12 @@ void mg_finish(bcg_ctx* c, const MgConst& m, int cur_wall)
     k_mg_finish<<<a.first[a.levels], 256, 0, c->stream>>>(m, a);
     k_mg_walls<<<dim3((unsigned)((most + 255) / 256), 3, (unsigned)m.A), 256, 0, c->stream>>>(m, a);
     c->launches += 2;
+    mg_solved(c);
+}
+
+/* the host's notes on the agar arrays after a solve, queued or replayed */
+void mg_solved(bcg_ctx* c)
+{
     c->mg_res0_stale = 1;
     c->mg_clean = 1;
     c->leg_old_stale = 1;        /* copyFromMG writes FieldAgar and oldFieldAgar alike */
@@ -1740,13 +1746,9 @@ static int mg_solve_graphed(bcg_ctx* c, int vcycles, int wall_buf, cudaStream_t 
             return mg_solve_impl(c, vcycles, wall_buf);
         }
         c->solve_graph_key = key;
-    } else {
-        /* the host state a solve leaves (mg_setup, mg_finish) */
-        c->mg_res0_stale = 1;
-        c->mg_clean = 1;
-        c->leg_old_stale = 1;
     }
     BCG_CUDA_TRY(cudaGraphLaunch(c->solve_graph, launch));
+    mg_solved(c);
     c->launches += c->solve_graph_launches;
     return BCG_OK;
 }

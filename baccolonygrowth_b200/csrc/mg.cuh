@@ -33,6 +33,7 @@ void mg_vcycle(bcg_ctx* c, const MgConst& m, int mu1, int mu2);
 void mg_setup(bcg_ctx* c, const MgConst& m);
 void mg_copy_to(bcg_ctx* c, const MgConst& m, int wall_buf);
 void mg_finish(bcg_ctx* c, const MgConst& m, int cur_wall);
+void mg_solved(bcg_ctx* c);
 int mg_solve_impl(bcg_ctx* c, int vcycles, int wall_buf);
 /* the TMA-staged fused smoother (mg_smooth.cu): S sweeps of level L from
  * E into E2 with about `target_warps` warps (one row segment of one strip

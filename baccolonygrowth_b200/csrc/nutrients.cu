@@ -773,21 +773,31 @@ static int nutrient_unit_graph(bcg_ctx* c, int sweeps, int last, cudaGraphExec_t
         c->nutrient_graph_sweeps = sweeps;
         c->nutrient_graph_blocked = blocked;
     }
+    /* a unit captured from clean Err and Res leaves out the first steps of
+     * setup(); one captured from any other state runs them and replays from both */
+    if (c->nutrient_graph[last] && c->nutrient_graph_clean[last] && !c->mg_clean) {
+        cudaGraphExecDestroy(c->nutrient_graph[last]);
+        c->nutrient_graph[last] = nullptr;
+    }
     if (!c->nutrient_graph[last]) {
-        cudaGraph_t g;
+        cudaGraph_t g = nullptr;
+        /* a capture runs nothing on the device: what it does to the host's
+         * notes on the agar arrays is undone */
+        const int s_clean = c->mg_clean, s_res0 = c->mg_res0_stale, s_leg = c->leg_old_stale;
         BCG_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         long long l0 = c->launches;
         int ce = 0, cw = 0, count = 0;
         int rc = mg_solve_impl(c, c->P.mg_vcycles, cw);
         if (rc == BCG_OK) run_sweeps(c, sweeps, ce, cw, count, last ? sweeps - 2 : sweeps);
         cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-        if (rc) return rc;
-        if (e != cudaSuccess) { bcg_set_cuda_error(e); return BCG_E_CUDA; }
+        c->mg_clean = s_clean; c->mg_res0_stale = s_res0; c->leg_old_stale = s_leg;
         c->nutrient_graph_launches[last] = (int)(c->launches - l0);
         c->launches = l0;
-        e = cudaGraphInstantiate(&c->nutrient_graph[last], g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) { bcg_set_cuda_error(e); return BCG_E_CUDA; }
+        if (rc == BCG_OK && e == cudaSuccess) e = cudaGraphInstantiate(&c->nutrient_graph[last], g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (rc) return rc;
+        if (e != cudaSuccess) { c->nutrient_graph[last] = nullptr; bcg_set_cuda_error(e); return BCG_E_CUDA; }
+        c->nutrient_graph_clean[last] = s_clean;
     }
     *out = c->nutrient_graph[last];
     return BCG_OK;
@@ -810,6 +820,7 @@ extern "C" int bcg_nutrient_update(bcg_ctx* c, int n, int sweeps)
             int rc = nutrient_unit_graph(c, sweeps, last, &ge);
             if (rc) return rc;
             BCG_CUDA_TRY(cudaGraphLaunch(ge, c->stream));
+            mg_solved(c);
             c->launches += c->nutrient_graph_launches[last];
         }
     } else {

@@ -1,0 +1,83 @@
+"""A nutrient update whose units replay captured graphs against one that
+captures them anew (changing the smoother form and back drops the graphs):
+the same kernels on the same values, so all of it is equal bit for bit, also
+what the library works out only when it is read (level 0's Res after a solve)
+and the second agar buffer that the legacy solver takes up after a solve."""
+import numpy as np
+import pytest
+
+from baccolonygrowth_b200 import params
+from baccolonygrowth_b200.colony import Colony, workload_colony
+
+pytestmark = pytest.mark.gpu
+SPECIES = ("CARBON", "OXYGEN", "ACETATE")
+
+
+def pair():
+    out = []
+    for _ in range(2):
+        col = Colony(params.workload_params("small_4k"), workload_colony("small_4k", n=1024))
+        col.update_density()
+        col.deplete_wall()
+        out.append(col)
+    return out
+
+
+def recapture(col):
+    for mode in (2, 3):
+        assert col.lib.bcg_set_relax_mode(col.h, mode) == 0
+
+
+def update(a, b, units=2):
+    """`a` replays, `b` captures."""
+    recapture(b)
+    a.nutrient_update(units)
+    b.nutrient_update(units)
+
+
+def equal(a, b, names):
+    for name in names:
+        for l in range(a.params.max_levels_mg):
+            assert np.array_equal(a.field(name, l), b.field(name, l)), (name, l)
+
+
+@pytest.mark.parametrize("between", ["density", "read", "none"])
+def test_res_after_replay(gpu, between):
+    a, b = pair()
+    update(a, b)
+    for _ in range(2):
+        for col in (a, b):
+            if between == "density":
+                col.update_density()
+            elif between == "read":
+                col.field("MG_SOL_CARBON", 0)
+        update(a, b)
+    equal(a, b, ["MG_%s_%s" % (k, s) for k in ("RES", "ERR", "SOL") for s in SPECIES])
+    assert np.abs(a.field("MG_RES_CARBON", 0)).max() > 0
+    a.close(); b.close()
+
+
+def test_legacy_after_replay(gpu):
+    a, b = pair()
+    update(a, b)
+    for _ in range(2):
+        for col in (a, b):
+            col.legacy_env_update(3)
+        update(a, b)
+    for col in (a, b):
+        col.legacy_env_update(3)
+    equal(a, b, ["AGARF_" + s for s in SPECIES] + ["%sWALLF_%s" % (o, s) for o in ("", "OLD") for s in SPECIES])
+    a.close(); b.close()
+
+
+def test_replay_after_write(gpu):
+    """Err and Res that a caller wrote are not taken for the zeros a solve
+    leaves."""
+    a, b = pair()
+    update(a, b)
+    err = np.random.default_rng(1).standard_normal(a.field("MG_ERR_CARBON", 0).size)
+    for col in (a, b):
+        col.set_field("MG_ERR_CARBON", err, 0)
+    update(a, b)
+    equal(a, b, ["MG_SOL_" + s for s in SPECIES])
+    a.close(); b.close()
