@@ -343,17 +343,30 @@ extern "C" int bcg_rebuild_neighbours(bcg_ctx* c)
 /* ======================================================================= */
 /* MoveCell + GrowCell                                                      */
 /* ======================================================================= */
-/* One lane per cell (G = 1): the neighbours' records pass through shared memory.
+/* STAGED (one lane per cell): the neighbours' records pass through shared memory.
  * A lane that gathers its own neighbour's 128 bytes touches a line of its own
  * with each of eight loads and waits for them; here the warp fetches its 32
  * neighbours together, eight lanes a record, asynchronously, the next neighbour
  * while it works on this one.  A record's 16-byte pieces are rotated by its lane,
  * so that the lanes' reads of one piece meet no bank twice.  Two slots a warp.
- * The cells' own records come and go the same way.  What remains is the FP64
- * chain of a pair's force: a scheduler issues an instruction every 2 cycles
- * (before, every 5), its FP64 pipe is 40% busy.  262144 cells with 6 neighbours:
- * 145 us, gathered 167. */
+ * The cells' own records come and go the same way.
+ *
+ * The copies pass L1 by, which serves a gathered record to several lanes, and
+ * cost instructions; they gain where a few waves of blocks leave the first loads
+ * unhidden and lose on larger colonies.  A launch of a dense colony (6
+ * neighbours) within its steps, us, one lane a cell, 4 blocks an SM:
+ *   cells             45000  80000  131072  200000  225000  262144  1048576
+ *   FP64 staged          48     77      95     143     162     188      647
+ *        gathered        50     81      99     137     145     173      557
+ *   FP32 staged          57     91     121     199     229     270     1038
+ *        gathered        58     91     112     165     190     220      797
+ * (with 3 blocks an SM staged 177 and 577 at 262144 and 1048576 cells, FP64).  A
+ * loose colony (2 neighbours) crosses at the same sizes: 74 and 75 us at
+ * 200000 cells, FP64.  In launches on a standing colony the staged form had looked
+ * the faster one at 262144 cells too (145 us, gathered 167). */
 #define STAGE_BYTES (32 * 128)
+#define STAGE_CELLS 200000           /* largest colony that is staged */
+#define STAGE_CELLS_F32 100000       /* ... with the FP32 contact search */
 __device__ __forceinline__ void stage_fetch(unsigned char* slot, const CellRec* __restrict__ rec, int id)
 {
     const int lane = threadIdx.x & 31, piece = lane & 7;
@@ -398,7 +411,7 @@ __device__ __forceinline__ Cst stage_read(const unsigned char* slot)
 /* Forces on `a` from its neighbour list (lanes of a G-wide group split the
  * list; the group reduces with a fixed butterfly), plus the wall, drag and
  * surface-tension terms (sum_forces, Forces.cpp:332-381). */
-template <int G, bool GEOM32>
+template <int G, bool GEOM32, bool STAGED>
 __device__ __forceinline__ void sum_forces_group(const Cst& a, int me, const CellRec* __restrict__ old,
                                                  const int* __restrict__ list, int cnt, double wall_z,
                                                  const FieldPtrs& fp, const MechParams& mp,
@@ -407,7 +420,7 @@ __device__ __forceinline__ void sum_forces_group(const Cst& a, int me, const Cel
     const int gl = threadIdx.x & (G - 1);
     V3 cm = avg_pq(a.p, a.q);
     V3 F = mk(0, 0, 0), T = mk(0, 0, 0);
-    if (G == 1) {
+    if (STAGED) {
         /* the caller has fetched the first neighbours into slot 0 */
         const int most = __reduce_max_sync(0xffffffffu, cnt);
         int next = 1 < cnt ? __ldg(&list[1]) : -1;
@@ -466,7 +479,7 @@ __device__ __forceinline__ void sum_forces_group(const Cst& a, int me, const Cel
 
 /* MB = the blocks of 128 threads an SM is to hold: 4 caps the registers at
  * 128 (some spill), 3 at 170 (none spill); the autotuner picks. */
-template <int G, bool GEOM32, int MB>
+template <int G, bool GEOM32, int MB, bool STAGED>
 __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const int* __restrict__ order,
         const CellRec* __restrict__ old, CellRec* __restrict__ nw,
         const int* __restrict__ nbr, const int* __restrict__ ncount,
@@ -483,14 +496,15 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
     int me = active ? (t < nbinned ? __ldg(&order[t]) : t) : 0;
     int near1 = 0, near2 = 0;
     bool told = false;             /* this lane left something for the last block to read */
-    constexpr int SLOTS = G == 1 ? 4 * 2 : 0;        /* two a warp of 128 threads */
+    static_assert(!STAGED || G == 1, "a staged record belongs to one lane");
+    constexpr int SLOTS = STAGED ? 4 * 2 : 0;        /* two a warp of 128 threads */
     __shared__ __align__(128) unsigned char stages[SLOTS ? SLOTS * STAGE_BYTES : 16];
-    unsigned char* stage = stages + (G == 1 ? (threadIdx.x >> 5) * 2 * STAGE_BYTES : 0);
+    unsigned char* stage = stages + (STAGED ? (threadIdx.x >> 5) * 2 * STAGE_BYTES : 0);
     {
         const int* list = nbr + (size_t)me * mp.kmax;
-        const int cnt = active || G > 1 ? __ldg(&ncount[me]) : 0;
+        const int cnt = active || !STAGED ? __ldg(&ncount[me]) : 0;
         Cst o;
-        if (G == 1) {
+        if (STAGED) {
             /* the cells' own records by the same way, then the first neighbours */
             stage_fetch(stage + STAGE_BYTES, old, me);
             stage_fetch(stage, old, cnt > 0 ? __ldg(&list[0]) : -1);
@@ -506,7 +520,7 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
         double wall_z = __ldg(&fp.wall[xi * mp.box_y + yi]);
         V3 F, T, sf, df;
         /* integrate, Integrate.cpp:11-32 */
-        sum_forces_group<G, GEOM32>(o, me, old, list, cnt, wall_z, fp, mp, F, T, sf, df, near1, stage, true);
+        sum_forces_group<G, GEOM32, STAGED>(o, me, old, list, cnt, wall_z, fp, mp, F, T, sf, df, near1, stage, true);
         Cst tmp = o;
         half_kick(dt, F, T, o, tmp.v, tmp.w);
         V3 rcmp = sub3(o.p, ocm), rcmq = sub3(o.q, ocm);
@@ -514,7 +528,7 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
         tmp.p = add3(o.p, scl3(vp, dt));
         tmp.q = add3(o.q, scl3(vq, dt));
         tmp.p.y = 0; tmp.q.y = 0;
-        sum_forces_group<G, GEOM32>(tmp, me, old, list, cnt, wall_z, fp, mp, F, T, sf, df, near2, stage, false);
+        sum_forces_group<G, GEOM32, STAGED>(tmp, me, old, list, cnt, wall_z, fp, mp, F, T, sf, df, near2, stage, false);
         Cst nc = tmp;
         half_kick(dt, F, T, tmp, nc.v, nc.w);
         nc.v.y = 0;
@@ -537,9 +551,9 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
         r.qR = make_double4(nc.q.x, nc.q.y, nc.q.z, nc.R);
         r.v = make_double4(nc.v.x, nc.v.y, nc.v.z, 0.0);
         r.w = make_double4(nc.w.x, nc.w.y, nc.w.z, 0.0);
-        if (G == 1) stage_store(stage, nw, active ? me : -1, r);
+        if (STAGED) stage_store(stage, nw, active ? me : -1, r);
         if (gl == 0 && active) {
-            if (G > 1) nw[me] = r;
+            if (!STAGED) nw[me] = r;
             soa.gr[me] = g;
             soa.dfx[me] = df.x; soa.dfy[me] = df.y; soa.dfz[me] = df.z;
             soa.sfx[me] = sf.x; soa.sfy[me] = sf.y; soa.sfz[me] = sf.z;
@@ -587,7 +601,7 @@ __global__ void __launch_bounds__(128, MB) k_move_grow(int n, int nbinned, const
  * of 4 blocks of 128 on 148 SMs, and one where a lane a cell fills more than
  * that.  Below the line more lanes shorten the walk over a cell's neighbours;
  * above it they only add what each lane does again.  Dense colonies (6
- * neighbours), us a launch:
+ * neighbours) that stand still, one lane staged, us a launch:
  *   cells      1000  4096  16384  32768  65536  262144
  *   8 lanes    18.8  21.2   32.5   48.0   77.9   268
  *   4          21.0  21.4   26.9   40.5   61.1   191
@@ -624,11 +638,13 @@ int launch_move_grow(bcg_ctx* c, double dt, int group, int occ)
         unsigned blocks = (unsigned)((tot + threads - 1) / threads);
         const CellRec* old = c->rec[c->cur];
         CellRec* nw = c->rec[c->cur ^ 1];
-#define MG_ARGS(G, M, B) k_move_grow<G, M, B><<<blocks, threads, 0, c->stream>>>(n, nb, c->box_ids, old, nw, c->nbr, c->ncount, \
+        const bool staged = n <= (c->pair_f32 ? STAGE_CELLS_F32 : STAGE_CELLS);
+#define MG_ARGS(G, M, B, S) k_move_grow<G, M, B, S><<<blocks, threads, 0, c->stream>>>(n, nb, c->box_ids, old, nw, c->nbr, c->ncount, \
             c->soa, fp, mp, dt, c->div_list, c->step, c->step_host)
 #define MG_GROUPS(M, B) switch (group) { \
-            case 1: MG_ARGS(1, M, B); break; case 2: MG_ARGS(2, M, B); break; case 4: MG_ARGS(4, M, B); break; \
-            case 8: MG_ARGS(8, M, B); break; default: MG_ARGS(16, M, B); break; }
+            case 1: if (staged) MG_ARGS(1, M, B, true); else MG_ARGS(1, M, B, false); break; \
+            case 2: MG_ARGS(2, M, B, false); break; case 4: MG_ARGS(4, M, B, false); break; \
+            case 8: MG_ARGS(8, M, B, false); break; default: MG_ARGS(16, M, B, false); break; }
         if (c->pair_f32) { if (occ == 3) { MG_GROUPS(true, 3) } else { MG_GROUPS(true, 4) } }
         else { if (occ == 3) { MG_GROUPS(false, 3) } else { MG_GROUPS(false, 4) } }
 #undef MG_GROUPS
