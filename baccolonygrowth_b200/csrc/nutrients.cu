@@ -17,6 +17,7 @@
  */
 #include "ctx.cuh"
 #include "mg.cuh"
+#include "sweep_rows.h"
 #include <float.h>
 #include <vector>
 
@@ -401,10 +402,6 @@ static void sweep_launch(dim3 grid, dim3 block, bcg_ctx* c, const NutConst& n, E
  * Measured a sweep, launches included: 33 thousand cells 8.9 -> 3.1 us (tiles of
  * 4), a million 19 -> 14.6 us (tiles of 16).  It is bound by instruction issue: 0.64
  * a cycle and scheduler at a million cells, 1.6 points computed for one owned. */
-#define SW_K 4               /* sweeps a launch, even: the buffers' roles return */
-#define SW_RZ 40             /* rows of a tile with its halo */
-#define SW_OWN0 (SW_RZ - 1 - SW_K)        /* rows z = 0 .. of the bottom tile where others follow */
-#define SW_OWN (SW_RZ - 2 * SW_K)         /* rows of the tiles above it */
 /* A tile's columns.  16 recompute least (1.6 points for one) and fill the SMs
  * from about 150 tiles on; fewer tiles leave SMs idle and a block's own chain of
  * instructions is what counts, so smaller tiles with a thread a point. */
@@ -540,10 +537,8 @@ __global__ void __launch_bounds__(SwTile<TX>::THREADS, TX == 16 ? 2 : 1) k_sweep
     }
     const int zt = blockIdx.y - 1, x0 = minx + blockIdx.x * TX;
     const bool floor_ = zt == 0;
-    const int z0 = floor_ ? 0 : SW_OWN0 + (zt - 1) * SW_OWN;
-    if (x0 > maxx || z0 > maxz) return;
-    /* a bottom tile that reaches over the box's top has no tile above */
-    const int z1 = floor_ ? (maxz + 2 < SW_RZ ? maxz + 1 : SW_OWN0) : z0 + SW_OWN;
+    if (x0 > maxx || zt >= sw_tile_rows(maxz)) return;
+    const int z0 = sw_first(zt), z1 = sw_end(zt, maxz);
     const int zb = floor_ ? -1 : z0 - SW_K, xb = x0 - SW_K;       /* of row and column 0 */
     double* v = reinterpret_cast<double*>(sw_smem);              /* [buffer][species][column][row] */
     double* sds = v + 8 * P;
@@ -665,7 +660,7 @@ static int sweep_tile(const bcg_ctx* c)
 {
     if (!sweeps_block(c)) return 0;
     const int* b = c->host_bbox;
-    const int w = b[1] - b[0] + 1, zt = b[2] + 2 < SW_RZ ? 1 : 1 + (b[2] + 1 - SW_OWN0 + SW_OWN - 1) / SW_OWN;
+    const int w = b[1] - b[0] + 1, zt = sw_tile_rows(b[2]);
     for (int tx = 4; tx < 16; tx *= 2) if ((w + tx - 1) / tx * zt <= 148) return tx;
     return 16;
 }
