@@ -79,8 +79,11 @@ int ctx_take_status(bcg_ctx* c)
 
 int ctx_check_status_bbox(bcg_ctx* c)
 {
-    BCG_CUDA_TRY(cudaMemcpyAsync(c->host_bbox, c->bbox, sizeof(c->host_bbox), cudaMemcpyDeviceToHost, c->stream));
-    return ctx_check_status(c);
+    int b[3];
+    BCG_CUDA_TRY(cudaMemcpyAsync(b, c->bbox, sizeof(b), cudaMemcpyDeviceToHost, c->stream));
+    const int rc = ctx_check_status(c);
+    if (rc == BCG_OK) memcpy(c->host_bbox, b, sizeof(b));
+    return rc;
 }
 
 int ensure_pinned(bcg_ctx* c, size_t bytes)

@@ -187,5 +187,5 @@ void mg_res0_materialise(bcg_ctx* c);
 int mg_kernel_attributes();
 int mech_kernel_attributes();
 int sweep_kernel_attributes();
-/* read bbox into host_bbox; part of the status check that ends a deposition */
+/* the status check that ends a deposition: bbox into host_bbox if it is BCG_OK */
 int ctx_check_status_bbox(bcg_ctx* c);
