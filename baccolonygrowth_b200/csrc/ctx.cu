@@ -98,11 +98,12 @@ int ensure_pinned(bcg_ctx* c, size_t bytes)
 
 void timer_begin(bcg_ctx* c, int t)
 {
+    c->timer_l0[t] = c->launches;
     if (c->timers_on) cudaEventRecord(c->ev[t][0], c->stream);
 }
-void timer_end(bcg_ctx* c, int t, int launches)
+void timer_end(bcg_ctx* c, int t)
 {
-    c->timer_launches[t] += launches;
+    c->timer_launches[t] += c->launches - c->timer_l0[t];
     if (c->timers_on) {
         cudaEventRecord(c->ev[t][1], c->stream);
         cudaEventSynchronize(c->ev[t][1]);

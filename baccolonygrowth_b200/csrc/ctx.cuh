@@ -136,7 +136,7 @@ struct bcg_ctx {
     int tl_cap, tl_n;
     cudaEvent_t ev[BCG_T_COUNT][2];
     double timer_ms[BCG_T_COUNT];
-    long long timer_launches[BCG_T_COUNT];
+    long long timer_launches[BCG_T_COUNT], timer_l0[BCG_T_COUNT];
     long long launches;    /* kernels queued by this context (all kinds) */
     /* kernel shapes of this context, chosen by bcg_autotune or set by the
      * caller (0 = default); no kernel choice is process-wide */
@@ -170,7 +170,7 @@ FieldPtrs field_ptrs(const bcg_ctx* c);
 int ctx_check_status(bcg_ctx* c);   /* syncs, reads the device status word */
 int ctx_take_status(bcg_ctx* c);    /* the word as the last synchronised read left it */
 void timer_begin(bcg_ctx* c, int t);
-void timer_end(bcg_ctx* c, int t, int launches);
+void timer_end(bcg_ctx* c, int t);  /* the launches since timer_begin count as t's */
 int ensure_pinned(bcg_ctx* c, size_t bytes);
 void nutrient_graphs_drop(bcg_ctx* c);
 int launch_move_grow(bcg_ctx* c, double dt, int group, int occ);

@@ -271,7 +271,7 @@ static int deposit(bcg_ctx* c, bool smooth)
     c->launches += 7;
     rc = launch_surface(c, smooth);
     if (rc) return rc;
-    timer_end(c, BCG_T_DENSITY, 0);
+    timer_end(c, BCG_T_DENSITY);
     return ctx_check_status_bbox(c);
 }
 
@@ -295,6 +295,6 @@ extern "C" int bcg_update_height(bcg_ctx* c)
     c->launches += 3;
     rc = launch_surface(c, true);
     if (rc) return rc;
-    timer_end(c, BCG_T_DENSITY, 0);
+    timer_end(c, BCG_T_DENSITY);
     return ctx_check_status(c);
 }

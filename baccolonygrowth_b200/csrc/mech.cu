@@ -336,7 +336,7 @@ extern "C" int bcg_rebuild_neighbours(bcg_ctx* c)
         c->launches++;
     }
     BCG_CUDA_TRY(cudaGetLastError());
-    timer_end(c, BCG_T_NEIGHBOURS, 5);
+    timer_end(c, BCG_T_NEIGHBOURS);
     return BCG_OK;
 }
 
@@ -686,7 +686,7 @@ extern "C" int bcg_move_grow(bcg_ctx* c, double dt, int* n_div, int64_t* fcw_cal
     timer_begin(c, BCG_T_MOVE_GROW);
     int rc = launch_move_grow(c, dt, force_group_of(c), force_occ_of(c));
     if (rc) return rc;
-    timer_end(c, BCG_T_MOVE_GROW, c->n > 0 ? 1 : 0);
+    timer_end(c, BCG_T_MOVE_GROW);
     return move_grow_finish(c, n_div, fcw_calls);
 }
 
@@ -1160,11 +1160,10 @@ extern "C" int bcg_divide(bcg_ctx* c, const float* draws, int n_draw_sets, doubl
 {
     if (!c) return BCG_E_ARG;
     timer_begin(c, BCG_T_DIVIDE);
-    const int ndiv = c->last_ndiv;
     int rc = divide_launch(c, draws, n_draw_sets, t);
     if (rc) return rc;
     rc = divide_finish(c, n_done, lineage);
-    timer_end(c, BCG_T_DIVIDE, ndiv > 0 ? 7 : 0);
+    timer_end(c, BCG_T_DIVIDE);
     return rc;
 }
 

@@ -1758,10 +1758,9 @@ extern "C" int bcg_mg_solve(bcg_ctx* c, int vcycles)
     if (!c) return BCG_E_ARG;
     if (vcycles <= 0) vcycles = c->P.mg_vcycles;
     timer_begin(c, BCG_T_MG_SOLVE);
-    long long l0 = c->launches;
     int rc = mg_solve_graphed(c, vcycles, 0, c->stream);
     if (rc) return rc;
-    timer_end(c, BCG_T_MG_SOLVE, (int)(c->launches - l0));
+    timer_end(c, BCG_T_MG_SOLVE);
     return ctx_check_status(c);
 }
 
@@ -1915,7 +1914,6 @@ extern "C" int bcg_mg_solve_tol(bcg_ctx* c, double rel_tol, int precision, int m
 {
     if (!c || rel_tol <= 0 || max_iters < 1 || (precision != 32 && precision != 64)) return BCG_E_ARG;
     timer_begin(c, BCG_T_MG_SOLVE);
-    long long l0 = c->launches;
     MgConst m = mg_const(c, c->P.mg_dt);
     mg_copy_to(c, m, 0);
     mg_setup(c, m);
@@ -1954,7 +1952,7 @@ extern "C" int bcg_mg_solve_tol(bcg_ctx* c, double rel_tol, int precision, int m
     } else rel = 0.0;
     mg_finish(c, m, 0);
     BCG_CUDA_TRY(cudaGetLastError());
-    timer_end(c, BCG_T_MG_SOLVE, (int)(c->launches - l0));
+    timer_end(c, BCG_T_MG_SOLVE);
     if (iters) *iters = it;
     if (rel_res) *rel_res = rel;
     return ctx_check_status(c);

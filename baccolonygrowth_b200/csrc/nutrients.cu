@@ -737,10 +737,9 @@ extern "C" int bcg_colony_sweeps(bcg_ctx* c, int sweeps, int count0)
     if (c->P.nutrient_gsi != 0) return BCG_E_UNSUPPORTED;
     timer_begin(c, BCG_T_SWEEPS);
     int ce = 0, cw = 0, count = count0;
-    long long l0 = c->launches;
     run_sweeps(c, sweeps, ce, cw, count, sweeps - 2);
     BCG_CUDA_TRY(cudaGetLastError());
-    timer_end(c, BCG_T_SWEEPS, (int)(c->launches - l0));
+    timer_end(c, BCG_T_SWEEPS);
     return ctx_check_status(c);
 }
 
@@ -807,7 +806,6 @@ extern "C" int bcg_nutrient_update(bcg_ctx* c, int n, int sweeps)
     if (n <= 0) n = P.solves_per_update > 0 ? P.solves_per_update : (int)(3600 * P.update_time * 740 / P.mg_dt);
     if (sweeps < 0) sweeps = P.sweeps_per_solve;
     timer_begin(c, BCG_T_SWEEPS);
-    long long l0 = c->launches;
     if (sweeps % 2 == 0 && sweeps >= 2) {
         for (int i = 0; i < n; i++) {
             int last = (i == n - 1);
@@ -827,7 +825,7 @@ extern "C" int bcg_nutrient_update(bcg_ctx* c, int n, int sweeps)
         }
     }
     BCG_CUDA_TRY(cudaGetLastError());
-    timer_end(c, BCG_T_SWEEPS, (int)(c->launches - l0));
+    timer_end(c, BCG_T_SWEEPS);
     return ctx_check_status(c);
 }
 
@@ -1295,7 +1293,6 @@ extern "C" int bcg_legacy_env_update(bcg_ctx* c, int min_iter, int max_iter, dou
     if ((rc = leg_transfer(c, 0))) return rc;
     BCG_CUDA_TRY(cudaMemsetAsync(leg_counts(c), 0, sizeof(unsigned long long) * (size_t)(max_iter > 0 ? max_iter : 1), c->stream));
     timer_begin(c, BCG_T_SWEEPS);
-    long long l0 = c->launches;
     LegArgs a;
     a.n = nut_const(c);
     a.ZA = P.box_z_agar;
@@ -1352,7 +1349,7 @@ extern "C" int bcg_legacy_env_update(bcg_ctx* c, int min_iter, int max_iter, dou
     }
     if ((rc = leg_transfer(c, 1))) return rc;
     BCG_CUDA_TRY(cudaGetLastError());
-    timer_end(c, BCG_T_SWEEPS, (int)(c->launches - l0));
+    timer_end(c, BCG_T_SWEEPS);
     if (iterations) *iterations = count;
     return ctx_check_status(c);
 }

@@ -429,7 +429,8 @@ int bcg_steady_vjp(bcg_steady* s, const double* dL_dC, double* grad_theta, doubl
 
 /* ------------------------------------------------------------------ */
 /* timing: device time of the kernels queued by the last call of each    */
-/* kind (CUDA events on the context stream), in milliseconds.            */
+/* kind (CUDA events on the context stream), in milliseconds, and the    */
+/* kernels they launched, since bcg_enable_timers.                       */
 /* ------------------------------------------------------------------ */
 typedef enum bcg_timer_id {
     BCG_T_MOVE_GROW = 0, BCG_T_DIVIDE = 1, BCG_T_NEIGHBOURS = 2,
