@@ -222,7 +222,7 @@ __device__ __forceinline__ void st_half_sweep(double* sx, double* sb, const doub
  * here (r -= alpha Ap, x += alpha p) with its max-norm.  SMOOTH = false (a
  * one-level hierarchy): the CG step alone. */
 template <int T, bool CG, bool SMOOTH>
-__global__ void __launch_bounds__(StTile<T>::THREADS) k_st_down(StLevel L, StLevel Lc, StCg cg)
+__global__ void __launch_bounds__(StTile<T>::THREADS) k_st_down(StLevel L, StLevel Lc, StCg cg, int row0)
 {
     constexpr int THREADS = StTile<T>::THREADS, HALO = SMOOTH ? 6 : 0, W = T + 2 * HALO;
     constexpr int PER = (W * W + THREADS - 1) / THREADS;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_down(StLevel L, StLev
     double* rcs = si + W * W;
     double* rcd = rcs + W;                   /* W + 1 */
     __shared__ double sh[64];
-    const int i0 = blockIdx.x * T, k0 = blockIdx.y * T, nx = L.nx, nz = L.nz;
+    const int kt = (T == 32 ? row0 : 0) + blockIdx.y, i0 = blockIdx.x * T, k0 = kt * T, nx = L.nx, nz = L.nz;
     const int done = cg.ctl[0];
     /* every load is under way before anything waits for one */
     double b[PER], a[PER], id[PER], pv[PER], xv[PER];
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_down(StLevel L, StLev
         }
         if (SMOOTH) { const int o = st_at<W>(li, lk); sx[o] = 0.0; sb[o] = b[j]; si[o] = id[j]; }
     }
-    if (CG) st_partial<true, THREADS>(rn, cg.part_rn, blockIdx.y * gridDim.x + blockIdx.x, sh);
+    if (CG) st_partial<true, THREADS>(rn, cg.part_rn, kt * gridDim.x + blockIdx.x, sh);
     if constexpr (SMOOTH) {
         __syncthreads();
         st_half_sweep<W, THREADS, false>(sx, sb, si, rcs, rcd, 0);
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_down(StLevel L, StLev
  * tile's share of r.z.  SMOOTH = false: the dot product alone (xo is there). */
 template <int T, bool CG, bool SMOOTH>
 __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_up(StLevel L, StLevel Lc, const int* __restrict__ ctl,
-                                                              const double* __restrict__ r, double* part_rz)
+                                                              const double* __restrict__ r, double* part_rz, int row0)
 {
     constexpr int THREADS = StTile<T>::THREADS, HALO = SMOOTH ? 4 : 0, W = T + 2 * HALO;
     constexpr int PER = (W * W + THREADS - 1) / THREADS;
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_up(StLevel L, StLevel
     double* rcs = si + W * W;
     double* rcd = rcs + W;                   /* W + 1 */
     __shared__ double sh[32];
-    const int i0 = blockIdx.x * T, k0 = blockIdx.y * T, nx = L.nx, nz = L.nz;
+    const int kt = (T == 32 ? row0 : 0) + blockIdx.y, i0 = blockIdx.x * T, k0 = kt * T, nx = L.nx, nz = L.nz;
     const double* bsrc = CG ? r : L.b;
     if constexpr (SMOOTH) {
         /* only the colour the first half-sweep reads needs its value */
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(StTile<T>::THREADS) k_st_up(StLevel L, StLevel
         if (SMOOTH) L.xo[p] = x;
         if (CG) rz += (SMOOTH ? sb[o] : r[p]) * x;
     }
-    if (CG) st_partial<false, THREADS>(rz, part_rz, blockIdx.y * gridDim.x + blockIdx.x, sh);
+    if (CG) st_partial<false, THREADS>(rz, part_rz, kt * gridDim.x + blockIdx.x, sh);
 }
 
 /* p = z + beta p (into the other buffer: neighbours read the old one), Ap and
@@ -915,7 +915,16 @@ static int st_tile(const StLevel& L)
 {
     return ((L.nx + 31) / 32) * ((L.nz + 31) / 32) >= 74 ? 32 : 16;
 }
-static dim3 st_tiles(const StLevel& L, int T) { return dim3((unsigned)((L.nx + T - 1) / T), (unsigned)((L.nz + T - 1) / T)); }
+/* the tiles' rows from row0 on that one launch takes: a grid has at most 65535
+ * blocks in y, fewer than the tallest levels have rows of tiles (of 32, since a
+ * level of tiles of 16 has at most 148) */
+#define ST_GRID_ROWS 65535
+static int st_tile_rows(const StLevel& L, int T) { return (L.nz + T - 1) / T; }
+static dim3 st_tiles(const StLevel& L, int T, int row0)
+{
+    const int rows = st_tile_rows(L, T) - row0;
+    return dim3((unsigned)((L.nx + T - 1) / T), (unsigned)(rows < ST_GRID_ROWS ? rows : ST_GRID_ROWS));
+}
 static size_t st_down_smem(int T) { const int W = T + 12; return sizeof(double) * (3 * W * W + 2 * W + 1); }
 static size_t st_up_smem(int T) { const int W = T + 8; return sizeof(double) * (3 * W * W + 2 * W + 1); }
 static size_t st_tail_smem(const bcg_steady* s)
@@ -931,15 +940,21 @@ template <bool CG, bool SMOOTH>
 static void st_down(bcg_steady* s, int l, const StCg& cg)
 {
     const StLevel &L = s->L[l], &Lc = s->L[l + 1 < s->nlev ? l + 1 : l];
-    if (st_tile(L) == 32) k_st_down<32, CG, SMOOTH><<<st_tiles(L, 32), 512, SMOOTH ? st_down_smem(32) : 0, s->stream>>>(L, Lc, cg);
-    else k_st_down<16, CG, SMOOTH><<<st_tiles(L, 16), 256, SMOOTH ? st_down_smem(16) : 0, s->stream>>>(L, Lc, cg);
+    const int T = st_tile(L);
+    for (int r0 = 0; r0 < st_tile_rows(L, T); r0 += ST_GRID_ROWS) {
+        if (T == 32) k_st_down<32, CG, SMOOTH><<<st_tiles(L, 32, r0), 512, SMOOTH ? st_down_smem(32) : 0, s->stream>>>(L, Lc, cg, r0);
+        else k_st_down<16, CG, SMOOTH><<<st_tiles(L, 16, 0), 256, SMOOTH ? st_down_smem(16) : 0, s->stream>>>(L, Lc, cg, 0);
+    }
 }
 template <bool CG, bool SMOOTH>
 static void st_up(bcg_steady* s, int l, const double* r, double* part_rz)
 {
     const StLevel &L = s->L[l], &Lc = s->L[l + 1 < s->nlev ? l + 1 : l];
-    if (st_tile(L) == 32) k_st_up<32, CG, SMOOTH><<<st_tiles(L, 32), 512, SMOOTH ? st_up_smem(32) : 0, s->stream>>>(L, Lc, s->ctl, r, part_rz);
-    else k_st_up<16, CG, SMOOTH><<<st_tiles(L, 16), 256, SMOOTH ? st_up_smem(16) : 0, s->stream>>>(L, Lc, s->ctl, r, part_rz);
+    const int T = st_tile(L);
+    for (int r0 = 0; r0 < st_tile_rows(L, T); r0 += ST_GRID_ROWS) {
+        if (T == 32) k_st_up<32, CG, SMOOTH><<<st_tiles(L, 32, r0), 512, SMOOTH ? st_up_smem(32) : 0, s->stream>>>(L, Lc, s->ctl, r, part_rz, r0);
+        else k_st_up<16, CG, SMOOTH><<<st_tiles(L, 16, 0), 256, SMOOTH ? st_up_smem(16) : 0, s->stream>>>(L, Lc, s->ctl, r, part_rz, 0);
+    }
 }
 
 /* the CG step of iteration `it` (0: the start), the stopping rule and the
@@ -1096,8 +1111,8 @@ extern "C" int bcg_steady_create(const bcg_steady_params* p, bcg_steady** out)
         s->tail = l;
     }
     {
-        const dim3 t0 = st_tiles(s->L[0], st_tile(s->L[0]));
-        s->nt0 = (int)(t0.x * t0.y);
+        const int T = st_tile(s->L[0]);
+        s->nt0 = ((p->nx + T - 1) / T) * st_tile_rows(s->L[0], T);
         s->ntd = (int)nblk(s->n) < 592 ? (int)nblk(s->n) : 592;     /* 4 blocks an SM */
     }
     const size_t np = (size_t)(s->nt0 > (int)nblk(s->n) ? s->nt0 : (int)nblk(s->n));
