@@ -1287,7 +1287,7 @@ static bool smooth_interpolates(const bcg_ctx* c, const MgConst& m, int l)
 }
 
 template <class T>
-static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps, bool interpolate = false)
+static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps, bool interpolate = false, bool tiles = true)
 {
     const int rows = c->mg[l].nz + 1;
     /* levels of 0-1 interior rows read across columns through the flat
@@ -1297,7 +1297,7 @@ static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps, bool i
         return;
     }
     if constexpr (sizeof(T) == 8) {
-        if (c->relax_mode == 3 && tile_takes(c->mg[l])) {
+        if (c->relax_mode == 3 && tiles && tile_takes(c->mg[l])) {
             const int warm = warm_rows(m, l);
             while (sweeps > 0) {
                 const int S = sweeps >= 3 ? 3 : sweeps;
@@ -1350,8 +1350,8 @@ static void smooth_level(bcg_ctx* c, const MgConst& m, int l, int sweeps, bool i
     }
 }
 
-/* device time (ms) of one level-0 launch of the fused 3-sweep smoother at
- * the shape bcg_autotune chose (0 before tuning) */
+/* device time (ms) of one level-0 launch of the fused 3-sweep smoother that
+ * bcg_autotune tunes, at the shape it chose (0 before tuning) */
 extern "C" int bcg_smoother_launch_ms(bcg_ctx* c, double* ms)
 {
     if (!c || !ms) return BCG_E_ARG;
@@ -1393,7 +1393,9 @@ int mg_kernel_attributes()
 /* bcg_autotune(BCG_TUNE_SMOOTHER): time the fused smoother on the finest
  * level for several warp targets (two launches each, so the correction
  * buffers end where they started) and keep the fastest.  TMA form: 1 to
- * 16 row segments; per-lane staging form: its resident-warp targets. */
+ * 16 row segments, also where FP64 solves take the level on register tiles,
+ * which have no target (the mixed solve's FP32 cycles take it in the TMA form);
+ * per-lane staging form: its resident-warp targets. */
 int mg_tune_smoother(bcg_ctx* c, int* choice)
 {
     const int rows = c->mg[0].nz + 1;
@@ -1419,11 +1421,11 @@ int mg_tune_smoother(bcg_ctx* c, int* choice)
     int best_t = saved > 0 ? saved : (c->relax_mode == 3 ? SMOOTH_TMA_WARPS_DEFAULT : SMOOTH_WARPS_DEFAULT);
     for (int ti = 0; ti < nt; ti++) {
         c->smooth_warps = targets[ti];
-        smooth_level<double>(c, m, 0, 3);                  /* warm-up */
-        smooth_level<double>(c, m, 0, 3);
+        smooth_level<double>(c, m, 0, 3, false, false);    /* warm-up */
+        smooth_level<double>(c, m, 0, 3, false, false);
         cudaEventRecord(a, c->stream);
-        smooth_level<double>(c, m, 0, 3);
-        smooth_level<double>(c, m, 0, 3);
+        smooth_level<double>(c, m, 0, 3, false, false);
+        smooth_level<double>(c, m, 0, 3, false, false);
         cudaEventRecord(b, c->stream);
         if (cudaEventSynchronize(b) != cudaSuccess || c->pending_error) {
             cudaEventDestroy(a); cudaEventDestroy(b); c->smooth_warps = saved;

@@ -28,6 +28,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "cell-steps/s"
+TILE_POINTS = 1800000          # csrc/mg.cu: levels an FP64 solve smooths on register tiles
 
 
 def parse():
@@ -993,11 +994,15 @@ def b200_arm(args):
                               "40 B on the composite levels, zeroing 16 B on the others"}
     # the dominant single kernel: the fused 3-sweep smoother on a finest
     # composite level, 24 B per point and species (R and E read, E2
-    # written), timed with CUDA events by the autotuner
+    # written), timed with CUDA events by the autotuner.  The autotuner times
+    # the form staged by the tensor memory accelerator; a solve takes levels
+    # of up to TILE_POINTS points on register tiles instead, so there the
+    # whole solve stands in the line
     sm_ms = tuned.get("smoother_launch_ms", 0.0)
     lvl0_pts = 3 * (p.box_x + 1) * (p.box_z_agar + 1)
     sm_bytes = 24.0 * lvl0_pts
-    if mg_ms >= mech_ms and sm_ms > 0:
+    on_tiles = tuned.get("relax_mode", 3) == 3 and lvl0_pts // 3 <= TILE_POINTS
+    if mg_ms >= mech_ms and sm_ms > 0 and not on_tiles:
         sm_gbs = sm_bytes / (sm_ms / 1e3) / 1e9
         # the smoother form in use (bcg_set_relax_mode; the library's default is 3)
         tma = tuned.get("relax_mode", 3) == 3

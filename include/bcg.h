@@ -363,8 +363,10 @@ int bcg_set_pair_precision(bcg_ctx* ctx, int bits);
  *                         needs binned cells and neighbour lists; leaves
  *                         the colony unchanged;
  *   BCG_TUNE_SMOOTHER     resident-warp target of the fused agar smoother
- *                         (how many row segments a level is cut into);
- *                         changes only the multigrid's correction scratch.
+ *                         (how many row segments a level is cut into) in
+ *                         the form that has one, relax mode 2's or 3's
+ *                         (there not the register tiles); changes only the
+ *                         multigrid's correction scratch.
  * Every kernel choice belongs to its context: no call changes another
  * context's kernels.  Synchronises the stream; not for use inside a
  * stream capture. */
@@ -388,7 +390,8 @@ int bcg_autotune(bcg_ctx* ctx, int what, int* choice);
  *                          (0 = default or tuned);
  *   bcg_smoother_launch_ms device time of one finest-level launch of the
  *                          fused smoother measured by the last
- *                          BCG_TUNE_SMOOTHER (0 before). */
+ *                          BCG_TUNE_SMOOTHER, in the form it tunes (0
+ *                          before). */
 int bcg_set_force_group(bcg_ctx* ctx, int lanes);
 int bcg_set_relax_mode(bcg_ctx* ctx, int mode);
 int bcg_set_smoother_warps(bcg_ctx* ctx, int warps);
