@@ -1203,7 +1203,7 @@ extern "C" int bcg_steady_solve(bcg_steady* s, const double* theta, const double
     k_st_deposit<<<nblk(n), 256, 0, s->stream>>>(n, s->P.h, s->P.c0, s->start, s->order, s->cell, s->w, s->q, s->C);
     int it = 0, cgt = 0, rc;
     double f0 = 0.0;
-    for (; it < 50; it++) {
+    for (; it < 50; it++) {                  /* a run to the end (it == 50) missed its bound */
         double fn;
         if ((rc = st_newton_rhs(s, vmax, km, &fn))) return rc;
         if (it == 0) f0 = fn > 0 ? fn : 1.0;

@@ -52,6 +52,9 @@ class Steady:
         self.ncell = len(a)
 
     def solve(self, theta, w, tol=1e-13):
+        """The steady field.  newton_iters is 50 afterwards where max|F| did
+        not fall to tol of its start, which on fine grids lies below its
+        rounding (bcg_steady_solve)."""
         th = np.ascontiguousarray(theta, dtype=np.float64).reshape(4)
         w = np.ascontiguousarray(w, dtype=np.float64).reshape(-1)
         assert w.size == self.ncell

@@ -419,9 +419,14 @@ int bcg_steady_destroy(bcg_steady* s);
 /* cells as 4 doubles each: centre x (from the grid's left edge), centre z
  * (from the agar bottom), length L, radius R; at most max_cells */
 int bcg_steady_set_cells(bcg_steady* s, const double* xzlr, int ncell);
-/* Newton to max|F| <= tol * (max|F| at C = c0); C_out (nx*nz, row k at
- * offset k*nx, optional) receives the field.  The converged state is kept
- * for bcg_steady_vjp. */
+/* Newton to max|F| <= tol * (max|F| at C = c0), 50 steps at most; C_out
+ * (nx*nz, row k at offset k*nx, optional) receives the field.
+ * *newton_iters (optional) receives the steps taken: below 50 the bound was
+ * met; 50 says that it was not, with BCG_OK all the same and the field of the
+ * last step.  F has a rounding of its own, which the steps do not get below
+ * (about 4e-13 of its start at 513 x 257 vertices), so a smaller tol runs all
+ * 50 on a field that has long converged.  The state is kept for
+ * bcg_steady_vjp. */
 int bcg_steady_solve(bcg_steady* s, const double* theta, const double* w, double tol,
                      double* C_out, int* newton_iters, int* cg_iters);
 /* Vector-Jacobian product at the last solve: given dL/dC (nx*nz), the
