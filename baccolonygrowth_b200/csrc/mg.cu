@@ -1268,9 +1268,11 @@ static int warm_rows(const MgConst& m, int l)
 }
 
 /* Levels the register-tiled smoother takes (relax mode 3).  Its time grows with
- * the points (39 us at 2305 x 513, 130 us at 4609 x 1025), the TMA form's hardly
- * does until its warps fill the SMs (57 and 87 us); the line lies where the two
- * meet. */
+ * the points, the TMA form's hardly does until its warps fill the SMs; the line
+ * lies where the two meet.  Three sweeps on one level, us:
+ *   points (millions)   1.18  1.48  1.77  1.85  1.97  2.17  2.36  2.95  4.72
+ *   tiles               39.3  48.3  56.8  57.9  63.8  69.2  71.9  88.7   139
+ *   TMA                 50.8  53.9  57.2  57.0  58.2  60.2  62.5  69.3  89.4 */
 #define TILE_POINTS 1800000
 static bool tile_takes(const MgLevel& L) { return (long)(L.nx + 1) * (L.nz + 1) <= TILE_POINTS; }
 

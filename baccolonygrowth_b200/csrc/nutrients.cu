@@ -400,8 +400,10 @@ static void sweep_launch(dim3 grid, dim3 block, bcg_ctx* c, const NutConst& n, E
  * wider than the colony by 5: blocks of its own take it.  Results go
  * to a second set of buffers, which the next launch reads.
  * Measured a sweep, launches included: 33 thousand cells 8.9 -> 3.1 us (tiles of
- * 4), a million 19 -> 14.6 us (tiles of 16).  It is bound by instruction issue: 0.64
- * a cycle and scheduler at a million cells, 1.6 points computed for one owned. */
+ * 4), a million 19 -> 14.6 us (tiles of 16, whose threads spill a little at the 64
+ * registers that two blocks an SM leave: 20 bytes stored, 64 loaded).  It is
+ * bound by instruction issue: 0.64 a cycle and scheduler at a million cells, 1.6
+ * points computed for one owned. */
 /* A tile's columns.  16 recompute least (1.6 points for one) and fill the SMs
  * from about 150 tiles on; fewer tiles leave SMs idle and a block's own chain of
  * instructions is what counts, so smaller tiles with a thread a point. */

@@ -859,6 +859,7 @@ def b200_arm(args):
     pair32 = None
     try:
         _abi.check(lib.bcg_set_pair_precision(ctx, 32), "pair precision 32")
+        _abi.check(lib.bcg_sim_run(sim, 1), "fp32 search warm-up")     # its first launch loads the kernel
         _abi.check(lib.bcg_enable_timers(ctx, 1), "timers")
         _abi.check(lib.bcg_sim_run(sim, kt_steps), "fp32 search steps")
         msx = ctypes.c_double(); nl = ctypes.c_int64()
