@@ -320,6 +320,7 @@ extern "C" int bcg_create(const bcg_params* p, bcg_ctx** out)
     double** f2[] = {&c->rws, &c->wds, &c->rw, &c->wd};
     for (auto a : f2) { DALLOC(*a, X * 8); if ((rc = fill(c, *a, 0.0, X))) { bcg_destroy(c); return rc; } }
     DALLOC(c->sweep_type, X * Z);
+    DALLOC(c->res0_inside, X * 8);
     DALLOC(c->bbox, 64);
     BCG_CUDA_TRY(cudaMemsetAsync(c->bbox, 0, 64, c->stream));
     /* multigrid levels, Multigrid.cpp:5-33: LocalAga defaults in all arrays */
@@ -366,7 +367,7 @@ extern "C" int bcg_destroy(bcg_ctx* c)
                     c->div_list, c->step, c->fcw_count, c->moved, c->delta_ids, c->delta_box, c->lineage,
                     c->draws_dev, c->div_rec, c->div_box, c->div_rect, c->div_pairs, c->div_par,
                     c->div_order, c->div_grp, c->height, c->rough_height, c->nrm_x, c->nrm_y, c->nrm_z,
-                    c->wall, c->rd, c->inside, c->rds, c->ds, c->dens, c->rws, c->wds, c->rw, c->wd, c->bbox, c->mg_scratch, c->sweep_type};
+                    c->wall, c->rd, c->inside, c->rds, c->ds, c->dens, c->rws, c->wds, c->rw, c->wd, c->bbox, c->mg_scratch, c->sweep_type, c->res0_inside};
     for (void* q : ptrs) if (q) cudaFree(q);
     for (int b = 0; b < 2; b++) {
         EnvBuf& e = c->env[b];

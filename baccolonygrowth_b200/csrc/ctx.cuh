@@ -149,8 +149,11 @@ struct bcg_ctx {
     /* multigrid Err (all levels) and Res (levels > 0) are zero, as the last
      * reset() left them; setup() then skips its resetZero */
     int mg_clean;
-    /* level 0's Res of the last reset() not computed yet (done on demand) */
+    /* level 0's Res of the last reset() not computed yet (done on demand): 1,
+     * from insideColonyDen; 2, the field has changed since and res0_inside
+     * holds its row z = 0, which is all that Res takes of it */
     int mg_res0_stale;
+    double* res0_inside;
     int pair_f32;          /* contact geometry in FP32 local to cell i (bcg_set_pair_precision) */
     int pending_error;     /* host-side set-up failure of a queued launch, returned by the next status check */
     /* legacy explicit agar solver (allocated on its first call): FieldAgar

@@ -14,9 +14,12 @@ int bin_cells(bcg_ctx* c, int buf);
 
 #define IX(x, z) ((size_t)(x) * Z + (z))
 
-__global__ void k_bbox_reset(int* bbox, int X)
+/* keep (may be null): insideColonyDen's row z = 0 as it was */
+__global__ void k_bbox_reset(int* bbox, int X, int Z, const double* __restrict__ inside, double* __restrict__ keep)
 {
-    if (threadIdx.x == 0) { bbox[0] = X; bbox[1] = 0; bbox[2] = 0; }
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x == 0) { bbox[0] = X; bbox[1] = 0; bbox[2] = 0; }
+    if (keep && x < X) keep[x] = inside[IX(x, 0)];
 }
 
 /* one box's share of the column's heights: the highest top among the cells
@@ -250,13 +253,17 @@ static int deposit(bcg_ctx* c, bool smooth)
 {
     const bcg_params& P = c->P;
     if (P.filter_len > 8 || P.refinement_grid_height > 8) return BCG_E_UNSUPPORTED;
-    mg_res0_materialise(c);            /* it reads insideColonyDen, rewritten here */
     c->host_bbox[0] = -1;              /* until this deposition has ended well */
     timer_begin(c, BCG_T_DENSITY);
     int rc = bin_cells(c, c->cur);
     if (rc) return rc;
     const int X = P.box_x, Z = P.box_z;
-    k_bbox_reset<<<1, 32, 0, c->stream>>>(c->bbox, X);
+    /* level 0's Res, if a caller asks for it, is worked out from the field as
+     * the solve saw it: at a million boxes a column's row costs 2 us to keep, the
+     * whole Res 70 */
+    const bool keep = c->mg_res0_stale == 1;
+    k_bbox_reset<<<(X + 127) / 128, 128, 0, c->stream>>>(c->bbox, X, Z, c->inside, keep ? c->res0_inside : nullptr);
+    if (keep) c->mg_res0_stale = 2;
     k_get_density<<<X, COLUMN_THREADS, 0, c->stream>>>(X, Z, P.refinement_grid_height, P.box_length, P.cell_radius,
         c->rec[c->cur], c->box_start, c->box_ids, c->rd, c->inside, c->height, c->bbox);
     k_inside_ring<<<(X * Z + 255) / 256, 256, 0, c->stream>>>(X, Z, c->inside);
@@ -288,7 +295,7 @@ extern "C" int bcg_update_height(bcg_ctx* c)
     int rc = bin_cells(c, c->cur);
     if (rc) return rc;
     const int X = P.box_x, Z = P.box_z;
-    k_bbox_reset<<<1, 32, 0, c->stream>>>(c->bbox, X);
+    k_bbox_reset<<<1, 32, 0, c->stream>>>(c->bbox, X, Z, nullptr, nullptr);
     k_get_height<<<(X + 3) / 4, COLUMN_THREADS, 0, c->stream>>>(X, Z, P.refinement_grid_height, P.box_length, P.cell_radius,
         c->rec[c->cur], c->box_start, c->box_ids, c->height, c->bbox);
     k_bbox_finish<<<1, 32, 0, c->stream>>>(c->bbox, X, Z, P.filter_len / 2, c->status);

@@ -1600,17 +1600,18 @@ static void update_sol(bcg_ctx* c, const MgConst& m, int l)
     k_mg_update_sol<<<grid_rows(L.nx + 1, L.nz + 1, 256), 256, 0, c->stream>>>(m, L, l);
     c->launches++;
 }
-static void update_res(bcg_ctx* c, const MgConst& m, int l, bool setup_clean = false)
+/* inside0: insideColonyDen's row z = 0, box_z values apart */
+static void update_res(bcg_ctx* c, const MgConst& m, int l, bool setup_clean, const double* inside0)
 {
     MgLvl L = mg_lvl(c, l), Lp = mg_lvl(c, l > 0 ? l - 1 : 0);
     dim3 grid((unsigned)((L.nx + 1 + 127) / 128), (unsigned)(L.nz + 1), 3);
     const ResConst rc = res_const(m, l);
     if (l == 0) {
-        if (setup_clean) k_mg_update_res<true, true><<<grid, 128, 0, c->stream>>>(m, L, Lp, l, rc, c->inside);
-        else k_mg_update_res<false, true><<<grid, 128, 0, c->stream>>>(m, L, Lp, l, rc, c->inside);
+        if (setup_clean) k_mg_update_res<true, true><<<grid, 128, 0, c->stream>>>(m, L, Lp, l, rc, inside0);
+        else k_mg_update_res<false, true><<<grid, 128, 0, c->stream>>>(m, L, Lp, l, rc, inside0);
     } else {
-        if (setup_clean) k_mg_update_res<true, false><<<grid, 128, 0, c->stream>>>(m, L, Lp, l, rc, c->inside);
-        else k_mg_update_res<false, false><<<grid, 128, 0, c->stream>>>(m, L, Lp, l, rc, c->inside);
+        if (setup_clean) k_mg_update_res<true, false><<<grid, 128, 0, c->stream>>>(m, L, Lp, l, rc, inside0);
+        else k_mg_update_res<false, false><<<grid, 128, 0, c->stream>>>(m, L, Lp, l, rc, inside0);
     }
     c->launches++;
 }
@@ -1622,12 +1623,12 @@ void mg_setup(bcg_ctx* c, const MgConst& m)
     if (c->mg_clean) {
         /* resetZero and updateSolAga have nothing to do but the clamp */
         c->mg_clean = 0;
-        for (int l = 0; l <= m.A - 1; l++) update_res(c, m, l, true);
+        for (int l = 0; l <= m.A - 1; l++) update_res(c, m, l, true, c->inside);
         return;
     }
     reset_zero(c);
     for (int l = 0; l <= m.A - 1; l++) update_sol(c, m, l);
-    for (int l = 0; l <= m.A - 1; l++) update_res(c, m, l);
+    for (int l = 0; l <= m.A - 1; l++) update_res(c, m, l, false, c->inside);
 }
 
 /* reset(), Multigrid.cpp:827-841 (evalUpdateRes's result is discarded there),
@@ -1670,12 +1671,16 @@ void mg_solved(bcg_ctx* c)
 }
 
 /* level 0's Res as reset() leaves it, before a caller reads or writes a
- * multigrid array or rewrites insideColonyDen */
+ * multigrid array or sets insideColonyDen (a deposition keeps the row of that
+ * field instead) */
 void mg_res0_materialise(bcg_ctx* c)
 {
     if (!c->mg_res0_stale) return;
+    const bool kept = c->mg_res0_stale == 2;
     c->mg_res0_stale = 0;
-    update_res(c, mg_const(c, c->P.mg_dt), 0);
+    MgConst m = mg_const(c, c->P.mg_dt);
+    if (kept) m.box_z = 1;                 /* the kept row lies side by side */
+    update_res(c, m, 0, false, kept ? c->res0_inside : c->inside);
 }
 
 void mg_copy_to(bcg_ctx* c, const MgConst& m, int wall_buf)

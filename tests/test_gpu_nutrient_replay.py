@@ -57,6 +57,33 @@ def test_res_after_replay(gpu, between):
     a.close(); b.close()
 
 
+@pytest.mark.parametrize("solve", ["update", "mg_solve"])
+def test_res_is_of_the_field_the_solve_saw(gpu, solve):
+    """Level 0's Res read before a deposition of other cells and after it, and
+    after two."""
+    out = []
+    for depositions in (0, 1, 2):
+        col, other = pair()
+        other.close()
+        for k in range(3):
+            col.nutrient_update(2) if solve == "update" else col.mg_solve()
+            if k < 2:
+                col.update_density()
+        for d in range(depositions):
+            cells = workload_colony("small_4k", n=1024)
+            cells["p"][:, 0] += 40.0 * (d + 1)
+            cells["q"][:, 0] += 40.0 * (d + 1)
+            before = col.field("INSIDE")
+            col.upload(cells)
+            col.update_density()
+            assert not np.array_equal(before, col.field("INSIDE"))
+        out.append([col.field("MG_RES_" + s, 0) for s in SPECIES])
+        col.close()
+    for o in out[1:]:
+        for x, y in zip(out[0], o):
+            assert np.abs(x).max() > 0 and np.array_equal(x, y)
+
+
 def test_legacy_after_replay(gpu):
     a, b = pair()
     update(a, b)
