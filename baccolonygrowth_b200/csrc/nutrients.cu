@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(SwTile<TX>::THREADS, TX == 16 ? 2 : 1) k_sweep
     }
     const int zt = blockIdx.y - 1, x0 = minx + blockIdx.x * TX;
     const bool floor_ = zt == 0;
-    if (x0 > maxx || zt >= sw_tile_rows(maxz)) return;
+    if (x0 > maxx || !sw_runs(zt, maxz)) return;
     const int z0 = sw_first(zt), z1 = sw_end(zt, maxz);
     const int zb = floor_ ? -1 : z0 - SW_K, xb = x0 - SW_K;       /* of row and column 0 */
     double* v = reinterpret_cast<double*>(sw_smem);              /* [buffer][species][column][row] */

@@ -24,5 +24,7 @@ SW_FN bool sw_one_row(int maxz) { return maxz + 2 < SW_RZ; }
 SW_FN int sw_tile_rows(int maxz) { return sw_one_row(maxz) ? 1 : 1 + (maxz + 1 - SW_OWN0 + SW_OWN - 1) / SW_OWN; }
 /* the points z0 <= z < z1 that row zt of the tiles owns */
 SW_FN int sw_first(int zt) { return zt == 0 ? 0 : SW_OWN0 + (zt - 1) * SW_OWN; }
+/* whether row zt has any (zt < sw_tile_rows(maxz), without its division) */
+SW_FN bool sw_runs(int zt, int maxz) { return sw_first(zt) <= maxz && (zt == 0 || !sw_one_row(maxz)); }
 SW_FN int sw_end(int zt, int maxz) { return zt > 0 ? sw_first(zt) + SW_OWN : sw_one_row(maxz) ? maxz + 1 : SW_OWN0; }
 #endif

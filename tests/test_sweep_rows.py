@@ -17,15 +17,16 @@ PROBE = r"""
 #include "sweep_rows.h"
 int main()
 {
-    /* a block of tile row zt runs if zt is below the count and then stores its rows up to maxz */
+    /* a block of tile row zt runs if sw_runs says so and then stores its rows up to maxz */
     for (int maxz = 0; maxz < 400; maxz++) {
         const int rows = sw_tile_rows(maxz);
         printf("%d %d", maxz, rows);
         for (int z = 0; z <= maxz; z++) {
             int owners = 0;
-            for (int zt = 0; zt < rows; zt++) owners += z >= sw_first(zt) && z < sw_end(zt, maxz);
+            for (int zt = 0; zt < 20; zt++) owners += sw_runs(zt, maxz) && z >= sw_first(zt) && z < sw_end(zt, maxz);
             if (owners != 1) printf(" row %d has %d owners", z, owners);
         }
+        for (int zt = 0; zt < 20; zt++) if (sw_runs(zt, maxz) != (zt < rows)) printf(" tile row %d is not counted", zt);
         /* a tile row that owns nothing */
         for (int zt = 0; zt < rows; zt++) if (sw_first(zt) > maxz) printf(" tile row %d is empty", zt);
         /* the bottom tile alone holds the box and the unswept row above it */
