@@ -674,7 +674,9 @@ extern "C" int bcg_set_field(bcg_ctx* c, int f, int level, const double* in, siz
     if (f == BCG_F_INSIDE) c->host_bbox[0] = -1;
     if (v.mg == 1) { c->mg_clean = 0; nutrient_graphs_drop(c); }   /* Err/Res may no longer be zero */
     if (!v.mg) {
-        BCG_CUDA_TRY(cudaMemcpy(v.ptr, in, v.n * 8, cudaMemcpyHostToDevice));
+        /* on the context's stream: the launch above reads insideColonyDen */
+        BCG_CUDA_TRY(cudaMemcpyAsync(v.ptr, in, v.n * 8, cudaMemcpyHostToDevice, c->stream));
+        BCG_CUDA_TRY(cudaStreamSynchronize(c->stream));
         return BCG_OK;
     }
     BCG_CUDA_TRY(cudaMemcpyAsync(c->mg[0].err2[0], in, sizeof(double) * v.n, cudaMemcpyHostToDevice, c->stream));

@@ -84,6 +84,19 @@ def test_res_is_of_the_field_the_solve_saw(gpu, solve):
             assert np.abs(x).max() > 0 and np.array_equal(x, y)
 
 
+def test_res_is_of_the_field_before_it_is_set(gpu):
+    """insideColonyDen that a caller sets after a solve does not reach the Res
+    that the solve left."""
+    a, b = pair()
+    for col in (a, b):
+        col.mg_solve()
+    want = [a.field("MG_RES_" + s, 0) for s in SPECIES]
+    b.set_field("INSIDE", 1.0 - b.field("INSIDE"))
+    for s, w in zip(SPECIES, want):
+        assert np.array_equal(b.field("MG_RES_" + s, 0), w), s
+    a.close(); b.close()
+
+
 def test_legacy_after_replay(gpu):
     a, b = pair()
     update(a, b)
