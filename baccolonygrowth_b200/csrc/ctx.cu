@@ -525,10 +525,12 @@ extern "C" int bcg_set_neighbours(bcg_ctx* c, const int* counts, const int* list
         if (counts[i] > c->kmax) { free(tmp); return BCG_E_NEIGH_OVERFLOW; }
         for (int j = 0; j < counts[i]; j++) tmp[(size_t)i * c->kmax + j] = lists[(size_t)i * stride + j];
     }
-    cudaError_t e1 = cudaMemcpy(c->ncount, counts, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice);
-    cudaError_t e2 = cudaMemcpy(c->nbr, tmp, sizeof(int) * (size_t)n * c->kmax, cudaMemcpyHostToDevice);
+    /* on the context's stream: a rebuild queued there writes the lists too */
+    cudaError_t e1 = cudaMemcpyAsync(c->ncount, counts, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream);
+    cudaError_t e2 = cudaMemcpyAsync(c->nbr, tmp, sizeof(int) * (size_t)n * c->kmax, cudaMemcpyHostToDevice, c->stream);
+    cudaError_t e3 = cudaStreamSynchronize(c->stream);
     free(tmp);
-    if (e1 || e2) { g_last_cuda = e1 ? e1 : e2; return BCG_E_CUDA; }
+    if (e1 || e2 || e3) { g_last_cuda = e1 ? e1 : (e2 ? e2 : e3); return BCG_E_CUDA; }
     return BCG_OK;
 }
 
