@@ -656,7 +656,7 @@ extern "C" int bcg_get_field(bcg_ctx* c, int f, int level, double* out, size_t n
         BCG_CUDA_TRY(cudaMemcpyAsync(out, v.ptr, v.n * 8, cudaMemcpyDeviceToHost, c->stream));
         return ctx_check_status(c);
     }
-    mg_res0_materialise(c);
+    if (f >= BCG_F_MG_RES_CARBON && f <= BCG_F_MG_RES_ACETATE && level == 0) mg_res0_materialise(c);
     int nz1 = v.mg == 1 ? v.nz + 1 : (int)(v.n / (v.nx + 1));   /* rows delivered */
     int k0 = v.mg == 1 ? 0 : 1;
     plane_turn(c, c->mg[0].err2[0], v.ptr, v.nx + 1, nz1, k0, v.pitch, 0);

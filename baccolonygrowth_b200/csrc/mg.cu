@@ -1635,8 +1635,8 @@ void mg_setup(bcg_ctx* c, const MgConst& m)
  * and copyFromMG (958-981) into the wall buffers: two launches over all
  * levels.  The reference recomputes Res on every composite level in reset(), and
  * its resetZero clears it again on levels > 0; level 0's is read by nothing before
- * the next setup() recomputes it: it is computed only when a caller reads a
- * multigrid array or changes its inputs (mg_res0_materialise). */
+ * the next setup() recomputes it: it is computed only when a caller reads it or
+ * changes its inputs (mg_res0_materialise). */
 void mg_finish(bcg_ctx* c, const MgConst& m, int cur_wall)
 {
     MgAll a;
@@ -1670,7 +1670,7 @@ void mg_solved(bcg_ctx* c)
     c->leg_old_stale = 1;        /* copyFromMG writes FieldAgar and oldFieldAgar alike */
 }
 
-/* level 0's Res as reset() leaves it, before a caller reads or writes a
+/* level 0's Res as reset() leaves it, before a caller reads it, writes a
  * multigrid array or sets insideColonyDen (a deposition keeps the row of that
  * field instead) */
 void mg_res0_materialise(bcg_ctx* c)
